@@ -364,8 +364,8 @@ bool ensure_lists(xr_ctx* c, long long E, long long P, long long B) {
   GROW(edge_pair, E);
   GROW(edge_dbslot, E);
   GROW(hval, E);
-  GROW(qch, E);
-  GROW(qcj, E);
+  GROW(qch, E + 4);  // the solver reads its rows in aligned quads
+  GROW(qcj, E + 4);
   GROW(pair_edge, P);
   GROW(pair_i, P);
   GROW(pair_bond, P);

@@ -880,9 +880,11 @@ __device__ inline void rows_sum_all(double* v, int m) {
 // Lanes per matrix row in the per-row loops over a block's m rows: as many as keep the rows within
 // two passes of the block's warps (at least 4), so short rows of small systems do not leave most
 // lanes idle; each lane keeps four entries' loads in flight.
-__device__ inline int row_group(int m) {
+// Long rows of many get at least 16 lanes, so that neighbouring lanes' loads share a cache line.
+__device__ inline int row_group(int m, int entries = 0) {
   int g = 32;
-  while (g > 4 && m * g > 2048) g >>= 1;
+  const int least = entries > 128 * m ? 16 : 4;
+  while (g > least && m * g > 2048) g >>= 1;
   return g;
 }
 
@@ -938,8 +940,8 @@ __device__ inline bool team_sumf(const Team& team, const XrWork& w, float* v, fl
 // for a system of n atoms of which this block owns m rows (r0 .. r1):
 //   yt[n4]  D v for every row of the system (v = M^-1 of the vector being multiplied), the vector the
 //           product gathers; n4 = n rounded up to a multiple of 4; two such buffers for a cluster
-//   own rows, m floats each: the constants D_ii, eta D^-1, c = H w1, w1 = M^-1 1, then the solver's
-//           x (the correction), p, s, r, u, and for the pipelined solver of grid teams q, z, w, m~
+//   own rows, a record each: the constants D_ii, eta D^-1, c = H w1, w1 = M^-1 1, then the solver's
+//           x (the correction), p, s, r, u, and for the pipelined solver of grid teams q, z, w, m~, hv
 //   binv[8m] row r of its group's inverse block (columns: the group's rows in order)
 //   rp[m + 1] row starts relative to the cache; first[m], size[m] the group of each row (16-bit)
 // M is block-Jacobi: groups of at most 8 consecutive own rows whose atoms are joined by distances
@@ -982,51 +984,106 @@ __device__ inline int qeq_aligned_split_warp(const XrWork& w, int a0, int n, int
   return r;
 }
 
-struct Rows32 {
-  float *yt, *dd, *etadi, *cw, *wv, *x, *p, *s, *rr, *u, *q, *z, *wq, *mt, *binv;
-  int* rp;
-  unsigned short *first, *size;
-  int n4;
-  // nyt gathered-vector buffers; nvec per-row vectors (rows32_vectors)
-  __device__ Rows32(unsigned char* base, int n, int m, int nyt, int nvec) {
-    float* f = reinterpret_cast<float*>(base);
-    n4 = (n + 3) / 4 * 4;
-    yt = f;
-    dd = f + nyt * n4;
-    etadi = dd + m;
-    cw = etadi + m;
-    wv = cw + m;
-    x = wv + m;
-    p = x + m;
-    s = p + m;
-    rr = s + m;
-    u = rr + m;
-    q = u + m;  // q, z, w, m~: the pipelined solver's only
-    z = q + m;
-    wq = z + m;
-    mt = wq + m;
-    binv = dd + nvec * m;
-    rp = reinterpret_cast<int*>(binv + kGroupMax * m);
-    first = reinterpret_cast<unsigned short*>(rp + m + 1);
-    size = first + m;
-  }
-  // FP32 scratch of the setup, 8 per row over dd .. rr
-  __device__ float* scratch32() const { return dd; }
-  // buffer k of the gathered vector (a cluster team alternates two)
-  __device__ float* ytb(int k) const { return yt + (k & 1) * n4; }
-};
-
 // Buffers of the gathered vector: two for a cluster team, whose blocks write into each other's.
 template <class Team>
 __host__ __device__ constexpr int rows32_yt_buffers() {
   return std::is_same<Team, ClusterTeam>::value ? 2 : 1;
 }
 
-// Per-row vectors: the constants D, eta D^-1, c, w1 and the textbook solver's x, p, s, r, u; the
-// pipelined solver of grid teams adds q, z, w, m~.
+// Values per row: the constants D, eta D^-1, c, w1 and the textbook solver's x, p, s, r, u; the
+// pipelined solver of grid teams adds q, z, w, m~ and the sums of streamed rows, and one unused to keep
+// the row stride odd (a thread per row then meets no bank conflict).
 template <class Team>
 __host__ __device__ constexpr int rows32_vectors() {
-  return std::is_same<Team, GridTeam>::value ? 13 : 9;
+  return std::is_same<Team, GridTeam>::value ? 15 : 9;
+}
+
+// One record of consecutive values per row: a row's values lie at constant offsets from one address (a
+// separate array per value cost the solvers a register per array, which they spilled).
+template <class Team>
+struct Rows32 {
+  static constexpr int kStride = rows32_vectors<Team>();
+  float *yt, *rec, *binv;
+  int* rp;
+  unsigned short *first, *size;
+  int n4;
+  __device__ Rows32(unsigned char* base, int n, int m) {
+    float* f = reinterpret_cast<float*>(base);
+    n4 = (n + 3) / 4 * 4;
+    yt = f;
+    rec = f + rows32_yt_buffers<Team>() * n4;
+    binv = rec + kStride * m;
+    rp = reinterpret_cast<int*>(binv + kGroupMax * m);
+    first = reinterpret_cast<unsigned short*>(rp + m + 1);
+    size = first + m;
+  }
+  __device__ float& at(int k, int i) const { return rec[kStride * i + k]; }
+  __device__ float& dd(int i) const { return at(0, i); }
+  __device__ float& etadi(int i) const { return at(1, i); }
+  __device__ float& cw(int i) const { return at(2, i); }
+  __device__ float& wv(int i) const { return at(3, i); }
+  __device__ float& x(int i) const { return at(4, i); }
+  __device__ float& p(int i) const { return at(5, i); }
+  __device__ float& s(int i) const { return at(6, i); }
+  __device__ float& rr(int i) const { return at(7, i); }
+  __device__ float& u(int i) const { return at(8, i); }
+  __device__ float& q(int i) const { return at(9, i); }  // q .. hv: the pipelined solver's only
+  __device__ float& z(int i) const { return at(10, i); }
+  __device__ float& wq(int i) const { return at(11, i); }
+  __device__ float& mt(int i) const { return at(12, i); }
+  __device__ float& hv(int i) const { return at(13, i); }
+  // FP32 scratch of the setup, 8 per row over the records
+  __device__ float* scratch32() const { return rec; }
+  // buffer k of the gathered vector (a cluster team alternates two)
+  __device__ float* ytb(int k) const { return yt + (k & 1) * n4; }
+};
+
+// Off-diagonal row sums H'yt of m rows that stream from global memory (the L2 cache): kStreamLanes
+// lanes share a row and each takes four consecutive entries at a time, a 16-byte load of values and
+// an 8-byte load of columns, kStreamQuads such quads in flight. Rows start anywhere, so quads lie on
+// multiples of four of the buffers (qch, qcj: the engine allocates them past the last quad) and
+// entries outside the row are masked. ch and cj point at the block's first entry, number ebeg of the
+// buffers; rp holds the row starts from there. Kept out of line: inlined into the solver, which
+// sits at its 64-register limit, the loop spilled. Bound by the L2 cache, which a system this large
+// does not quite fit: on the 36,864-atom water box (94 MB of rows an iteration, 2.8 ms of QEq) 8 lanes a
+// row took 3.7 ms, 16 lanes 3.2 ms, 32 lanes 3.04 ms with one quad in flight more or less 0.4 ms
+// slower, and 2.8 ms with the values marked as the first to evict; the solver with Jacobi,
+// two reductions an iteration and gathers from global memory took 9.2 ms.
+constexpr int kStreamLanes = 32, kStreamQuads = 2;
+__device__ __noinline__ void stream_rows(const float* ch, const unsigned short* cj, int ebeg, const int* rp, int m,
+                                         const float* yt, float* out, int stride) {
+  const float* const h0 = ch - ebeg;
+  const unsigned short* const j0 = cj - ebeg;
+  constexpr int kRows = 32 / kStreamLanes;  // rows a warp takes at a time
+  const int sub = threadIdx.x & (kStreamLanes - 1);
+  for (int ib = (int)(threadIdx.x >> 5) * kRows; ib < m; ib += (int)(blockDim.x >> 5) * kRows) {  // uniform per warp
+    const int i = ib + (int)(threadIdx.x & 31) / kStreamLanes;
+    const int beg = i < m ? rp[i] + ebeg : 0, end = i < m ? rp[i + 1] + ebeg : 0;
+    float s = 0.0f;
+    for (int e = (beg & ~3) + 4 * sub; e < end; e += 4 * kStreamLanes * kStreamQuads) {
+      float4 h[kStreamQuads];
+      ushort4 j[kStreamQuads];
+#pragma unroll
+      for (int u = 0; u < kStreamQuads; ++u) {
+        const int q = e + 4 * kStreamLanes * u;
+        if (q < end) {
+          h[u] = __ldcs(reinterpret_cast<const float4*>(h0 + q));
+          j[u] = __ldcg(reinterpret_cast<const ushort4*>(j0 + q));
+        }
+      }
+#pragma unroll
+      for (int u = 0; u < kStreamQuads; ++u) {
+        const int q = e + 4 * kStreamLanes * u;
+        if (q >= beg && q < end) s += h[u].x * yt[j[u].x];
+        if (q + 1 >= beg && q + 1 < end) s += h[u].y * yt[j[u].y];
+        if (q + 2 >= beg && q + 2 < end) s += h[u].z * yt[j[u].z];
+        if (q + 3 >= beg && q + 3 < end) s += h[u].w * yt[j[u].w];
+      }
+    }
+#pragma unroll
+    for (int o = kStreamLanes / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    if (sub == 0 && i < m) out[stride * i] = s;
+  }
 }
 
 template <class Team>
@@ -1048,7 +1105,7 @@ __device__ __noinline__ bool qeq_rows32_setup(const XrWork& w, const double* ata
   constexpr bool kGrid = std::is_same<Team, GridTeam>::value;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, tid = threadIdx.x;
   const int m = r1 - r0;
-  Rows32 R(qeq_dyn, n, m, rows32_yt_buffers<Team>(), rows32_vectors<Team>());
+  const Rows32<Team> R(qeq_dyn, n, m);
   const double* DI = &QW(Q_DINV, 0);
   const int gs = row_group(m), sub = lane & (gs - 1), gpw = 32 / gs;
   // 1. for every own row, the latest of the kGroupMax - 1 own rows before it that is bonded to it
@@ -1147,7 +1204,7 @@ __device__ __noinline__ bool qeq_rows32_setup(const XrWork& w, const double* ata
       for (int q = 0; q < kGroupMax; ++q) R.binv[kGroupMax * (f + r) + q] = q >= k ? 0.0f : ok ? a[q] : (q == r ? di : 0.0f);
     }
   }
-  __syncthreads();  // the scratch (dd .. rr) is free again
+  __syncthreads();  // the scratch is free again
   // 5. Jacobi rows, w = M^-1 1 (the stored inverse rows' sums), D, eta D^-1, the row starts
   double s1[1] = {0.0};
   for (int i = tid; i < m; i += blockDim.x) {
@@ -1161,9 +1218,9 @@ __device__ __noinline__ bool qeq_rows32_setup(const XrWork& w, const double* ata
       wsum = 0.0f;
       for (int c = 0; c < kGroupMax; ++c) wsum += R.binv[kGroupMax * i + c];
     }
-    R.wv[i] = wsum;
-    R.dd[i] = float(1.0 / di);
-    R.etadi[i] = float(atom_prm(atab, w.type[a], A_ETA) * di);
+    R.wv(i) = wsum;
+    R.dd(i) = float(1.0 / di);
+    R.etadi(i) = float(atom_prm(atab, w.type[a], A_ETA) * di);
     R.rp[i] = w.cnt[a] - M.ebeg;
     s1[0] += double(wsum);
   }
@@ -1176,7 +1233,7 @@ __device__ __noinline__ bool qeq_rows32_setup(const XrWork& w, const double* ata
   unsigned remote = 0;
   if constexpr (kCluster) remote = smem_u32(R.yt + r0);
   for (int i = tid; i < m; i += blockDim.x) {
-    const float v = R.wv[i] * R.dd[i];
+    const float v = R.wv(i) * R.dd(i);
     R.yt[r0 + i] = v;
     if constexpr (kCluster) {
       for (int r = 0; r < team.nb; ++r)
@@ -1195,7 +1252,7 @@ __device__ __noinline__ bool qeq_rows32_setup(const XrWork& w, const double* ata
     if (i < m)
       for (int e = R.rp[i] + sub; e < R.rp[i + 1]; e += gs) t += M.cache_h[e] * R.yt[M.cache_j[e]];
     for (int o = gs / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-    if (sub == 0 && i < m) R.cw[i] = t + R.etadi[i] * R.yt[r0 + i];
+    if (sub == 0 && i < m) R.cw(i) = t + R.etadi(i) * R.yt[r0 + i];
   }
   __syncthreads();
   return true;
@@ -1221,7 +1278,7 @@ __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, Qeq
   constexpr bool kCluster = std::is_same<Team, ClusterTeam>::value;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, tid = threadIdx.x;
   const int m = r1 - r0;
-  Rows32 R(qeq_dyn, n, m, rows32_yt_buffers<Team>(), rows32_vectors<Team>());
+  const Rows32<Team> R(qeq_dyn, n, m);
   // the row cache: in this block's shared memory, or FP32 rows in global memory
   const bool cache_shared = __isShared(M.cache_h);
   const float* const ch_g = M.cache_h;
@@ -1250,23 +1307,23 @@ __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, Qeq
     const int f = R.first[i], k = R.size[i];
     const float* bi = R.binv + kGroupMax * i;
     float t = 0.0f;
-    for (int b = 0; b < k; ++b) t += bi[b] * R.rr[f + b];
+    for (int b = 0; b < k; ++b) t += bi[b] * R.rr(f + b);
     return t;
   };
   for (int i = tid; i < m; i += blockDim.x) {
-    R.rr[i] = float(__ldcg(G + a0 + r0 + i));
-    R.p[i] = 0.0f;
-    R.s[i] = 0.0f;
-    R.x[i] = 0.0f;
+    R.rr(i) = float(__ldcg(G + a0 + r0 + i));
+    R.p(i) = 0.0f;
+    R.s(i) = 0.0f;
+    R.x(i) = 0.0f;
   }
   __syncthreads();
   float u0 = 0.0f, u1 = 0.0f;
   for (int i = tid; i < m; i += blockDim.x) {
     const float y = group_apply(i);
-    R.u[i] = y;
-    publish(i, y * R.dd[i]);
-    u0 += R.wv[i] * R.rr[i];
-    u1 += R.rr[i] * y;
+    R.u(i) = y;
+    publish(i, y * R.dd(i));
+    u0 += R.wv(i) * R.rr(i);
+    u1 += R.rr(i) * y;
   }
   // start: lambda = <w, g> / <w, 1>, and <g - lambda, M^-1 (g - lambda)> = <g, M^-1 g> - lambda <w, g>
   float acc[2] = {u0, u1};
@@ -1314,15 +1371,15 @@ __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, Qeq
         s = cache_shared ? row_dot(ch_s, cj_s, R.rp[i] + sub, R.rp[i + 1]) : row_dot(ch_g, cj_g, R.rp[i] + sub, R.rp[i + 1]);
       for (int o = gs / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
       if (sub == 0 && i < m) {
-        const float hz = s + R.etadi[i] * yt[r0 + i] - lam * R.cw[i];
-        const float z = R.u[i] - lam * R.wv[i];
-        const float pv = -z + beta * R.p[i];
-        const float hpv = -hz + beta * R.s[i];
-        R.p[i] = pv;
-        R.s[i] = hpv;
-        R.rr[i] -= lam;
+        const float hz = s + R.etadi(i) * yt[r0 + i] - lam * R.cw(i);
+        const float z = R.u(i) - lam * R.wv(i);
+        const float pv = -z + beta * R.p(i);
+        const float hpv = -hz + beta * R.s(i);
+        R.p(i) = pv;
+        R.s(i) = hpv;
+        R.rr(i) -= lam;
         php0 += pv * hpv;
-        php1 += R.wv[i] * hpv;
+        php1 += R.wv(i) * hpv;
       }
     }
     acc[0] = php0;
@@ -1340,8 +1397,8 @@ __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, Qeq
     if (sh.sc_state != 0) break;
     const float alpha = sh.sf_alpha, step = sh.sf_step;
     for (int i = tid; i < m; i += blockDim.x) {
-      R.rr[i] = (R.rr[i] + alpha * R.s[i]) - step;
-      R.x[i] += alpha * R.p[i];
+      R.rr(i) = (R.rr(i) + alpha * R.s(i)) - step;
+      R.x(i) += alpha * R.p(i);
     }
     __syncthreads();  // the group products read the other rows of the group
     u0 = 0.0f;
@@ -1349,10 +1406,10 @@ __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, Qeq
     buf ^= 1;
     for (int i = tid; i < m; i += blockDim.x) {
       const float y = group_apply(i);
-      R.u[i] = y;
-      publish(i, y * R.dd[i]);
-      u0 += R.wv[i] * R.rr[i];
-      u1 += R.rr[i] * y;
+      R.u(i) = y;
+      publish(i, y * R.dd(i));
+      u0 += R.wv(i) * R.rr(i);
+      u1 += R.rr(i) * y;
     }
     acc[0] = u0;
     acc[1] = u1;
@@ -1367,7 +1424,7 @@ __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, Qeq
       return -1;
     yt = yt_of(buf);
   }
-  for (int i = tid; i < m; i += blockDim.x) y_out[a0 + r0 + i] = R.x[i];
+  for (int i = tid; i < m; i += blockDim.x) y_out[a0 + r0 + i] = R.x(i);
   __syncthreads();
   return it;
 }
@@ -1400,7 +1457,9 @@ __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, Qeq
 // after staging exchange k - 2's buffer. (Written for any team: a cluster alternates two shared
 // buffers the same way.) The iteration stops when gamma falls to `ratio` times its start value.
 // The correction y of the own rows is written to y_out (global, indexed by atom).
-template <class Team>
+// kStream: the rows stream from global memory (stream_rows) instead of lying in this block's shared
+// memory; two instances, so that neither spills for the other's sake.
+template <class Team, bool kStream>
 __device__ __noinline__ int qeq_cg_rows32_pipelined(const XrWork& w, const Team& team, QeqShared& sh, int a0, int n,
                                                     int r0, int r1, const QeqMatrix<float>& M, float* y_out,
                                                     double ratio, int max_it, float* gyt0, float* gyt1, int* slot) {
@@ -1409,15 +1468,12 @@ __device__ __noinline__ int qeq_cg_rows32_pipelined(const XrWork& w, const Team&
   constexpr bool kGrid = std::is_same<Team, GridTeam>::value;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, tid = threadIdx.x;
   const int m = r1 - r0;
-  Rows32 R(qeq_dyn, n, m, rows32_yt_buffers<Team>(), rows32_vectors<Team>());
-  // the row cache: in this block's shared memory, or FP32 rows in global memory
-  const bool cache_shared = __isShared(M.cache_h);
-  const float* const ch_g = M.cache_h;
-  const unsigned short* const cj_g = M.cache_j;
-  const float* const ch_s =
-      reinterpret_cast<const float*>(qeq_dyn + (cache_shared ? (reinterpret_cast<const unsigned char*>(M.cache_h) - qeq_dyn) : 0));
+  const Rows32<Team> R(qeq_dyn, n, m);
+  // the row cache in this block's shared memory (offsets from the dynamic base: shared-memory loads)
+  const float* const ch_s = reinterpret_cast<const float*>(
+      qeq_dyn + (kStream ? 0 : reinterpret_cast<const unsigned char*>(M.cache_h) - qeq_dyn));
   const unsigned short* const cj_s = reinterpret_cast<const unsigned short*>(
-      qeq_dyn + (cache_shared ? (reinterpret_cast<const unsigned char*>(M.cache_j) - qeq_dyn) : 0));
+      qeq_dyn + (kStream ? 0 : reinterpret_cast<const unsigned char*>(M.cache_j) - qeq_dyn));
   const double* G = &QW(Q_G, 0);
   float* red = reinterpret_cast<float*>(sh.red);
   const float s1 = float(sh.sd_s1w);
@@ -1456,11 +1512,11 @@ __device__ __noinline__ int qeq_cg_rows32_pipelined(const XrWork& w, const Team&
       __syncthreads();
     }
   };
-  auto group_apply = [&](const float* v, int i) {  // (M^-1 v)_i over the group of row i
+  auto group_apply = [&](int v, int i) {  // M^-1 of the rows' value v, row i: over its group
     const int f = R.first[i], k = R.size[i];
     const float* bi = R.binv + kGroupMax * i;
     float t = 0.0f;
-    for (int b = 0; b < k; ++b) t += bi[b] * v[f + b];
+    for (int b = 0; b < k; ++b) t += bi[b] * R.at(v, f + b);
     return t;
   };
   // lanes per row: the fewest that take the block's rows in one pass over its warps (a block of 33
@@ -1486,33 +1542,38 @@ __device__ __noinline__ int qeq_cg_rows32_pipelined(const XrWork& w, const Team&
       for (; e < ee; e += gs) t += ch[e] * yt[cj[e]];
       return t;
     };
-    for (int ib = wid * gpw; ib < m; ib += nw * gpw) {
-      const int i = ib + lane / gs;
-      float t = 0.0f;
-      if (i < m)
-        t = cache_shared ? row_dot(ch_s, cj_s, R.rp[i] + sub, R.rp[i + 1]) : row_dot(ch_g, cj_g, R.rp[i] + sub, R.rp[i + 1]);
-      for (int o = gs / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-      if (sub == 0 && i < m) epi(i, t + R.etadi[i] * yt[r0 + i]);
+    if constexpr (!kStream) {
+      for (int ib = wid * gpw; ib < m; ib += nw * gpw) {
+        const int i = ib + lane / gs;
+        float t = 0.0f;
+        if (i < m) t = row_dot(ch_s, cj_s, R.rp[i] + sub, R.rp[i + 1]);
+        for (int o = gs / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
+        if (sub == 0 && i < m) epi(i, t + R.etadi(i) * yt[r0 + i]);
+      }
+    } else {
+      stream_rows(M.cache_h, M.cache_j, M.ebeg, R.rp, m, yt, &R.hv(0), R.kStride);
+      __syncthreads();
+      for (int i = tid; i < m; i += blockDim.x) epi(i, R.hv(i) + R.etadi(i) * yt[r0 + i]);
     }
   };
   // start: r = -g0, u~ = M^-1 r exchanged with the reduction of <w1, r> and <r, u~>; then
   // u = u~ - w1 <w1, r>/s1 and w = H u = H u~ - c <w1, r>/s1
   for (int i = tid; i < m; i += blockDim.x) {
-    R.rr[i] = -float(__ldcg(G + a0 + r0 + i));
-    R.x[i] = 0.0f;
-    R.p[i] = 0.0f;
-    R.s[i] = 0.0f;
-    R.q[i] = 0.0f;
-    R.z[i] = 0.0f;
+    R.rr(i) = -float(__ldcg(G + a0 + r0 + i));
+    R.x(i) = 0.0f;
+    R.p(i) = 0.0f;
+    R.s(i) = 0.0f;
+    R.q(i) = 0.0f;
+    R.z(i) = 0.0f;
   }
   __syncthreads();
   float acc[3] = {0.0f, 0.0f, 0.0f};
   for (int i = tid; i < m; i += blockDim.x) {
-    const float t = group_apply(R.rr, i);
-    R.u[i] = t;
-    publish(i, t * R.dd[i]);
-    acc[0] += R.wv[i] * R.rr[i];
-    acc[1] += R.rr[i] * t;
+    const float t = group_apply(7, i);
+    R.u(i) = t;
+    publish(i, t * R.dd(i));
+    acc[0] += R.wv(i) * R.rr(i);
+    acc[1] += R.rr(i) * t;
   }
   if (!team_sumf<2>(team, w, acc, red, [&](const float* t) {
         const float shift = t[0] / s1;
@@ -1526,8 +1587,8 @@ __device__ __noinline__ int qeq_cg_rows32_pipelined(const XrWork& w, const Team&
   if (sh.sc_state == 0) {
     const float shift = sh.sf_shift;
     product([&](int i, float hv) {
-      R.wq[i] = hv - shift * R.cw[i];
-      R.u[i] -= shift * R.wv[i];
+      R.wq(i) = hv - shift * R.cw(i);
+      R.u(i) -= shift * R.wv(i);
     });
     __syncthreads();  // the group products read the other rows of the group
   }
@@ -1537,12 +1598,12 @@ __device__ __noinline__ int qeq_cg_rows32_pipelined(const XrWork& w, const Team&
     buf ^= 1;
     acc[0] = acc[1] = acc[2] = 0.0f;
     for (int i = tid; i < m; i += blockDim.x) {
-      const float t = group_apply(R.wq, i);
-      R.mt[i] = t;
-      publish(i, t * R.dd[i]);
-      acc[0] += R.rr[i] * R.u[i];
-      acc[1] += R.wq[i] * R.u[i];
-      acc[2] += R.wv[i] * R.wq[i];
+      const float t = group_apply(11, i);
+      R.mt(i) = t;
+      publish(i, t * R.dd(i));
+      acc[0] += R.rr(i) * R.u(i);
+      acc[1] += R.wq(i) * R.u(i);
+      acc[2] += R.wv(i) * R.wq(i);
     }
     const bool more = it < max_it;
     if (!team_sumf<3>(team, w, acc, red, [&](const float* t) {
@@ -1569,25 +1630,25 @@ __device__ __noinline__ int qeq_cg_rows32_pipelined(const XrWork& w, const Team&
     stage();
     const float alpha = sh.sf_alpha, beta = sh.sf_beta, shift = sh.sf_shift;
     product([&](int i, float hv) {
-      const float nv = hv - shift * R.cw[i];
-      const float mv = R.mt[i] - shift * R.wv[i];
-      const float zv = nv + beta * R.z[i];
-      const float qv = mv + beta * R.q[i];
-      const float sv = R.wq[i] + beta * R.s[i];
-      const float pv = R.u[i] + beta * R.p[i];
-      R.z[i] = zv;
-      R.q[i] = qv;
-      R.s[i] = sv;
-      R.p[i] = pv;
-      R.x[i] += alpha * pv;
-      R.rr[i] -= alpha * sv;
-      R.u[i] -= alpha * qv;
-      R.wq[i] -= alpha * zv;
+      const float nv = hv - shift * R.cw(i);
+      const float mv = R.mt(i) - shift * R.wv(i);
+      const float zv = nv + beta * R.z(i);
+      const float qv = mv + beta * R.q(i);
+      const float sv = R.wq(i) + beta * R.s(i);
+      const float pv = R.u(i) + beta * R.p(i);
+      R.z(i) = zv;
+      R.q(i) = qv;
+      R.s(i) = sv;
+      R.p(i) = pv;
+      R.x(i) += alpha * pv;
+      R.rr(i) -= alpha * sv;
+      R.u(i) -= alpha * qv;
+      R.wq(i) -= alpha * zv;
     });
     __syncthreads();  // the group products read the other rows of the group
     ++it;
   }
-  for (int i = tid; i < m; i += blockDim.x) y_out[a0 + r0 + i] = R.x[i];
+  for (int i = tid; i < m; i += blockDim.x) y_out[a0 + r0 + i] = R.x(i);
   __syncthreads();
   return it;
 }
@@ -1602,7 +1663,7 @@ __device__ bool qeq_residual(const XrWork& w, const double* atab, const Team& te
   double* X = &QW(Q_X, 0);
   double* G = &QW(Q_G, 0);
   const double* DI = &QW(Q_DINV, 0);
-  const int gs = row_group(r1 - r0), sub = lane & (gs - 1), gpw = 32 / gs;
+  const int gs = row_group(r1 - r0, w.cnt[a0 + r1] - w.cnt[a0 + r0]), sub = lane & (gs - 1), gpw = 32 / gs;
   double acc[1] = {0.0};
   for (int rb = r0 + wid * gpw; rb < r1; rb += nw * gpw) {
     const int r = rb + lane / gs, a = a0 + r;
@@ -1695,7 +1756,7 @@ __device__ void qeq_solve(const XrWork& w, const double* atab, const Team& team,
   // rows fit, else FP64 values + columns (10 B), else nothing (rows read from global memory).
   // A block that solves a system of at most 1024 atoms alone keeps every row's FP32 state in shared
   // memory instead, and so does each block of a cluster team for its rows plus the whole vector the
-  // product gathers (layout Rows32: 4 B per atom of the system, 8 B in a cluster, and 76 B per own row, 92 B in a
+  // product gathers (layout Rows32: 4 B per atom of the system, 8 B in a cluster, and 76 B per own row, 100 B in a
   // grid team), and at least
   // the n doubles of the FP64 stage of a fallback.
   constexpr bool kBlock = std::is_same<Team, BlockTeam>::value;
@@ -1704,12 +1765,16 @@ __device__ void qeq_solve(const XrWork& w, const double* atab, const Team& team,
   constexpr bool kGridTeam = std::is_same<Team, GridTeam>::value;
   int team_rows = n;  // the most rows any block of the team owns (the same value in every block)
   if constexpr (kGridTeam) team_rows = min(n, ((n + team.nb - 1) / team.nb + 31) / 32 * 32 + kGroupMax);
+  // A grid team takes the row solver while that layout fits at all (up to about 45,000 atoms on 152
+  // blocks), also where it leaves no room for the rows, which then stream from the L2 cache
+  // (stream_rows).
   const bool small_rows =
-      dyn != nullptr && ((kBlock || kCluster) ? n <= 1024 : rows32_bytes<Team>(n, team_rows) <= (size_t)dyn_bytes / 2);
-  const int stage_n = (dyn != nullptr && (small_rows || n * 8 <= dyn_bytes / 2)) ? n : 0;
-  const size_t stage_bytes =
-      small_rows ? std::max<size_t>(rows32_bytes<Team>(n, r1 - r0), 8 * (size_t)n) : 8 * (size_t)stage_n;
-  void* gstage = stage_n > 0 ? dyn : nullptr;
+      dyn != nullptr && ((kBlock || kCluster) ? n <= 1024 : rows32_bytes<Team>(n, team_rows) <= (size_t)dyn_bytes);
+  // The FP64 solve that may follow the FP32 sweeps stages its gradient over the whole space (it reads
+  // the rows from hval), when the n doubles fit.
+  const bool stage64 = small_rows ? 8 * (size_t)n <= (size_t)dyn_bytes : n * 8 <= dyn_bytes / 2;
+  const size_t stage_bytes = dyn == nullptr ? 0 : small_rows ? rows32_bytes<Team>(n, r1 - r0) : stage64 ? 8 * (size_t)n : 0;
+  void* gstage = dyn != nullptr && stage64 ? dyn : nullptr;
   unsigned char* region = dyn != nullptr ? dyn + stage_bytes : nullptr;
   const long long region_bytes = dyn != nullptr ? dyn_bytes - (long long)stage_bytes : 0;
   // Rows that do not fit are kept in FP32 in global memory (L2-resident for a batch) instead, so the
@@ -1718,7 +1783,7 @@ __device__ void qeq_solve(const XrWork& w, const double* atab, const Team& team,
   const bool fits32 = region != nullptr && cols16 && nent <= region_bytes / 6;
   const bool glob32 = !fits32 && cols16 && w.qch != nullptr;
   const bool mixed = fits32 || glob32;
-  const bool cached64 = !mixed && region != nullptr && cols16 && nent <= region_bytes / 10;
+  const bool cached64 = !mixed && !small_rows && region != nullptr && cols16 && nent <= region_bytes / 10;
   void* cache_h = region;
   unsigned short* cache_j = nullptr;
   if (fits32) cache_j = reinterpret_cast<unsigned short*>(region + 4 * (size_t)(region_bytes / 6));
@@ -1729,7 +1794,7 @@ __device__ void qeq_solve(const XrWork& w, const double* atab, const Team& team,
   if (cached64) cache_j = reinterpret_cast<unsigned short*>(region + 8 * (size_t)(region_bytes / 10));
   // 1. Jacobi diagonal (eta + self-image shields) of the owned rows, and the start point: the
   //    uniform x0 = Q/n, or the caller's charges of an earlier step (already summing to Q).
-  const int gs = row_group(r1 - r0), sub = lane & (gs - 1), gpw = 32 / gs;
+  const int gs = row_group(r1 - r0, nent), sub = lane & (gs - 1), gpw = 32 / gs;
   for (int rb = r0 + wid * gpw; rb < r1; rb += nw * gpw) {
     const int r = rb + lane / gs, a = a0 + r;
     double d = 0;
@@ -1943,7 +2008,10 @@ __device__ void qeq_solve(const XrWork& w, const double* atab, const Team& team,
       int it = 0;
       if (small_rows) {
         if constexpr (kGridTeam)
-          it = qeq_cg_rows32_pipelined(w, team, sh, a0, n, r0, r1, M32, v32.y, sh.sd_ratio, budget, v32.g, v32.g2, &slot);
+          it = fits32 ? qeq_cg_rows32_pipelined<Team, false>(w, team, sh, a0, n, r0, r1, M32, v32.y, sh.sd_ratio, budget, v32.g,
+                                                             v32.g2, &slot)
+                      : qeq_cg_rows32_pipelined<Team, true>(w, team, sh, a0, n, r0, r1, M32, v32.y, sh.sd_ratio, budget, v32.g,
+                                                            v32.g2, &slot);
         else
           it = qeq_cg_rows32(w, team, sh, a0, n, r0, r1, M32, v32.y, sh.sd_ratio, budget, &slot);
       } else {
@@ -2062,7 +2130,7 @@ __global__ void __launch_bounds__(1024, 1) k_qeq_grid(XrWork w, XrFF ff, const i
   if ((int)blockIdx.x < nteam) {
     const int4 m = map[blockIdx.x];
     const XrSystem& S = w.sys[m.x];
-    // the rows of this block (k_qeq_splits: equal shares of 32-row multiples, no molecule cut)
+    // the rows of this block (k_qeq_splits: equal shares, no molecule cut)
     const int r0 = w.qsplit[2 * blockIdx.x], r1 = max(r0, w.qsplit[2 * blockIdx.x + 1]);
     GridTeam team{w.barrier + m.w, w.red + (size_t)32 * m.w, m.z, m.y};
     qeq_solve(w, atoms_of_system(ff, S), team, S.atom_off, S.natoms, r0, r1, adjoint ? 0.0 : S.total_charge,
@@ -2076,7 +2144,7 @@ __global__ void __launch_bounds__(1024, 1) k_qeq_grid(XrWork w, XrFF ff, const i
 // the solve). Cluster teams (map == null): qsplit[k * (csize + 1) + q] for system big[k] and
 // q = 0 .. csize, at about the same number of matrix entries per block. Grid teams: qsplit[2 b] and
 // qsplit[2 b + 1] for team block b (map[b] = {system, rank, team size, first block}), at the team's
-// equal shares of 32-row multiples. Each split then moves to the nearest one that cuts no molecule.
+// equal shares. Each split then moves to the nearest one that cuts no molecule.
 __global__ void k_qeq_splits(XrWork w, const int* big, int nbig, int csize, const int4* map, int nteam) {
   const int t = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
   const int lane = threadIdx.x & 31;
@@ -2104,7 +2172,10 @@ __global__ void k_qeq_splits(XrWork w, const int* big, int nbig, int csize, cons
     const int4 m = map[t >> 1];
     sys = m.x;
     const int n = w.sys[sys].natoms;
-    const int per = ((n + m.z - 1) / m.z + 31) / 32 * 32;
+    // whole tiles of 32 rows for a team that has about one a block (fewer rows would leave lanes idle),
+    // equal shares above that (256 rows for 242 would leave 8 of 152 blocks without any)
+    int per = (n + m.z - 1) / m.z;
+    if (per <= 64) per = (per + 31) / 32 * 32;
     r = min(n, (m.y + (t & 1)) * per);
   }
   const XrSystem& S = w.sys[sys];
