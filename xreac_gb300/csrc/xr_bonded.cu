@@ -127,7 +127,13 @@ __device__ inline void bo1_tile(const XrWork& w, const XrFF& ff0, int b, int nb)
     BFV(BF_DPI, b) = dpi;
     BFV(BF_DPP, b) = dpp;
     BFV(BF_MASK, b) = mask ? 1.0 : 0.0;
-    if (!mask) {  // the corrected orders of an inactive bond are zero; k_bo2 visits active bonds only
+    if (mask) {  // what the terms of an active bond are added to
+      BJV(BJ_BO, b) = 0.0;
+      BJV(BJ_PI, b) = 0.0;
+      BJV(BJ_PP, b) = 0.0;
+    } else {  // the corrected orders of an inactive bond are zero; k_bo2 visits active bonds only
+      BEV(0, b) = 0.0;
+      BEV(1, b) = 0.0;
       BFV(BF_BO, b) = 0.0;
       BFV(BF_PI, b) = 0.0;
       BFV(BF_PP, b) = 0.0;
@@ -370,8 +376,8 @@ __device__ inline void k_bond_energy_one(const XrWork& w, const XrFF& ff0, int b
       atomicAdd(gp + P_BE2, Des * sig * ex * be1 * powv * xr_log(sig));
     }
   }
-  BJV(BJ_PI, b) += -Dep;
-  BJV(BJ_PP, b) += -Depp;
+  atomicAdd(&BJV(BJ_PI, b), -Dep);  // (k_torsions may add at the same time)
+  atomicAdd(&BJV(BJ_PP, b), -Depp);
   double e_c2 = 0.0, dbo = 0.0;
   if (g[5] > 0.001 && __ldg(ff.is_carbon + ti) && __ldg(ff.is_carbon + tj)) {
     const int ends[2] = {i, j};
@@ -1312,41 +1318,55 @@ __global__ void k_chain_radial(XrWork w, XrFF ff) {
 // the cut), grid-striding over its device-side length.
 static int active_grid(const XrWork& w, int tb) { return std::max(1, std::min((w.nB + tb - 1) / tb, 152 * 8)); }
 
-void xr_launch_bond_orders(const XrWork& w, const XrFF& ff, cudaStream_t st) {
+void xr_launch_bond_orders(const XrWork& w, const XrFF& ff, const XrFork& fork) {
   const int tb = 128;
   const int gB = (w.nB + tb - 1) / tb;
+  const cudaStream_t st = fork.bonded;
+  fork.wait(st, fork.lists);
   // (the torsion-middle and active-bond counters were zeroed by k_prep)
   if (w.nB > 0) k_bo1<<<gB, tb, 0, st>>>(w, ff);
   k_deltap<<<(w.A + 3) / 4, 128, 0, st>>>(w);
   if (w.nB > 0) k_bo2<<<active_grid(w, tb), tb, 0, st>>>(w, ff);
+  fork.record(fork.orders, st);
 }
 
-void xr_launch_bonded(const XrWork& w, const XrFF& ff, cudaStream_t st) {
+void xr_launch_bonded(const XrWork& w, const XrFF& ff, const XrFork& fork) {
   const int tb = 128;
   const int gA = (w.A + tb - 1) / tb;
-  const int gB = (w.nB + tb - 1) / tb;
   const int gM = active_grid(w, tb);
+  const cudaStream_t st = fork.bonded, st_t = fork.torsion, st_h = fork.hbond;
   k_atom1<<<gA, tb, 0, st>>>(w, ff);
+  fork.record(fork.atoms, st);
+  // middles from the corrected orders; torsions and hydrogen bonds from the active rows of k_atom1
+  if (w.nB > 0) {
+    const int gT = std::min((w.nB + kMidTile - 1) / kMidTile, 152 * 16);
+    fork.wait(st_t, fork.orders);
+    k_mid_count<<<gT, kMidTile, 0, st_t>>>(w);
+    k_mid_scan<<<1, 1024, 0, st_t>>>(w);
+    k_mid_fill<<<gT, kMidTile, 0, st_t>>>(w);
+    fork.wait(st_t, fork.atoms);
+    const int chunks = (w.nB + kUnits - 1) / kUnits;
+    const int blocks = std::min((chunks + kBondedWarps - 1) / kBondedWarps, 152 * 16);
+    k_torsions<<<blocks, 32 * kBondedWarps, 0, st_t>>>(w, ff);
+    fork.record(fork.torsions, st_t);
+  }
+  fork.wait(st_h, fork.atoms);
+  k_hbonds<<<(w.A + kHbWarps - 1) / kHbWarps, 32 * kHbWarps, 0, st_h>>>(w, ff);
+  fork.record(fork.hbonds, st_h);
   k_atom2<<<gA, tb, 0, st>>>(w, ff);
   if (w.nB > 0) k_bond_energy<<<gM, tb, 0, st>>>(w, ff);
   {
     const int chunks = (w.A + kUnits - 1) / kUnits;
     k_angles<<<(chunks + kBondedWarps - 1) / kBondedWarps, 32 * kBondedWarps, 0, st>>>(w, ff);
   }
-  if (w.nB > 0) {
-    const int gT = std::min((w.nB + kMidTile - 1) / kMidTile, 152 * 16);
-    k_mid_count<<<gT, kMidTile, 0, st>>>(w);
-    k_mid_scan<<<1, 1024, 0, st>>>(w);
-    k_mid_fill<<<gT, kMidTile, 0, st>>>(w);
-    const int chunks = (w.nB + kUnits - 1) / kUnits;
-    const int blocks = std::min((chunks + kBondedWarps - 1) / kBondedWarps, 152 * 16);
-    k_torsions<<<blocks, 32 * kBondedWarps, 0, st>>>(w, ff);
-  }
-  k_hbonds<<<(w.A + kHbWarps - 1) / kHbWarps, 32 * kHbWarps, 0, st>>>(w, ff);
+  if (w.nB > 0) fork.wait(st, fork.torsions);
+  fork.wait(st, fork.hbonds);
   k_chain_atom<<<gA, tb, 0, st>>>(w, ff);
   if (w.nB > 0) {
     k_chain_bond<<<gM, tb, 0, st>>>(w, ff);
     k_chain_deltap<<<gA, tb, 0, st>>>(w);
+    fork.wait(st, fork.pairs);
     k_chain_radial<<<gM, tb, 0, st>>>(w, ff);
   }
+  fork.record(fork.done, st);
 }

@@ -314,20 +314,20 @@ void xr_launch_topology(const XrWork& w, cudaStream_t st);  // xr_launch_prep, t
 void xr_launch_prep(const XrWork& w, cudaStream_t st);      // wrapped FP32 coordinates (k_prep)
 void xr_launch_count(const XrWork& w, cudaStream_t st);     // all-pairs image scan, counts (k_neighbors<false>)
 void xr_launch_rows(const XrWork& w, cudaStream_t st);      // all-pairs image scan, rows (k_neighbors<true>)
-void xr_launch_scan(const XrWork& w, cudaStream_t st);
+int xr_launch_scan(const XrWork& w, cudaStream_t st);  // (this and the next four: the kernels launched)
 void xr_launch_topology_fill(const XrWork& w, cudaStream_t st);
 // Candidate list at the cutoff of w.sys (descriptors at rc + 2 skin): fill=false counts into cand_cnt
 // and scans it (total into counts[5]); fill=true writes cand_edge.
-void xr_launch_candidates(const XrWork& w, bool fill, cudaStream_t st);
+int xr_launch_candidates(const XrWork& w, bool fill, cudaStream_t st);
 // The edges within the cutoff of the candidate list: fill=false counts into cnt (scanned by
 // xr_launch_scan), fill=true writes the rows, pairs and bonds.
 void xr_launch_filter(const XrWork& w, bool fill, cudaStream_t st);
 // Cell list of the atoms binned by k_prep (atom_cell): counts per cell, their scan, cell_atoms.
-void xr_launch_cells(const XrWork& w, cudaStream_t st);
+int xr_launch_cells(const XrWork& w, cudaStream_t st);
 // Candidate list at the cutoff of w.sys from the cell list, in no particular order within a row:
 // fill=false counts into cand_cnt, scans it (total into counts[5]) and records the longest row in
 // counts[6]; fill=true writes cand_edge.
-void xr_launch_cell_candidates(const XrWork& w, bool fill, cudaStream_t st);
+int xr_launch_cell_candidates(const XrWork& w, bool fill, cudaStream_t st);
 // Sorts every candidate row into canonical (j, Sx, Sy, Sz) order; rows hold at most max_row entries
 // (at most XR_ROW_SORT_MAX).
 void xr_launch_row_sort(const XrWork& w, int max_row, cudaStream_t st);
@@ -350,7 +350,23 @@ constexpr int kQeqClusterSingle = 8;
 int xr_qeq_max_clusters(int csize);
 int xr_launch_qeq_cluster(const XrWork& w, const XrFF& ff, cudaStream_t st, int csize, int nblocks, const int* list,
                           int nbig, int nsmall, bool adjoint = false);
-void xr_launch_bond_orders(const XrWork& w, const XrFF& ff, cudaStream_t st);  // k_bo1, k_deltap, k_bo2
-void xr_launch_bonded(const XrWork& w, const XrFF& ff, cudaStream_t st);       // energy terms and adjoint chain
+// The streams of a call's launch sequence after the lists. The bonded terms need the lists and the
+// positions only, and the charges the pair kernel only, so the bond orders and bonded terms run beside
+// the pair kernel and the QEq solve, and the torsions and hydrogen bonds beside the angles; the parts
+// join before the bond-order chain's radial terms (which add to the pair kernel's) and the force
+// assembly. Without a fork (timed stages) every member is the call's own stream.
+struct XrFork {
+  bool on;
+  cudaStream_t main, bonded, torsion, hbond;
+  cudaEvent_t lists, pairs, orders, atoms, torsions, hbonds, done;
+  void record(cudaEvent_t e, cudaStream_t s) const {
+    if (on) cudaEventRecord(e, s);
+  }
+  void wait(cudaStream_t s, cudaEvent_t e) const {
+    if (on) cudaStreamWaitEvent(s, e, 0);
+  }
+};
+void xr_launch_bond_orders(const XrWork& w, const XrFF& ff, const XrFork& fork);  // k_bo1, k_deltap, k_bo2
+void xr_launch_bonded(const XrWork& w, const XrFF& ff, const XrFork& fork);       // energy terms and adjoint chain
 void xr_launch_forces(const XrWork& w, const XrFF& ff, cudaStream_t st);
 void xr_launch_reduce(const XrWork& w, const XrFF& ff, cudaStream_t st);

@@ -99,6 +99,9 @@ struct xr_ctx {
   static constexpr size_t kGraphCache = 128;
   static constexpr size_t kGraphSeen = 4096;
   int last_graph = 0;  // of the last call: 0 launched directly, 1 recorded, 2 replayed
+  // Side streams and events of the launch sequence (XrFork).
+  cudaStream_t side[3] = {};
+  cudaEvent_t fork_ev[7] = {};
   // Cell list (xr_ctx_set_cell_list): 0 chooses per call, 1 always, -1 never.
   int cell_mode = 0;
   int* atom_cell = nullptr;
@@ -1101,12 +1104,10 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     cudaMemsetAsync(c->cand_cnt, 0, sizeof(int) * ((size_t)A + 1), st);
     wl.cand_cnt = c->cand_cnt;
     if (ncells > 0) {
-      xr_launch_cells(wl, st);
-      xr_launch_cell_candidates(wl, false, st);
-      launches += 8;
+      launches += xr_launch_cells(wl, st);
+      launches += xr_launch_cell_candidates(wl, false, st);
     } else {
-      xr_launch_candidates(wl, false, st);
-      launches += 4;
+      launches += xr_launch_candidates(wl, false, st);
     }
     cudaMemcpyAsync(c->h_small + 9, c->counts + 5, 2 * sizeof(int), cudaMemcpyDeviceToHost, st);
     cudaMemcpyAsync(c->h_small + 4, c->status, sizeof(int), cudaMemcpyDeviceToHost, st);
@@ -1135,8 +1136,7 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     xr_launch_filter(w, false, st);
     launches += 1;
   }
-  xr_launch_scan(w, st);
-  launches += 3;
+  launches += xr_launch_scan(w, st);
   cudaMemcpyAsync(c->h_small, c->counts, 4 * sizeof(int), cudaMemcpyDeviceToHost, st);
   cudaMemcpyAsync(c->h_small + 4, c->status, sizeof(int), cudaMemcpyDeviceToHost, st);
   d2h += 5 * sizeof(int);
@@ -1174,6 +1174,9 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     return qcluster ? xr_launch_qeq_cluster(w, ff->d, st, qcsize, qblocks, c->qsmall, qbig, qsmall, adjoint)
                     : xr_launch_qeq(w, ff->d, st, qblocks, c->qmap, qteam, c->qsmall, qsmall, adjoint);
   };
+  const bool forked = !c->profile;
+  const XrFork fork = {forked, st, forked ? c->side[0] : st, forked ? c->side[1] : st, forked ? c->side[2] : st,
+                       c->fork_ev[0], c->fork_ev[1], c->fork_ev[2], c->fork_ev[3], c->fork_ev[4], c->fork_ev[5], c->fork_ev[6]};
   // The launch sequence: rows, pairs, QEq, bond orders, bonded terms, Coulomb energy and forces,
   // reductions, bond export. Returns 0 or a CUDA error of a launch.
   auto sequence = [&]() -> int {
@@ -1184,18 +1187,20 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
       xr_launch_filter(w, true, st);
     xr_launch_reverse(w, st);
     launches += 2;
-    cudaMemsetAsync(c->a_adj, 0, sizeof(double) * (size_t)AJ_N * A, st);
-    cudaMemsetAsync(c->f, 0, sizeof(double) * 3 * (size_t)A, st);
-    cudaMemsetAsync(c->b_adj, 0, sizeof(double) * (size_t)BJ_N * c->capB, st);
-    cudaMemsetAsync(c->b_e, 0, sizeof(double) * 4 * c->capB, st);
+    fork.record(fork.lists, st);
     stage(c, 2, st);
     xr_launch_pairs(w, ff->d, st);
     launches += 2;
+    fork.record(fork.pairs, st);
     stage(c, 3, st);
     if (qteam > 0) cudaMemcpyAsync(c->qmap, c->h_qmap_p, sizeof(int4) * qteam, cudaMemcpyHostToDevice, st);
     if (nlist > 0) cudaMemcpyAsync(c->qsmall, c->h_qsmall_p, sizeof(int) * nlist, cudaMemcpyHostToDevice, st);
     if (int le = launch_qeq(false)) return le;
     launches += (qcluster ? qbig > 0 : qteam > 0) ? 2 : 1;  // the teams' row splits, then the solver
+    if (fork.on) {  // issued before an adjoint solve, beside both
+      xr_launch_bond_orders(w, ff->d, fork);
+      xr_launch_bonded(w, ff->d, fork);
+    }
     stage(c, 4, st);
     const bool qeq_grad = w.pgrad && (flags & XR_FLAG_QEQ_GRADIENT);
     if (w.full_derivative || qeq_grad) {
@@ -1204,22 +1209,23 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
       xr_launch_charge_response(w, ff->d, st, 0);
       if (int le = launch_qeq(true)) return le;
       launches += (qcluster ? qbig > 0 : qteam > 0) ? 4 : 3;
-      if (w.full_derivative) {
-        xr_launch_charge_response(w, ff->d, st, 1);
-        launches += 1;
-      }
       if (qeq_grad) {
         xr_launch_qeq_param_gradient(w, ff->d, st);
         launches += 1;
       }
     }
     stage(c, 5, st);
-    xr_launch_bond_orders(w, ff->d, st);
+    if (!fork.on) xr_launch_bond_orders(w, ff->d, fork);
     launches += 3;
     stage(c, 6, st);
-    xr_launch_bonded(w, ff->d, st);
+    if (!fork.on) xr_launch_bonded(w, ff->d, fork);
     launches += 13;
     stage(c, 7, st);
+    fork.wait(st, fork.done);
+    if (w.full_derivative) {  // adds to the pairs' radial terms, as the bond-order chain does
+      xr_launch_charge_response(w, ff->d, st, 1);
+      launches += 1;
+    }
     xr_launch_forces(w, ff->d, st);
     launches += 1;
     xr_launch_reduce(w, ff->d, st);
@@ -1289,7 +1295,10 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     }
   }
   if (!done)
-    if (int le = sequence()) return cuda_fail(c, (cudaError_t)le, "launch");
+    if (int le = sequence()) {
+      for (cudaStream_t s : c->side) cudaStreamSynchronize(s);  // not joined: nothing may run on past the call
+      return cuda_fail(c, (cudaError_t)le, "launch");
+    }
   // Results: the per-atom values (k_pack, or the caller's device arrays), then energies, properties,
   // counters, QEq iterations and scans (k_gather_tail) into the result block, where k_bond_export has
   // written the exported bonds (at most nB records); one copy brings the block back, and the call
@@ -1697,9 +1706,15 @@ int xr_ctx_create(int device, void* stream, xr_ctx** out) {
   if (stream) {
     c->stream = (cudaStream_t)stream;
   } else {
-    cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
+    // ahead of the side streams: a QEq solve that needs whole SMs is placed before their small blocks
+    int least = 0, greatest = 0;
+    cudaDeviceGetStreamPriorityRange(&least, &greatest);
+    cudaStreamCreateWithPriority(&c->stream, cudaStreamNonBlocking, greatest);
     c->own_stream = true;
   }
+  bool made = c->stream != nullptr || stream != nullptr;
+  for (cudaStream_t& s : c->side) made = made && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
+  for (cudaEvent_t& v : c->fork_ev) made = made && cudaEventCreateWithFlags(&v, cudaEventDisableTiming) == cudaSuccess;
   cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device);
   c->coop_per_sm = xr_qeq_coop_blocks_per_sm();
   c->max_clusters = xr_qeq_max_clusters(kQeqClusterSingle);
@@ -1707,7 +1722,7 @@ int xr_ctx_create(int device, void* stream, xr_ctx** out) {
   int coop_ok = 0;
   cudaDeviceGetAttribute(&coop_ok, cudaDevAttrCooperativeLaunch, device);
   if (!coop_ok) c->coop_per_sm = 0;
-  bool ok = cudaMalloc((void**)&c->status, sizeof(int)) == cudaSuccess &&
+  bool ok = made && cudaMalloc((void**)&c->status, sizeof(int)) == cudaSuccess &&
             cudaMalloc((void**)&c->counts, 8 * sizeof(int)) == cudaSuccess &&
             cudaMalloc((void**)&c->barrier, (kQeqBlocks + 1) * sizeof(unsigned)) == cudaSuccess &&
             cudaMalloc((void**)&c->qmap, kQeqBlocks * sizeof(int4)) == cudaSuccess &&
@@ -1726,6 +1741,8 @@ void xr_ctx_destroy(xr_ctx* c) {
   if (!c) return;
   cudaSetDevice(c->device);
   if (c->stream) cudaStreamSynchronize(c->stream);
+  for (cudaStream_t s : c->side)  // joined by every call; not by one that failed half way
+    if (s) cudaStreamSynchronize(s);
   for (auto& e : c->gcache) cudaGraphExecDestroy(e.second.exec);
   void* bufs[] = {c->x, c->type, c->sys_of, c->wrap, c->xw, c->fw, c->cnt, c->a_fwd, c->a_adj, c->a_e, c->q, c->f,
                   c->qwork, c->outbuf, c->edge, c->edge_pair, c->edge_dbslot, c->hval, c->qch, c->qcj, c->pair_edge, c->pair_i,
@@ -1746,6 +1763,10 @@ void xr_ctx_destroy(xr_ctx* c) {
   if (c->h_small) cudaFreeHost(c->h_small);
   for (int k = 0; k <= xr_ctx::kStages; ++k)
     if (c->ev[k]) cudaEventDestroy(c->ev[k]);
+  for (cudaEvent_t v : c->fork_ev)
+    if (v) cudaEventDestroy(v);
+  for (cudaStream_t s : c->side)
+    if (s) cudaStreamDestroy(s);
   if (c->own_stream && c->stream) cudaStreamDestroy(c->stream);
   delete c;
 }

@@ -32,6 +32,10 @@ __global__ void k_prep(XrWork w) {
       *w.bx_count = 0;
     }
     if (a < w.S) w.qiters[a] = 0;
+    // what the energy kernels only add to: the gradient and four adjoints per atom (a bond's accumulators
+    // and energies are zeroed where its order is formed)
+    for (int k = 0; k < 3; ++k) w.f[3 * (size_t)a + k] = 0.0;
+    for (int k = AJ_TOTAL; k <= AJ_SBO2; ++k) w.a_adj[(size_t)k * w.A + a] = 0.0;
     w.qb_first[a] = 0x7fffffff;
     w.qb_last[a] = -1;
   }
@@ -663,14 +667,45 @@ __global__ void k_scan_apply(int* base, int L, const int* block_sums, int nblock
   }
 }
 
+// The whole scan of one array by one block, tile after tile: for arrays of a few tiles, where the three
+// kernels above are three launches of a few microseconds.
+constexpr int kScanOneTiles = 4;
+__global__ void k_scan_one(int* base, int L, int* totals) {
+  __shared__ int smem[33];
+  int* a = base + (size_t)blockIdx.x * L;
+  int carry = 0;
+  for (int b0 = 0; b0 < L; b0 += kScanTile) {
+    const int first = b0 + threadIdx.x * kScanPer;
+    int v[kScanPer];
+    int s = 0;
+    for (int t = 0; t < kScanPer; ++t) {
+      v[t] = (first + t < L) ? a[first + t] : 0;
+      s += v[t];
+    }
+    int total;
+    int ex = block_excl_scan(s, smem, &total) + carry;
+    for (int t = 0; t < kScanPer; ++t) {
+      if (first + t < L) a[first + t] = ex;
+      ex += v[t];
+    }
+    carry += total;
+  }
+  if (threadIdx.x == 0) totals[blockIdx.x] = carry;
+}
+
 // Exclusive scans in place of `narrays` arrays of length L laid out one after another (the last
 // slot of each holds 0 on entry and the total on exit); totals[k] receives each total. block_sums
-// needs narrays * ceil(L / kScanTile) ints.
-void scan_arrays(int* base, int L, int narrays, int* block_sums, int* totals, cudaStream_t st) {
+// needs narrays * ceil(L / kScanTile) ints. Returns the kernels launched.
+int scan_arrays(int* base, int L, int narrays, int* block_sums, int* totals, cudaStream_t st) {
   const int nblocks = (L + kScanTile - 1) / kScanTile;
+  if (nblocks <= kScanOneTiles) {
+    k_scan_one<<<narrays, kScanThreads, 0, st>>>(base, L, totals);
+    return 1;
+  }
   k_scan_blocks<<<dim3(nblocks, narrays), kScanThreads, 0, st>>>(base, L, block_sums, nblocks);
   k_scan_sums<<<narrays, kScanThreads, 0, st>>>(block_sums, nblocks, totals);
   k_scan_apply<<<dim3(nblocks, narrays), kScanThreads, 0, st>>>(base, L, block_sums, nblocks);
+  return 3;
 }
 
 }  // namespace
@@ -693,19 +728,19 @@ void xr_launch_rows(const XrWork& w, cudaStream_t st) {
 }
 
 // Needs w.red to hold at least 4 * ceil((A+1)/4096) ints.
-void xr_launch_scan(const XrWork& w, cudaStream_t st) {
-  scan_arrays(w.cnt, w.A + 1, 4, reinterpret_cast<int*>(w.red), w.counts, st);
+int xr_launch_scan(const XrWork& w, cudaStream_t st) {
+  return scan_arrays(w.cnt, w.A + 1, 4, reinterpret_cast<int*>(w.red), w.counts, st);
 }
 
-void xr_launch_candidates(const XrWork& w, bool fill, cudaStream_t st) {
+int xr_launch_candidates(const XrWork& w, bool fill, cudaStream_t st) {
   const int warps_per_block = 8;
   const int blocks = (w.A + warps_per_block - 1) / warps_per_block;
   if (fill) {
     k_candidates<true><<<blocks, 32 * warps_per_block, 0, st>>>(w);
-  } else {
-    k_candidates<false><<<blocks, 32 * warps_per_block, 0, st>>>(w);
-    scan_arrays(w.cand_cnt, w.A + 1, 1, reinterpret_cast<int*>(w.red), w.counts + 5, st);
+    return 1;
   }
+  k_candidates<false><<<blocks, 32 * warps_per_block, 0, st>>>(w);
+  return 1 + scan_arrays(w.cand_cnt, w.A + 1, 1, reinterpret_cast<int*>(w.red), w.counts + 5, st);
 }
 
 void xr_launch_filter(const XrWork& w, bool fill, cudaStream_t st) {
@@ -717,22 +752,23 @@ void xr_launch_filter(const XrWork& w, bool fill, cudaStream_t st) {
     k_filter<false><<<blocks, 32 * warps_per_block, 0, st>>>(w);
 }
 
-void xr_launch_cells(const XrWork& w, cudaStream_t st) {
+int xr_launch_cells(const XrWork& w, cudaStream_t st) {
   cudaMemsetAsync(w.cell_cnt, 0, sizeof(int) * ((size_t)w.ncells + 1), st);
   k_cell_count<<<(w.A + 255) / 256, 256, 0, st>>>(w);
-  scan_arrays(w.cell_cnt, w.ncells + 1, 1, reinterpret_cast<int*>(w.red), w.counts + 7, st);
+  const int scans = scan_arrays(w.cell_cnt, w.ncells + 1, 1, reinterpret_cast<int*>(w.red), w.counts + 7, st);
   k_cell_fill<<<(w.A + 255) / 256, 256, 0, st>>>(w);
+  return 2 + scans;
 }
 
-void xr_launch_cell_candidates(const XrWork& w, bool fill, cudaStream_t st) {
+int xr_launch_cell_candidates(const XrWork& w, bool fill, cudaStream_t st) {
   const int warps_per_block = 8;
   const int blocks = (w.A + warps_per_block - 1) / warps_per_block;
   if (fill) {
     k_cell_candidates<true><<<blocks, 32 * warps_per_block, 0, st>>>(w);
-  } else {
-    k_cell_candidates<false><<<blocks, 32 * warps_per_block, 0, st>>>(w);
-    scan_arrays(w.cand_cnt, w.A + 1, 1, reinterpret_cast<int*>(w.red), w.counts + 5, st);
+    return 1;
   }
+  k_cell_candidates<false><<<blocks, 32 * warps_per_block, 0, st>>>(w);
+  return 1 + scan_arrays(w.cand_cnt, w.A + 1, 1, reinterpret_cast<int*>(w.red), w.counts + 5, st);
 }
 
 void xr_launch_row_sort(const XrWork& w, int max_row, cudaStream_t st) {
