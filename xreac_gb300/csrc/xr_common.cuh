@@ -224,7 +224,9 @@ struct XrWork {
   // charges and forces
   double* q;
   const double* qguess;       // [A] initial QEq charges of systems with has_guess (sum = total charge)
-  int* qiters;                // [S] QEq conjugate-gradient iterations of each system
+  int* qiters;                // [S] QEq iterations of each system: conjugate-gradient ones, or the direct solver's refinement steps
+  int* qretry;                // [4 + 2 S] systems the direct solver leaves to CG: their number and the next one to take, for
+                              // the charges and for the adjoint solve, then the two lists
   double* qrhs;               // [A] adjoint QEq right-hand side (-dE/dq), full-derivative forces
   double* qadj;               // [A] adjoint QEq solution lambda (sum lambda = 0 per system)
   // Force-field parameter gradient dE/dtheta (null unless requested), summed over the batch:

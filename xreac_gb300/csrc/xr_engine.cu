@@ -15,6 +15,7 @@
 #include "xr_common.cuh"
 #include "xr_describe.h"
 #include "xr_lists.h"
+#include "xr_qeq_direct.h"
 #include "xreac_gb300.h"
 
 namespace {
@@ -100,8 +101,9 @@ struct xr_ctx {
   static constexpr size_t kGraphSeen = 4096;
   int last_graph = 0;  // of the last call: 0 launched directly, 1 recorded, 2 replayed
   // Side streams and events of the launch sequence (XrFork).
-  cudaStream_t side[3] = {};
-  cudaEvent_t fork_ev[7] = {};
+  cudaStream_t side[5] = {};     // bonded, torsions, hydrogen bonds; direct QEq solves beside CG ones, their small class
+  cudaEvent_t fork_ev[10] = {};
+  bool qeq_direct = false;       // the direct QEq solver fits the device's shared memory
   // Cell list (xr_ctx_set_cell_list): 0 chooses per call, 1 always, -1 never.
   int cell_mode = 0;
   int* atom_cell = nullptr;
@@ -133,6 +135,8 @@ struct xr_ctx {
   long long h2d_bytes = 0, d2h_bytes = 0;  // host<->device bytes moved by the last evaluation
   int qeq_iterations = 0;                   // CG iterations of the last evaluation (largest system)
   long long list_sizes[6] = {};             // edges, pairs, bond candidates, bond rows, active bonds, middles
+  int* qretry = nullptr;                    // [4 + 2 S] systems the direct solver left to CG (XrWork::qretry)
+  size_t cqretry = 0;
   int* qiters = nullptr;                    // [S] per-system iterations (device)
   size_t cqiters = 0;
   std::vector<int> h_qiters;
@@ -347,6 +351,7 @@ bool ensure_atoms(xr_ctx* c, int A, int S) {
   GROW(qb_last, A);
   GROW(qsmall, S);
   GROW(qiters, S);
+  GROW(qretry, 4 + 2 * (size_t)S);
   GROW(sys, S);
   GROW(qsplit, 9 * (size_t)S + 2 * (size_t)kQeqBlocks + 9);  // cluster teams' splits, or two per grid-team block
   GROW(energy, 16 * (size_t)S);
@@ -501,6 +506,7 @@ void attach_lists(xr_ctx* c, XrWork& w) {
   w.qrhs = c->qrhs;
   w.qadj = c->qadj;
   w.qiters = c->qiters;
+  w.qretry = c->qretry;
   w.mlist = c->mlist;
 }
 
@@ -677,11 +683,11 @@ constexpr int kQeqSmall = 160;
 constexpr int kQeqTeamRows = XR_QEQ_TEAM_ROWS;  // rows per block of a grid-wide team (a multiple of 32)
 constexpr int kQeqBatchBlock = 1024;
 
-void plan_qeq(xr_ctx* c, const xr_system* sys, int nsys, int* nblocks, int* nteam, int* nsmall) {
+void plan_qeq(xr_ctx* c, const xr_system* sys, int nsys, const std::vector<int>& ids, int* nblocks, int* nteam, int* nsmall) {
   const int budget = std::min(c->nsm * c->coop_per_sm, kQeqBlocks);
   const int team_above = nsys > 1 ? kQeqBatchBlock : kQeqSmall;
   std::vector<int> large, small;
-  for (int s = 0; s < nsys; ++s) (sys[s].natoms > team_above ? large : small).push_back(s);
+  for (int s : ids) (sys[s].natoms > team_above ? large : small).push_back(s);
   std::sort(large.begin(), large.end(), [&](int a, int b) { return sys[a].natoms > sys[b].natoms; });
   std::vector<int> team(large.size());
   for (;;) {
@@ -724,13 +730,14 @@ void plan_qeq(xr_ctx* c, const xr_system* sys, int nsys, int* nblocks, int* ntea
 // each largest first.
 constexpr int kQeqClusterMax = 640;
 
-bool plan_qeq_cluster(xr_ctx* c, const xr_system* sys, int nsys, int* csize, int* nblocks, int* nbig, int* nsmall) {
+bool plan_qeq_cluster(xr_ctx* c, const xr_system* sys, int nsys, const std::vector<int>& ids, int* csize, int* nblocks, int* nbig,
+                      int* nsmall) {
   *csize = nsys > 1 ? kQeqClusterBatch : kQeqClusterSingle;
   if ((nsys > 1 ? c->max_clusters_batch : c->max_clusters) < 1) return false;
   const int cs = *csize;
   const int limit = nsys > 1 ? kQeqBatchBlock : kQeqClusterMax;
   std::vector<int> big, small;
-  for (int s = 0; s < nsys; ++s) {
+  for (int s : ids) {
     if (sys[s].natoms > limit) return false;
     (sys[s].natoms > kQeqSmall ? big : small).push_back(s);
   }
@@ -744,6 +751,23 @@ bool plan_qeq_cluster(xr_ctx* c, const xr_system* sys, int nsys, int* csize, int
   c->h_qsmall.assign(big.begin(), big.end());
   c->h_qsmall.insert(c->h_qsmall.end(), small.begin(), small.end());
   return true;
+}
+
+// The systems small enough for the direct solver (xr_qeq_direct.cu), largest first, and the others
+// (for the CG plans). A caller that bounds the CG iterations, or the test that makes a
+// team wait run out, gets the CG solver whose iterations and waits those are.
+constexpr int kQeqDirectIterations = 400;
+
+void plan_qeq_direct(const xr_ctx* c, const xr_system* sys, int nsys, std::vector<int>& large, std::vector<int>& small,
+                     std::vector<int>& rest) {
+  const bool on = c->qeq_direct && c->cg_max >= kQeqDirectIterations && c->wait_polls == 0 && c->wait_fail_at == 0;
+  for (int s = 0; s < nsys; ++s) {
+    const int n = sys[s].natoms;
+    (!on || n > kQeqDirectMax ? rest : n > kQeqDirectSmall ? large : small).push_back(s);
+  }
+  auto larger = [&](int a, int b) { return sys[a].natoms > sys[b].natoms; };
+  std::sort(large.begin(), large.end(), larger);
+  std::sort(small.begin(), small.end(), larger);
 }
 
 // Whether the kept skin list serves this call: the same systems (atom counts, types, pbc, cells) at
@@ -1155,10 +1179,17 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
   // plan (its tables go through pinned buffers that a replay copies again) and the bond export.
   int qblocks = 0, qteam = 0, qsmall = 0, qbig = 0, qcsize = 0, nlist = 0;
   bool qcluster = false;
+  std::vector<int> qdl, qds, qrest;  // direct solves (two classes), and the systems of the CG solvers
   if (c->coop_per_sm > 0) {
-    qcluster = plan_qeq_cluster(c, sys, nsys, &qcsize, &qblocks, &qbig, &qsmall);
-    if (!qcluster) plan_qeq(c, sys, nsys, &qblocks, &qteam, &qsmall);
-    nlist = qbig + qsmall;
+    plan_qeq_direct(c, sys, nsys, qdl, qds, qrest);
+    c->h_qsmall.clear();
+    if (!qrest.empty()) {
+      qcluster = plan_qeq_cluster(c, sys, nsys, qrest, &qcsize, &qblocks, &qbig, &qsmall);
+      if (!qcluster) plan_qeq(c, sys, nsys, qrest, &qblocks, &qteam, &qsmall);
+    }
+    c->h_qsmall.insert(c->h_qsmall.end(), qdl.begin(), qdl.end());
+    c->h_qsmall.insert(c->h_qsmall.end(), qds.begin(), qds.end());
+    nlist = (int)c->h_qsmall.size();
     if (!host_grow(&c->h_qmap_p, &c->ch_qmap_p, (size_t)std::max(qteam, 1)) ||
         !host_grow(&c->h_qsmall_p, &c->ch_qsmall_p, (size_t)std::max(nlist, 1)))
       return cuda_fail(c, cudaErrorMemoryAllocation, "allocation");
@@ -1170,13 +1201,47 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
   if (!grow(c, &c->outbuf, &c->coutbuf, RL.end) || !host_grow(&c->h_out, &c->ch_out, RL.end))
     return cuda_fail(c, cudaErrorMemoryAllocation, "result block");
   XrBondRecord* const bx_rec = reinterpret_cast<XrBondRecord*>(c->outbuf + RL.bonds);
-  auto launch_qeq = [&](bool adjoint) {
-    return qcluster ? xr_launch_qeq_cluster(w, ff->d, st, qcsize, qblocks, c->qsmall, qbig, qsmall, adjoint)
-                    : xr_launch_qeq(w, ff->d, st, qblocks, c->qmap, qteam, c->qsmall, qsmall, adjoint);
-  };
   const bool forked = !c->profile;
   const XrFork fork = {forked, st, forked ? c->side[0] : st, forked ? c->side[1] : st, forked ? c->side[2] : st,
                        c->fork_ev[0], c->fork_ev[1], c->fork_ev[2], c->fork_ev[3], c->fork_ev[4], c->fork_ev[5], c->fork_ev[6]};
+  // The charges: the CG solvers on the call's stream, direct solves beside them, then what those left
+  // to CG. (The direct solves' launches come second: a CG team needs whole SMs.)
+  const int ndl = (int)qdl.size(), nds = (int)qds.size(), nd = ndl + nds;
+  const int largest_dl = ndl ? sys[qdl[0]].natoms : 0, largest_ds = nds ? sys[qds[0]].natoms : 0;
+  auto launch_qeq = [&](bool adjoint) -> int {
+    const bool beside = fork.on && !qrest.empty() && nd > 0;
+    const cudaStream_t sd = beside ? c->side[3] : st;
+    const bool apart = fork.on && ndl > 0 && nds > 0;  // the two classes of direct solves
+    const cudaStream_t ss = apart ? c->side[4] : sd;
+    if (beside || apart) {
+      cudaEventRecord(c->fork_ev[7], st);
+      if (beside) cudaStreamWaitEvent(sd, c->fork_ev[7], 0);
+      if (apart) cudaStreamWaitEvent(ss, c->fork_ev[7], 0);
+    }
+    if (!qrest.empty() || nd == 0) {
+      const int le = qcluster ? xr_launch_qeq_cluster(w, ff->d, st, qcsize, qblocks, c->qsmall, qbig, qsmall, adjoint)
+                              : xr_launch_qeq(w, ff->d, st, qblocks, c->qmap, qteam, c->qsmall, qsmall, adjoint);
+      launches += (qcluster ? qbig > 0 : qteam > 0) ? 2 : 1;  // the teams' row splits, then the solver
+      if (le) return le;
+    }
+    if (nd == 0) return 0;
+    const int* const dlist = c->qsmall + (nlist - nd);
+    if (ndl > 0)
+      if (int le = xr_launch_qeq_direct(w, ff->d, sd, dlist, ndl, largest_dl, adjoint)) return le;
+    if (nds > 0)
+      if (int le = xr_launch_qeq_direct(w, ff->d, ss, dlist + ndl, nds, largest_ds, adjoint)) return le;
+    if (apart) {
+      cudaEventRecord(c->fork_ev[8], ss);
+      cudaStreamWaitEvent(sd, c->fork_ev[8], 0);
+    }
+    if (int le = xr_launch_qeq_retry(w, ff->d, sd, std::min(nd, c->nsm), adjoint)) return le;
+    launches += (ndl > 0) + (nds > 0) + 1;
+    if (beside) {
+      cudaEventRecord(c->fork_ev[9], sd);
+      cudaStreamWaitEvent(st, c->fork_ev[9], 0);
+    }
+    return 0;
+  };
   // The launch sequence: rows, pairs, QEq, bond orders, bonded terms, Coulomb energy and forces,
   // reductions, bond export. Returns 0 or a CUDA error of a launch.
   auto sequence = [&]() -> int {
@@ -1196,7 +1261,6 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     if (qteam > 0) cudaMemcpyAsync(c->qmap, c->h_qmap_p, sizeof(int4) * qteam, cudaMemcpyHostToDevice, st);
     if (nlist > 0) cudaMemcpyAsync(c->qsmall, c->h_qsmall_p, sizeof(int) * nlist, cudaMemcpyHostToDevice, st);
     if (int le = launch_qeq(false)) return le;
-    launches += (qcluster ? qbig > 0 : qteam > 0) ? 2 : 1;  // the teams' row splits, then the solver
     if (fork.on) {  // issued before an adjoint solve, beside both
       xr_launch_bond_orders(w, ff->d, fork);
       xr_launch_bonded(w, ff->d, fork);
@@ -1208,7 +1272,7 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
       // and the QEq parameters' gradient
       xr_launch_charge_response(w, ff->d, st, 0);
       if (int le = launch_qeq(true)) return le;
-      launches += (qcluster ? qbig > 0 : qteam > 0) ? 4 : 3;
+      launches += 2;
       if (qeq_grad) {
         xr_launch_qeq_param_gradient(w, ff->d, st);
         launches += 1;
@@ -1245,7 +1309,7 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
   bool done = false;
   if (c->graphs && !c->profile && qteam == 0) {
     const int ints[] = {(int)mode, qcluster ? 1 : 0, qcsize, qblocks, qteam, qsmall, qbig, nlist, nE > 0, nP > 0, nB > 0,
-                        (int)flags};
+                        (int)flags, ndl, nds, largest_dl, largest_ds};
     const void* ptrs[] = {c->h_qmap_p, c->h_qsmall_p, c->qmap, c->qsmall, bx_rec, c->bx_count, c->outbuf};
     const int nptrs = (int)(sizeof(ptrs) / sizeof(ptrs[0]));
     const std::vector<unsigned char> kv = launch_key(w, ff->d, ints, (int)(sizeof(ints) / sizeof(int)), ptrs, nptrs);
@@ -1717,6 +1781,7 @@ int xr_ctx_create(int device, void* stream, xr_ctx** out) {
   for (cudaEvent_t& v : c->fork_ev) made = made && cudaEventCreateWithFlags(&v, cudaEventDisableTiming) == cudaSuccess;
   cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device);
   c->coop_per_sm = xr_qeq_coop_blocks_per_sm();
+  c->qeq_direct = xr_qeq_direct_ready();
   c->max_clusters = xr_qeq_max_clusters(kQeqClusterSingle);
   c->max_clusters_batch = xr_qeq_max_clusters(kQeqClusterBatch);
   int coop_ok = 0;
@@ -1748,7 +1813,7 @@ void xr_ctx_destroy(xr_ctx* c) {
                   c->qwork, c->outbuf, c->edge, c->edge_pair, c->edge_dbslot, c->hval, c->qch, c->qcj, c->pair_edge, c->pair_i,
                   c->pair_bond, c->p_r, c->p_shield, c->p_dshield, c->p_g, c->p_evdw, c->p_ecoul, c->bond_pair,
                   c->bond_i, c->bond_j, c->b_r, c->b_v, c->b_fwd, c->b_adj, c->b_e, c->dbrow, c->sys, c->energy,
-                  c->props, c->status, c->counts, c->barrier, c->qmap, c->qsmall, c->qiters, c->red, c->qguess, c->qrhs, c->qadj, c->pgrad, c->bx_count,
+                  c->props, c->status, c->counts, c->barrier, c->qmap, c->qsmall, c->qiters, c->qretry, c->red, c->qguess, c->qrhs, c->qadj, c->pgrad, c->bx_count,
                   c->arow, c->nact, c->nzrow, c->nnz, c->qb_first, c->qb_last, c->chunk_part, c->mids, c->nmids, c->mlist,
                   c->cand_cnt, c->cand_edge, c->sys_list, c->atom_cell, c->atom_slot, c->cell_cnt, c->cell_atoms,
                   c->mid_tiles, c->qsplit};
@@ -2011,7 +2076,7 @@ long long xr_footprint_bytes(int atoms, int systems, long long edges, long long 
   // the buffers of ensure_atoms, ensure_lists and xr_ctx_reserve, per element
   const long long per_atom = sizeof(double4_32a) + 2 * sizeof(int) + sizeof(int4) + 2 * sizeof(float4) + 4 * sizeof(int) +
                              (AF_N + AJ_N + 8 + 4 + 3 + XR_QW_N + 8) * sizeof(double) + 8 * sizeof(int);
-  const long long per_system = sizeof(int2) + 3 * sizeof(int) + sizeof(XrSystem) + 20 * sizeof(double);
+  const long long per_system = sizeof(int2) + 5 * sizeof(int) + sizeof(XrSystem) + 20 * sizeof(double);
   const long long per_edge = sizeof(int2) + 2 * sizeof(int) + sizeof(double) + sizeof(float) + sizeof(unsigned short);
   const long long per_pair = 3 * sizeof(int) + 6 * sizeof(double);
   const long long per_bond = kBondBytes + 32;  // + the exported-bond record of the result block

@@ -15,6 +15,7 @@
 
 #include "xr_common.cuh"
 #include "xr_dfloat.cuh"
+#include "xr_qeq_direct.h"
 #include "xreac_gb300.h"
 
 namespace {
@@ -2219,6 +2220,16 @@ __global__ void __launch_bounds__(1024, 1) k_qeq_cluster(XrWork w, XrFF ff, cons
   cluster_barrier_all();  // no block leaves while a peer may still write into its shared memory
 }
 
+// The systems that the direct solver left (usually none), one block each.
+__global__ void __launch_bounds__(1024, 1) k_qeq_retry(XrWork w, XrFF ff, int adjoint) {
+  __shared__ QeqShared sh;
+  extern __shared__ __align__(16) unsigned char dyn[];
+  int* const retry = w.qretry + (adjoint ? 2 : 0);
+  const int count = retry[0];
+  if (count == 0) return;
+  qeq_small_systems(w, ff, w.qretry + 4 + (adjoint ? w.S : 0), count, reinterpret_cast<unsigned*>(retry + 1), adjoint, sh, dyn);
+}
+
 // Fallback without cooperative launch: one block per system, no shared-memory row cache.
 __global__ void __launch_bounds__(1024, 1) k_qeq_block(XrWork w, XrFF ff, int adjoint) {
   __shared__ QeqShared sh;
@@ -2461,6 +2472,7 @@ void xr_launch_pairs(const XrWork& w, const XrFF& ff, cudaStream_t st) {
 
 int xr_qeq_coop_blocks_per_sm() {
   cudaFuncSetAttribute(k_qeq_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, kQeqMaxDyn);
+  cudaFuncSetAttribute(k_qeq_retry, cudaFuncAttributeMaxDynamicSharedMemorySize, kQeqMaxDyn);
   int nb = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_qeq_grid, 1024, kQeqMaxDyn);
   return nb;
@@ -2531,6 +2543,11 @@ int xr_launch_qeq(const XrWork& w, const XrFF& ff, cudaStream_t st, int nblocks,
     return (int)e;
   }
   k_qeq_block<<<w.S, 1024, 0, st>>>(w, ff, adj);
+  return (int)cudaGetLastError();
+}
+
+int xr_launch_qeq_retry(const XrWork& w, const XrFF& ff, cudaStream_t st, int count, bool adjoint) {
+  k_qeq_retry<<<count, 1024, kQeqMaxDyn, st>>>(w, ff, adjoint ? 1 : 0);
   return (int)cudaGetLastError();
 }
 

@@ -30,6 +30,7 @@ __global__ void k_prep(XrWork w) {
       w.nmids[0] = 0;
       w.nmids[1] = 0;
       *w.bx_count = 0;
+      for (int k = 0; k < 4; ++k) w.qretry[k] = 0;
     }
     if (a < w.S) w.qiters[a] = 0;
     // what the energy kernels only add to: the gradient and four adjoints per atom (a bond's accumulators
