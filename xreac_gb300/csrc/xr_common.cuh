@@ -133,6 +133,13 @@ struct XrFF {
   const double* hbond;        // [H][4]
 };
 
+// One exported bond: (bond id, i, j, image code) and its corrected order.
+struct __align__(16) XrBondRecord {
+  int4 meta;
+  double bo;
+  double pad;
+};
+
 // Device work state of one batch. Sizes: A atoms, E edges, P pairs, B bonds, D = 2B bond-row
 // entries, S systems. Capacities (cap_*) are the allocated lengths; counts live on the device.
 struct XrWork {
@@ -214,7 +221,10 @@ struct XrWork {
   int* nnz;                   // [A] number of such entries per atom (every other entry has zero bond orders)
   int* mids;                  // [B] bonds with bo > 0.001 (torsion middles), compacted
   int* nmids;                 // device count of mids
-  int* mid_tiles;             // [ceil(cap_B / 128)] per-tile counts, then offsets, of the middles
+  // [ceil(cap_B / 128)] per 128-bond tile the number of torsion middles (low word) and of bonds to export
+  // (high word), then their offsets
+  unsigned long long* mid_tiles;
+  XrBondRecord* bx_rec;       // the exported bonds (nonzero corrected orders), in bond order, in the result block
   int* mlist;                 // [B] active bonds (uncorrected order passed the cut), in any order
   int* nmask;                 // length of mlist (device)
   // per-atom forward intermediates [AF_N][A] and adjoints [AJ_N][A] (structure of arrays)

@@ -192,7 +192,7 @@ struct xr_ctx {
   size_t cnnz = 0;
   int* mids = nullptr;
   int* nmids = nullptr;  // [2] torsion middles, active bonds
-  int* mid_tiles = nullptr;  // per 128-bond tile: middles counts, then offsets
+  unsigned long long* mid_tiles = nullptr;  // XrWork::mid_tiles
   size_t cmid_tiles = 0;
   int* qsplit = nullptr;     // row splits of the cluster teams' systems
   size_t cqsplit = 0;
@@ -254,8 +254,7 @@ struct xr_ctx {
   long long stage_calls = 0;
   // compact export of nonzero bonds: {bond, i, j, code} and bo
   int* bx_count = nullptr;
-  std::vector<int4> h_bx_meta;
-  std::vector<double> h_bx_bo;
+  std::vector<XrBondRecord> h_bx;  // the last call's exported bonds, in bond order
   // pinned host staging (every host<->device copy of a call is asynchronous from/to these)
   double4_32a* h_x = nullptr;
   size_t ch_x = 0;
@@ -510,15 +509,9 @@ void attach_lists(xr_ctx* c, XrWork& w) {
   w.mlist = c->mlist;
 }
 
-// One exported bond: (bond id, i, j, image code) and its corrected order.
-struct __align__(16) XrBondRecord {
-  int4 meta;
-  double bo;
-  double pad;
-};
-
 // The result block of a call, in doubles from the start of outbuf (device) and h_out (host): per-atom
-// values [8 A], energies [16 S], properties [4 S], the tail of ints (kTailInts counters, the systems'
+// values (forces [3 A], then charges, total bond orders, lone pairs and bond counts [A] each, as the caller's
+// arrays hold them), energies [16 S], properties [4 S], the tail of ints (kTailInts counters, the systems'
 // QEq iterations [S], the scans [4 (A + 1)]), then the exported bonds as 32-byte records. Kernels
 // write all of it, so one copy brings a call's results back.
 constexpr int kTailInts = 5;  // status, exported bonds, QEq iterations, torsion middles, active bonds
@@ -527,27 +520,13 @@ struct ResultLayout {
 };
 ResultLayout result_layout(int A, int nsys, long long nB) {
   ResultLayout L;
-  L.energy = 8 * (size_t)A;
+  L.energy = 7 * (size_t)A;
   L.props = L.energy + 16 * (size_t)nsys;
   L.tail = L.props + 4 * (size_t)nsys;
   const size_t tail_ints = kTailInts + (size_t)nsys + 4 * (size_t)(A + 1);
   L.bonds = (L.tail + (tail_ints + 1) / 2 + 3) / 4 * 4;
   L.end = L.bonds + 4 * (size_t)std::max<long long>(nB, 0);
   return L;
-}
-
-// Packs forces (-dE/dx), charges, total bond orders, lone pairs and bond counts per atom.
-__global__ void k_pack(XrWork w, double* out) {
-  const int a = blockIdx.x * blockDim.x + threadIdx.x;
-  if (a >= w.A) return;
-  out[8 * a + 0] = -w.f[3 * a + 0];
-  out[8 * a + 1] = -w.f[3 * a + 1];
-  out[8 * a + 2] = -w.f[3 * a + 2];
-  out[8 * a + 3] = w.q[a];
-  out[8 * a + 4] = w.a_fwd[(size_t)AF_TOTAL * w.A + a];
-  out[8 * a + 5] = w.a_fwd[(size_t)AF_NLP * w.A + a];
-  out[8 * a + 6] = w.a_fwd[(size_t)AF_COUNT30 * w.A + a];
-  out[8 * a + 7] = 0.0;
 }
 
 // Device-output variant for a single system: writes straight into the caller's arrays.
@@ -565,10 +544,20 @@ __global__ void k_unpack_device(XrWork w, double* forces, double* charges, doubl
   if (counts) counts[a] = (int)w.a_fwd[(size_t)AF_COUNT30 * w.A + a];
 }
 
-// Energies, properties and the tail of ints into the result block (its layout: result_layout), after
-// every other kernel of the call.
-__global__ void k_gather_tail(XrWork w, double* block, size_t energy_off, size_t tail_off) {
-  const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x;
+// The result block (its layout: result_layout) after every other kernel of the call: the per-atom values
+// (unless the caller's device arrays took them), energies, properties and the tail of ints.
+__global__ void k_results(XrWork w, double* block, int per_atom, size_t energy_off, size_t tail_off) {
+  const int t = blockIdx.x * blockDim.x + threadIdx.x, nt = gridDim.x * blockDim.x, A = w.A;
+  if (per_atom) {
+    for (int k = t; k < 3 * A; k += nt) block[k] = -w.f[k];
+    double* v = block + 3 * (size_t)A;
+    for (int k = t; k < A; k += nt) {
+      v[k] = w.q[k];
+      v[A + k] = w.a_fwd[(size_t)AF_TOTAL * A + k];
+      v[2 * (size_t)A + k] = w.a_fwd[(size_t)AF_NLP * A + k];
+      v[3 * (size_t)A + k] = w.a_fwd[(size_t)AF_COUNT30 * A + k];
+    }
+  }
   double* e = block + energy_off;
   for (int k = t; k < 20 * w.S; k += nt) e[k] = k < 16 * w.S ? w.energy[k] : w.props[k - 16 * w.S];
   int* ti = reinterpret_cast<int*>(block + tail_off);
@@ -581,7 +570,7 @@ __global__ void k_gather_tail(XrWork w, double* block, size_t energy_off, size_t
   }
   for (int k = t; k < w.S; k += nt) ti[kTailInts + k] = w.qiters[k];
   int* tc = ti + kTailInts + w.S;
-  const int nc = 4 * (w.A + 1);
+  const int nc = 4 * (A + 1);
   for (int k = t; k < nc; k += nt) tc[k] = w.cnt[k];
 }
 
@@ -589,30 +578,6 @@ __global__ void k_positions_from_device(const double* pos, double4_32a* x, int n
   const int a = blockIdx.x * blockDim.x + threadIdx.x;
   if (a >= n) return;
   x[a] = make_double4_32a(pos[3 * a], pos[3 * a + 1], pos[3 * a + 2], 0.0);
-}
-
-// Nonzero corrected bond orders, compacted with warp-aggregated atomics; the host restores bond order.
-__global__ void k_bond_export(XrWork w, XrBondRecord* rec, int* counter) {
-  const int nb = xr_num_bonds(w);
-  const int lane = threadIdx.x & 31;
-  for (int b0 = blockIdx.x * blockDim.x; b0 < nb; b0 += gridDim.x * blockDim.x) {  // uniform per block
-    const int b = b0 + threadIdx.x;
-    const double bo = b < nb ? w.b_fwd[(size_t)BF_BO * w.cap_B + b] : 0.0;
-    const bool keep = b < nb && bo != 0.0;
-    const unsigned m = __ballot_sync(0xffffffffu, keep);
-    int base = 0;
-    if (lane == 0 && m) base = atomicAdd(counter, __popc(m));
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (keep) {
-      const int slot = base + __popc(m & ((1u << lane) - 1u));
-      const int code = w.edge[w.pair_edge[w.bond_pair[b]]].y;
-      XrBondRecord r;
-      r.meta = make_int4(b, w.bond_i[b], w.bond_j[b], code);
-      r.bo = bo;
-      r.pad = 0.0;
-      rec[slot] = r;
-    }
-  }
 }
 
 void stage(xr_ctx* c, int k, cudaStream_t st) {
@@ -1200,7 +1165,7 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
   const ResultLayout RL = result_layout(A, nsys, nB);
   if (!grow(c, &c->outbuf, &c->coutbuf, RL.end) || !host_grow(&c->h_out, &c->ch_out, RL.end))
     return cuda_fail(c, cudaErrorMemoryAllocation, "result block");
-  XrBondRecord* const bx_rec = reinterpret_cast<XrBondRecord*>(c->outbuf + RL.bonds);
+  w.bx_rec = reinterpret_cast<XrBondRecord*>(c->outbuf + RL.bonds);
   const bool forked = !c->profile;
   const XrFork fork = {forked, st, forked ? c->side[0] : st, forked ? c->side[1] : st, forked ? c->side[2] : st,
                        c->fork_ev[0], c->fork_ev[1], c->fork_ev[2], c->fork_ev[3], c->fork_ev[4], c->fork_ev[5], c->fork_ev[6]};
@@ -1294,10 +1259,6 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     launches += 1;
     xr_launch_reduce(w, ff->d, st);
     launches += 2;
-    if (nB > 0) {  // (its counter was zeroed by k_prep)
-      k_bond_export<<<(nB + 255) / 256, 256, 0, st>>>(w, bx_rec, c->bx_count);
-      ++launches;
-    }
     return (int)cudaGetLastError();
   };
   // A sequence is recorded as a CUDA graph the second time its launch key occurs (a relaxation or MD
@@ -1310,7 +1271,7 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
   if (c->graphs && !c->profile && qteam == 0) {
     const int ints[] = {(int)mode, qcluster ? 1 : 0, qcsize, qblocks, qteam, qsmall, qbig, nlist, nE > 0, nP > 0, nB > 0,
                         (int)flags, ndl, nds, largest_dl, largest_ds};
-    const void* ptrs[] = {c->h_qmap_p, c->h_qsmall_p, c->qmap, c->qsmall, bx_rec, c->bx_count, c->outbuf};
+    const void* ptrs[] = {c->h_qmap_p, c->h_qsmall_p, c->qmap, c->qsmall, c->outbuf};
     const int nptrs = (int)(sizeof(ptrs) / sizeof(ptrs[0]));
     const std::vector<unsigned char> kv = launch_key(w, ff->d, ints, (int)(sizeof(ints) / sizeof(int)), ptrs, nptrs);
     const std::string key(reinterpret_cast<const char*>(kv.data()), kv.size());
@@ -1363,26 +1324,27 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
       for (cudaStream_t s : c->side) cudaStreamSynchronize(s);  // not joined: nothing may run on past the call
       return cuda_fail(c, (cudaError_t)le, "launch");
     }
-  // Results: the per-atom values (k_pack, or the caller's device arrays), then energies, properties,
-  // counters, QEq iterations and scans (k_gather_tail) into the result block, where k_bond_export has
-  // written the exported bonds (at most nB records); one copy brings the block back, and the call
-  // synchronises once more only at its end. The parameter gradient, when asked for, comes separately.
+  // Results: the per-atom values, energies, properties, counters, QEq iterations and scans (k_results) into
+  // the result block, where k_mid_fill has written the exported bonds; one copy brings the block back,
+  // with the records of kBondsPerAtom bonds per atom (a molecule's or a crystal's active bonds; the block
+  // has room for every candidate within 5 A, ten times as many), and the call synchronises once more only
+  // at its end, or again for records past those. The parameter gradient, when asked for, comes separately.
   if (dev_io) {
     const xr_result& r = out[0];
     k_unpack_device<<<(A + 255) / 256, 256, 0, st>>>(w, r.forces, r.charges, r.total_bond_orders, r.lone_pairs,
                                                     r.bond_counts);
-  } else {
-    k_pack<<<(A + 255) / 256, 256, 0, st>>>(w, c->outbuf);
+    ++launches;
   }
   {
-    const long long tail_n = 20ll * nsys + 4ll * (A + 1) + nsys;
-    const int gb = (int)std::min<long long>((tail_n + 255) / 256, 152 * 4);
-    k_gather_tail<<<gb, 256, 0, st>>>(w, c->outbuf, RL.energy, RL.tail);
+    const int gb = (int)std::min<long long>((20ll * nsys + 4ll * (A + 1) + 255) / 256, 152 * 4);
+    k_results<<<gb, 256, 0, st>>>(w, c->outbuf, dev_io ? 0 : 1, RL.energy, RL.tail);
+    ++launches;
   }
-  launches += 2;
+  constexpr int kBondsPerAtom = 4;
+  const int nx_first = (int)std::min<long long>(std::max(nB, 0), (long long)kBondsPerAtom * A + 64);
   {
     const size_t from = dev_io ? RL.energy : 0;
-    const size_t count = RL.bonds + 4 * (size_t)std::max(nB, 0) - from;
+    const size_t count = RL.bonds + 4 * (size_t)nx_first - from;
     cudaMemcpyAsync(c->h_out + from, c->outbuf + from, sizeof(double) * count, cudaMemcpyDeviceToHost, st);
     d2h += (long long)(sizeof(double) * count);
   }
@@ -1405,17 +1367,15 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
   const XrBondRecord* recs = reinterpret_cast<const XrBondRecord*>(c->h_out + RL.bonds);
   {
     const int nx = std::min(tail[1], std::max(nB, 0));
-    d2h += (sizeof(int4) + sizeof(double)) * (long long)nB;
-    // exported in arrival order; sorted by bond id (system, then pair order) for the exporters
-    std::vector<int> order(nx);
-    for (int k = 0; k < nx; ++k) order[k] = k;
-    std::sort(order.begin(), order.end(), [&](int a, int b) { return recs[a].meta.x < recs[b].meta.x; });
-    c->h_bx_meta.resize(nx);
-    c->h_bx_bo.resize(nx);
-    for (int k = 0; k < nx; ++k) {
-      c->h_bx_meta[k] = recs[order[k]].meta;
-      c->h_bx_bo[k] = recs[order[k]].bo;
+    if (nx > nx_first) {
+      const size_t from = RL.bonds + 4 * (size_t)nx_first, count = 4 * (size_t)(nx - nx_first);
+      if ((e = cudaMemcpyAsync(c->h_out + from, c->outbuf + from, sizeof(double) * count, cudaMemcpyDeviceToHost, st)) !=
+              cudaSuccess ||
+          (e = cudaStreamSynchronize(st)) != cudaSuccess)
+        return cuda_fail(c, e, "bond records");
+      d2h += (long long)(sizeof(double) * count);
     }
+    c->h_bx.assign(recs, recs + nx);
   }
   c->h_qiters.assign(tail + kTailInts, tail + kTailInts + nsys);
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(c, e, "kernel launch");
@@ -1447,25 +1407,19 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
   for (int s = 0; s < nsys; ++s) {
     const xr_result& r = out[s];
     const int n = sys[s].natoms;
-    const double* pa = c->h_out + 8 * (size_t)off;
     const double* pe = c->h_out + RL.energy + 16 * s;
     const double* pp = c->h_out + RL.props + 4 * s;
     if (r.energy)
       for (int k = 0; k < 15; ++k) r.energy[k] = pe[k];
     if (r.dipole)
       for (int k = 0; k < 3; ++k) r.dipole[k] = pp[k];
-    for (int a = 0; a < n; ++a) {
-      const double* v = pa + 8 * a;
-      if (r.forces) {
-        r.forces[3 * a + 0] = v[0];
-        r.forces[3 * a + 1] = v[1];
-        r.forces[3 * a + 2] = v[2];
-      }
-      if (r.charges) r.charges[a] = v[3];
-      if (r.total_bond_orders) r.total_bond_orders[a] = v[4];
-      if (r.lone_pairs) r.lone_pairs[a] = v[5];
-      if (r.bond_counts) r.bond_counts[a] = (int)v[6];
-    }
+    const double* v = c->h_out + 3 * (size_t)A + off;
+    if (r.forces) std::memcpy(r.forces, c->h_out + 3 * (size_t)off, sizeof(double) * 3 * n);
+    if (r.charges) std::memcpy(r.charges, v, sizeof(double) * n);
+    if (r.total_bond_orders) std::memcpy(r.total_bond_orders, v + A, sizeof(double) * n);
+    if (r.lone_pairs) std::memcpy(r.lone_pairs, v + 2 * (size_t)A, sizeof(double) * n);
+    if (r.bond_counts)
+      for (int a = 0; a < n; ++a) r.bond_counts[a] = (int)v[3 * (size_t)A + a];
     // the charge constraint check of src/xreac/calculator.py:153-154
     if (r.charges) {
       double sq = 0;
@@ -2018,21 +1972,21 @@ int xr_get_bonds(xr_ctx* c, int index, int* i, int* j, int* S, double* bo, long 
   const int a1 = index < 0 ? c->last_A : a0 + c->host_sys[index].natoms;
   const int b0 = c->host_cnt[2 * L + a0], b1 = c->host_cnt[2 * L + a1];
   // exported entries are sorted by bond id: the system's are one contiguous run
-  const auto& m = c->h_bx_meta;
-  const auto lo = std::lower_bound(m.begin(), m.end(), b0, [](const int4& v, int key) { return v.x < key; });
-  const auto hi = std::lower_bound(m.begin(), m.end(), b1, [](const int4& v, int key) { return v.x < key; });
+  const auto& m = c->h_bx;
+  const auto lo = std::lower_bound(m.begin(), m.end(), b0, [](const XrBondRecord& v, int key) { return v.meta.x < key; });
+  const auto hi = std::lower_bound(m.begin(), m.end(), b1, [](const XrBondRecord& v, int key) { return v.meta.x < key; });
   const long long n = hi - lo;
   *count = n;
   if (capacity < n || !i || !j || !S || !bo) return XR_OK;
   long long k = 0;
   for (auto it = lo; it != hi; ++it, ++k) {
-    const uint32_t code = (uint32_t)it->w;
-    i[k] = it->y - a0;
-    j[k] = it->z - a0;
+    const uint32_t code = (uint32_t)it->meta.w;
+    i[k] = it->meta.y - a0;
+    j[k] = it->meta.z - a0;
     S[3 * k + 0] = xr_sx(code);
     S[3 * k + 1] = xr_sy(code);
     S[3 * k + 2] = xr_sz(code);
-    bo[k] = c->h_bx_bo[it - m.begin()];
+    bo[k] = it->bo;
   }
   return XR_OK;
 }
