@@ -93,7 +93,7 @@ def build_host(force=False, verbose=False):
     if not force and not _stale(out, [src]):
         return out
     cxx = os.environ.get("CXX", "g++")
-    cmd = [cxx, "-O2", "-std=c++17", "-shared", "-fPIC", "-I", include, str(src), "-o", str(out)]
+    cmd = [cxx, "-O2", "-std=c++17", "-ffp-contract=off", "-shared", "-fPIC", "-I", include, str(src), "-o", str(out)]
     if verbose:
         print(" ".join(cmd), flush=True)
     try:

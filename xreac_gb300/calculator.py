@@ -18,7 +18,7 @@ from typing import NamedTuple
 import numpy as np
 
 from . import _native as nat
-from .geometry import (boundary, cell_repetitions, periodic_cell, validate_expansion_limit, validate_input,
+from .geometry import (ALL_PBC, boundary, cell_repetitions, periodic_cell, validate_expansion_limit, validate_input,
                        validate_total_charge)
 
 COMPONENTS = (
@@ -113,29 +113,32 @@ RELAX_SKIN = 0.3
 _BATCH_FIELDS = frozenset(("forces", "charges", "components", "total_bond_orders", "lone_pairs", "bond_counts",
                            "dipole", "bonds"))
 del Evaluation.bonds
+if _host is not None:  # the same access in native code
+    _host.set_components(COMPONENTS)
+    Evaluation.__getattr__ = _host.field
 
 
 class _BatchResults:
     """The result arrays of one ``xr_eval_batch`` call; the fields of its k-th system are views."""
 
-    __slots__ = ("energy", "forces", "per_atom", "counts", "dipole", "offsets", "bonds", "cut")
+    __slots__ = ("energy", "forces", "charges", "total_bond_orders", "lone_pairs", "_counts", "_counts64", "dipole",
+                 "offsets", "bonds", "cut")
 
     def __init__(self, energy, forces, per_atom, counts, dipole, offsets, bonds, cut):
-        self.energy, self.forces, self.per_atom, self.counts = energy, forces, per_atom, counts
+        self.energy, self.forces, self._counts, self._counts64 = energy, forces, counts, None
+        self.charges, self.total_bond_orders, self.lone_pairs = per_atom
         self.dipole, self.offsets, self.bonds, self.cut = dipole, offsets, bonds, cut
+
+    @property
+    def bond_counts(self):
+        if self._counts64 is None:
+            self._counts64 = self._counts.astype(np.int64)
+        return self._counts64
 
     def field(self, name, k):
         a0, a1 = self.offsets[k], self.offsets[k + 1]
-        if name == "forces":
-            return self.forces[a0:a1]
-        if name == "charges":
-            return self.per_atom[0, a0:a1]
-        if name == "total_bond_orders":
-            return self.per_atom[1, a0:a1]
-        if name == "lone_pairs":
-            return self.per_atom[2, a0:a1]
-        if name == "bond_counts":
-            return self.counts[a0:a1].astype(np.int64)
+        if name in ("forces", "charges", "total_bond_orders", "lone_pairs", "bond_counts"):
+            return getattr(self, name)[a0:a1]
         if name == "dipole":
             return self.dipole[k]
         if name == "bonds":
@@ -241,6 +244,15 @@ def _guess(initial_charges, n):
 
 def _is_carbon(ff):
     return np.array([s.upper() == "C" for s in ff.elements], dtype=np.int32)
+
+
+def _request_tuples(systems):
+    """``(symbols, positions, total_charge, cell, pbc, initial_charges)`` of keyword dicts."""
+    items = _host.items(systems) if _host is not None else None
+    if items is None:
+        items = [(s["symbols"], s["positions"], s.get("total_charge", 0), s.get("cell"), s.get("pbc"),
+                  s.get("initial_charges")) for s in systems]
+    return items
 
 
 class Calculator:
@@ -541,9 +553,7 @@ class Calculator:
         the atom-table rows ``(S, T, 24)`` as a fourth item. ``qeq``: see :meth:`parameter_gradient`."""
         sets = self._sets(parameter_sets, len(systems))
         flags_ = nat.XR_FLAG_PARAM_GRADIENT | (nat.XR_FLAG_QEQ_GRADIENT if qeq else 0)
-        results = self._evaluate_items([(s["symbols"], s["positions"], s.get("total_charge", 0), s.get("cell"),
-                                         s.get("pbc"), s.get("initial_charges")) for s in systems], full_derivative,
-                                       flags_, sets)
+        results = self._evaluate_items(_request_tuples(systems), full_derivative, flags_, sets)
         T = len(self.force_field.elements)
         if raw:
             np_, na, nat_ = T * T * 28, 7 * len(self._angle_rows), T * 24
@@ -584,9 +594,7 @@ class Calculator:
         :meth:`load_parameter_sets`.
         """
         sets = self._sets(parameter_sets, len(systems))
-        return self._evaluate_items([(s["symbols"], s["positions"], s.get("total_charge", 0), s.get("cell"),
-                                      s.get("pbc"), s.get("initial_charges")) for s in systems], full_derivative,
-                                    0, sets)
+        return self._evaluate_items(_request_tuples(systems), full_derivative, 0, sets)
 
     def _evaluate_items(self, items, full_derivative=False, extra_flags=0, sets=None):
         """``evaluate_many`` on tuples (symbols, positions, total_charge, cell, pbc, initial_charges)."""
@@ -641,13 +649,16 @@ class Calculator:
             types[a0:a1] = tk
             x[a0:a1] = xk
             flags_l[k], cells[k], reps[k] = fk, ck, rk
-        cutoff = None
+        cutoff = float(self.force_field.general[12])
         slow_set = set(slow)
-        for k, it in enumerate(items):
-            cell, pbc = it[3], it[4]
-            if k not in slow_set and not ((pbc is None and cell is None) or pbc is False):
-                if cutoff is None:
-                    cutoff = float(self.force_field.general[12])
+        block = np.empty((n_sys, 3, 3))
+        taken, rest = _host.cells(items, cutoff, self.max_expanded_atoms, block)
+        for k, rk in taken:
+            if k not in slow_set:
+                flags_l[k], cells[k], reps[k] = ALL_PBC, block[k], rk
+        for k in rest:
+            if k not in slow_set:
+                cell, pbc = items[k][3], items[k][4]
                 fast = periodic_cell(cell, pbc, cutoff, sizes[k], self.max_expanded_atoms)
                 if fast is not None:
                     flags_l[k], cells[k], reps[k] = fast
@@ -782,6 +793,8 @@ class Calculator:
         held = _BatchResults(energy, forces, per_atom, counts, dipole, offsets.tolist(), (bi, bj, bS, bbo),
                              cut.tolist())
         etot = energy[:, 14].tolist()
+        if _host is not None:
+            return _host.evaluations(Evaluation, etot, full_derivative, list(reps), backend, held)
         results = []
         new = object.__new__
         for k in range(n_sys):

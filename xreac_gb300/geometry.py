@@ -69,8 +69,8 @@ def cell_repetitions(cutoff, flags, m, atoms, max_expanded_atoms=512):
     return tuple(int(v) for v in reps)
 
 
-_ALL_PBC = np.ones(3, dtype=bool)
-_ALL_PBC.flags.writeable = False
+ALL_PBC = np.ones(3, dtype=bool)
+ALL_PBC.flags.writeable = False
 
 
 def periodic_cell(cell, pbc, cutoff, atoms, max_expanded_atoms):
@@ -111,7 +111,7 @@ def periodic_cell(cell, pbc, cutoff, atoms, max_expanded_atoms):
     copies = reps[0] * reps[1] * reps[2]
     if copies > 1 and copies * atoms > max_expanded_atoms:
         return None
-    return _ALL_PBC, m, tuple(reps)
+    return ALL_PBC, m, tuple(reps)
 
 
 def validate_input(symbols, positions, total_charge=0, cell=None, pbc=None):
