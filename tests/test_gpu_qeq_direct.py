@@ -1,7 +1,7 @@
-"""The direct QEq solver (systems of up to 288 atoms) against the oracle's dense KKT solve of src/xreac/energy.py:89-103.
+"""The direct QEq solvers (one block up to 288 atoms, a cluster of blocks up to 736) against the oracle's dense KKT solve of src/xreac/energy.py:89-103.
 
-Sizes lie on both sides of its 32-row tiles, of its launch classes (32, 96 atoms) and of its end; the next size takes
-the CG solver. Cells so small that an atom sees its own images, net charges, warm starts, adjoint solves
+Sizes lie on both sides of their 32-row tiles, of their launch classes (32, 96, 288, 608 atoms) and of their end; the
+next size takes the CG solver. Cells so small that an atom sees its own images, net charges, warm starts, adjoint solves
 and batches go through it too. Charges agree to 1e-10 e, the limit of the reference's backend comparison
 (scripts/validate.py:122-146), whatever the solver.
 """
@@ -45,7 +45,8 @@ def _dense(symbols, x, cell=None, charge=0.0):
     return oracle.qeq_charges(oracle._Model(ff, symbols, edges), np.sqrt((v * v).sum(axis=1)), charge)
 
 
-SIZES = [1, 2, 3, 31, 32, 33, 63, 64, 65, 95, 96, 97, 128, 129, 160, 191, 256, 257, 287, 288, 289]
+SIZES = [1, 2, 3, 31, 32, 33, 63, 64, 65, 95, 96, 97, 128, 129, 160, 191, 256, 257, 287, 288, 289,
+         320, 321, 415, 416, 417, 512, 513, 607, 608, 609, 641, 704, 735, 736, 737]
 
 
 @pytest.mark.parametrize("n", SIZES)
@@ -55,12 +56,12 @@ def test_cluster_charges(n):
     r = calc.evaluate(symbols, x, total_charge=1.0 if n % 2 else 0.0)
     np.testing.assert_allclose(r.charges, _dense(symbols, x, charge=1.0 if n % 2 else 0.0), atol=1e-10, rtol=0)
     steps = calc.qeq_work()[0]
-    assert steps <= 8 if n <= 288 else steps > 8  # refinement steps, or CG iterations
+    assert steps <= 8 if n <= 736 else steps > 8  # refinement steps, or CG iterations
     warm = calc.evaluate(symbols, x + 1e-3, total_charge=1.0 if n % 2 else 0.0, initial_charges=r.charges + 0.01)
     np.testing.assert_allclose(warm.charges, r.charges, atol=1e-10, rtol=0)
 
 
-@pytest.mark.parametrize("n_mol,side", [(1, 4.0), (8, 6.5), (27, 9.4), (60, 12.3)])
+@pytest.mark.parametrize("n_mol,side", [(1, 4.0), (8, 6.5), (27, 9.4), (60, 12.3), (110, 15.0), (205, 18.4)])
 def test_small_cells_with_self_images(n_mol, side):
     from xreac_gb300 import Calculator, ForceField
     from xreac_gb300.workloads import water_box
@@ -73,7 +74,7 @@ def test_small_cells_with_self_images(n_mol, side):
 
 
 def test_batch_equals_cg_with_charge_response():
-    items = [dict(symbols=s, positions=x) for s, x in (_cluster(n, seed=n) for n in (3, 30, 96, 99, 180, 288, 300, 420))]
+    items = [dict(symbols=s, positions=x) for s, x in (_cluster(n, seed=n) for n in (3, 30, 96, 99, 180, 288, 300, 420, 608, 650))]
     direct, cg = _calc(), _cg(_calc())
     for full in (False, True):
         a, b = direct.evaluate_many(items, full_derivative=full), cg.evaluate_many(items, full_derivative=full)

@@ -101,9 +101,10 @@ struct xr_ctx {
   static constexpr size_t kGraphSeen = 4096;
   int last_graph = 0;  // of the last call: 0 launched directly, 1 recorded, 2 replayed
   // Side streams and events of the launch sequence (XrFork).
-  cudaStream_t side[5] = {};     // bonded, torsions, hydrogen bonds; direct QEq solves beside CG ones, their small class
-  cudaEvent_t fork_ev[10] = {};
+  cudaStream_t side[6] = {};     // bonded, torsions, hydrogen bonds; the direct QEq solves' classes
+  cudaEvent_t fork_ev[11] = {};
   bool qeq_direct = false;       // the direct QEq solver fits the device's shared memory
+  int direct8 = 0, direct16 = 0;  // the largest systems of its clusters of 8 and 16 blocks (0: not available)
   // Cell list (xr_ctx_set_cell_list): 0 chooses per call, 1 always, -1 never.
   int cell_mode = 0;
   int* atom_cell = nullptr;
@@ -697,15 +698,16 @@ constexpr int kQeqClusterMax = 640;
 
 bool plan_qeq_cluster(xr_ctx* c, const xr_system* sys, int nsys, const std::vector<int>& ids, int* csize, int* nblocks, int* nbig,
                       int* nsmall) {
-  *csize = nsys > 1 ? kQeqClusterBatch : kQeqClusterSingle;
-  if ((nsys > 1 ? c->max_clusters_batch : c->max_clusters) < 1) return false;
-  const int cs = *csize;
   const int limit = nsys > 1 ? kQeqBatchBlock : kQeqClusterMax;
   std::vector<int> big, small;
   for (int s : ids) {
     if (sys[s].natoms > limit) return false;
     (sys[s].natoms > kQeqSmall ? big : small).push_back(s);
   }
+  // wide clusters while every cluster system gets one at once
+  const bool wide = nsys == 1 || (int)big.size() * kQeqClusterSingle <= c->nsm;
+  if ((wide ? c->max_clusters : c->max_clusters_batch) < 1) return false;
+  const int cs = *csize = wide ? kQeqClusterSingle : kQeqClusterBatch;
   auto larger = [&](int a, int b) { return sys[a].natoms > sys[b].natoms; };
   std::sort(big.begin(), big.end(), larger);
   std::sort(small.begin(), small.end(), larger);
@@ -718,21 +720,37 @@ bool plan_qeq_cluster(xr_ctx* c, const xr_system* sys, int nsys, const std::vect
   return true;
 }
 
-// The systems small enough for the direct solver (xr_qeq_direct.cu), largest first, and the others
-// (for the CG plans). A caller that bounds the CG iterations, or the test that makes a
-// team wait run out, gets the CG solver whose iterations and waits those are.
+// The systems small enough for the direct solvers (xr_qeq_direct.cu) by class, each largest first, and the
+// others (for the CG plans). A caller that bounds the CG iterations, or the test that makes a team wait
+// run out, gets the CG solver whose iterations and waits those are.
 constexpr int kQeqDirectIterations = 400;
 
-void plan_qeq_direct(const xr_ctx* c, const xr_system* sys, int nsys, std::vector<int>& large, std::vector<int>& small,
-                     std::vector<int>& rest) {
+struct DirectPlan {
+  std::vector<int> cluster, block, small;  // clusters of `nb` blocks; single blocks; single blocks of small systems
+  int nb = 8;
+};
+
+void plan_qeq_direct(const xr_ctx* c, const xr_system* sys, int nsys, DirectPlan& d, std::vector<int>& rest) {
   const bool on = c->qeq_direct && c->cg_max >= kQeqDirectIterations && c->wait_polls == 0 && c->wait_fail_at == 0;
   for (int s = 0; s < nsys; ++s) {
     const int n = sys[s].natoms;
-    (!on || n > kQeqDirectMax ? rest : n > kQeqDirectSmall ? large : small).push_back(s);
+    if (!on)
+      rest.push_back(s);
+    else if (n <= kQeqDirectSmall)
+      d.small.push_back(s);
+    else if (n <= kQeqDirectMax)
+      d.block.push_back(s);
+    else if (n <= c->direct8)
+      d.cluster.push_back(s);
+    else if (nsys == 1 && n <= c->direct16) {  // a system alone also takes the wider clusters
+      d.cluster.push_back(s);
+      d.nb = 16;
+    } else {
+      rest.push_back(s);
+    }
   }
   auto larger = [&](int a, int b) { return sys[a].natoms > sys[b].natoms; };
-  std::sort(large.begin(), large.end(), larger);
-  std::sort(small.begin(), small.end(), larger);
+  for (std::vector<int>* v : {&d.cluster, &d.block, &d.small}) std::sort(v->begin(), v->end(), larger);
 }
 
 // Whether the kept skin list serves this call: the same systems (atom counts, types, pbc, cells) at
@@ -1144,16 +1162,17 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
   // plan (its tables go through pinned buffers that a replay copies again) and the bond export.
   int qblocks = 0, qteam = 0, qsmall = 0, qbig = 0, qcsize = 0, nlist = 0;
   bool qcluster = false;
-  std::vector<int> qdl, qds, qrest;  // direct solves (two classes), and the systems of the CG solvers
+  DirectPlan qd;
+  std::vector<int> qrest;  // the systems of the CG solvers
   if (c->coop_per_sm > 0) {
-    plan_qeq_direct(c, sys, nsys, qdl, qds, qrest);
+    plan_qeq_direct(c, sys, nsys, qd, qrest);
     c->h_qsmall.clear();
     if (!qrest.empty()) {
       qcluster = plan_qeq_cluster(c, sys, nsys, qrest, &qcsize, &qblocks, &qbig, &qsmall);
       if (!qcluster) plan_qeq(c, sys, nsys, qrest, &qblocks, &qteam, &qsmall);
     }
-    c->h_qsmall.insert(c->h_qsmall.end(), qdl.begin(), qdl.end());
-    c->h_qsmall.insert(c->h_qsmall.end(), qds.begin(), qds.end());
+    for (const std::vector<int>* v : {&qd.cluster, &qd.block, &qd.small})
+      c->h_qsmall.insert(c->h_qsmall.end(), v->begin(), v->end());
     nlist = (int)c->h_qsmall.size();
     if (!host_grow(&c->h_qmap_p, &c->ch_qmap_p, (size_t)std::max(qteam, 1)) ||
         !host_grow(&c->h_qsmall_p, &c->ch_qsmall_p, (size_t)std::max(nlist, 1)))
@@ -1169,41 +1188,49 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
   const bool forked = !c->profile;
   const XrFork fork = {forked, st, forked ? c->side[0] : st, forked ? c->side[1] : st, forked ? c->side[2] : st,
                        c->fork_ev[0], c->fork_ev[1], c->fork_ev[2], c->fork_ev[3], c->fork_ev[4], c->fork_ev[5], c->fork_ev[6]};
-  // The charges: the CG solvers on the call's stream, direct solves beside them, then what those left
-  // to CG. (The direct solves' launches come second: a CG team needs whole SMs.)
-  const int ndl = (int)qdl.size(), nds = (int)qds.size(), nd = ndl + nds;
-  const int largest_dl = ndl ? sys[qdl[0]].natoms : 0, largest_ds = nds ? sys[qds[0]].natoms : 0;
+  // The charges: the CG solvers on the call's stream, each class of direct solves beside them on a stream of
+  // its own (the first class takes the call's when there is no CG), then what those left to CG. The CG
+  // launch comes first: its teams need whole SMs.
+  const std::vector<int>* const dclass[3] = {&qd.cluster, &qd.block, &qd.small};
+  const int dcount[3] = {(int)qd.cluster.size(), (int)qd.block.size(), (int)qd.small.size()};
+  int dlargest[3], nd = 0;
+  for (int k = 0; k < 3; ++k) {
+    dlargest[k] = dcount[k] ? sys[(*dclass[k])[0]].natoms : 0;
+    nd += dcount[k];
+  }
   auto launch_qeq = [&](bool adjoint) -> int {
-    const bool beside = fork.on && !qrest.empty() && nd > 0;
-    const cudaStream_t sd = beside ? c->side[3] : st;
-    const bool apart = fork.on && ndl > 0 && nds > 0;  // the two classes of direct solves
-    const cudaStream_t ss = apart ? c->side[4] : sd;
-    if (beside || apart) {
-      cudaEventRecord(c->fork_ev[7], st);
-      if (beside) cudaStreamWaitEvent(sd, c->fork_ev[7], 0);
-      if (apart) cudaStreamWaitEvent(ss, c->fork_ev[7], 0);
+    const bool cg = !qrest.empty() || nd == 0;
+    cudaStream_t dst[3] = {};
+    bool free_main = !cg;
+    if (nd > 0 && (cg || (dcount[0] > 0) + (dcount[1] > 0) + (dcount[2] > 0) > 1)) cudaEventRecord(c->fork_ev[7], st);
+    for (int k = 0; k < 3; ++k) {
+      if (dcount[k] == 0) continue;
+      dst[k] = free_main ? st : c->side[3 + k];
+      if (!free_main) cudaStreamWaitEvent(dst[k], c->fork_ev[7], 0);
+      free_main = false;
     }
-    if (!qrest.empty() || nd == 0) {
+    if (cg) {
       const int le = qcluster ? xr_launch_qeq_cluster(w, ff->d, st, qcsize, qblocks, c->qsmall, qbig, qsmall, adjoint)
                               : xr_launch_qeq(w, ff->d, st, qblocks, c->qmap, qteam, c->qsmall, qsmall, adjoint);
       launches += (qcluster ? qbig > 0 : qteam > 0) ? 2 : 1;  // the teams' row splits, then the solver
       if (le) return le;
     }
-    if (nd == 0) return 0;
-    const int* const dlist = c->qsmall + (nlist - nd);
-    if (ndl > 0)
-      if (int le = xr_launch_qeq_direct(w, ff->d, sd, dlist, ndl, largest_dl, adjoint)) return le;
-    if (nds > 0)
-      if (int le = xr_launch_qeq_direct(w, ff->d, ss, dlist + ndl, nds, largest_ds, adjoint)) return le;
-    if (apart) {
-      cudaEventRecord(c->fork_ev[8], ss);
-      cudaStreamWaitEvent(sd, c->fork_ev[8], 0);
+    const int* list = c->qsmall + (nlist - nd);
+    for (int k = 0; k < 3; ++k) {
+      if (dcount[k] == 0) continue;
+      const int le = k == 0 ? xr_launch_qeq_direct_cluster(w, ff->d, dst[0], list, dcount[0], dlargest[0], qd.nb, adjoint)
+                            : xr_launch_qeq_direct(w, ff->d, dst[k], list, dcount[k], dlargest[k], adjoint);
+      if (le) return le;
+      list += dcount[k];
+      ++launches;
+      if (dst[k] != st) {
+        cudaEventRecord(c->fork_ev[8 + k], dst[k]);
+        cudaStreamWaitEvent(st, c->fork_ev[8 + k], 0);
+      }
     }
-    if (int le = xr_launch_qeq_retry(w, ff->d, sd, std::min(nd, c->nsm), adjoint)) return le;
-    launches += (ndl > 0) + (nds > 0) + 1;
-    if (beside) {
-      cudaEventRecord(c->fork_ev[9], sd);
-      cudaStreamWaitEvent(st, c->fork_ev[9], 0);
+    if (nd > 0) {
+      ++launches;
+      if (int le = xr_launch_qeq_retry(w, ff->d, st, std::min(nd, c->nsm), adjoint)) return le;
     }
     return 0;
   };
@@ -1270,7 +1297,7 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
   bool done = false;
   if (c->graphs && !c->profile && qteam == 0) {
     const int ints[] = {(int)mode, qcluster ? 1 : 0, qcsize, qblocks, qteam, qsmall, qbig, nlist, nE > 0, nP > 0, nB > 0,
-                        (int)flags, ndl, nds, largest_dl, largest_ds};
+                        (int)flags, dcount[0], dcount[1], dcount[2], dlargest[0], dlargest[1], dlargest[2], qd.nb};
     const void* ptrs[] = {c->h_qmap_p, c->h_qsmall_p, c->qmap, c->qsmall, c->outbuf};
     const int nptrs = (int)(sizeof(ptrs) / sizeof(ptrs[0]));
     const std::vector<unsigned char> kv = launch_key(w, ff->d, ints, (int)(sizeof(ints) / sizeof(int)), ptrs, nptrs);
@@ -1736,6 +1763,10 @@ int xr_ctx_create(int device, void* stream, xr_ctx** out) {
   cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device);
   c->coop_per_sm = xr_qeq_coop_blocks_per_sm();
   c->qeq_direct = xr_qeq_direct_ready();
+  if (c->qeq_direct) {
+    c->direct8 = xr_qeq_direct_cluster_max(8);
+    c->direct16 = xr_qeq_direct_cluster_max(16);
+  }
   c->max_clusters = xr_qeq_max_clusters(kQeqClusterSingle);
   c->max_clusters_batch = xr_qeq_max_clusters(kQeqClusterBatch);
   int coop_ok = 0;

@@ -1,4 +1,4 @@
-// QEq by a dense FP32 factorization under FP64 refinement, one thread block per system.
+// QEq by a dense FP32 factorization under FP64 refinement, one thread block or one cluster per system.
 //
 // A system of up to kQeqDirectMax atoms has its whole matrix in one block's shared memory. The CG
 // it would take otherwise needs 30 to 140 iterations of 2 to 7 us (two team reductions each).
@@ -319,18 +319,51 @@ __device__ inline void substitute(const DirectLayout& L, const DirectShared& sh,
   }
 }
 
-// G = H X of the system's rows in FP64 (the caller adds the diagonal and chi): a group of lanes per
-// row, X in shared memory.
-__device__ inline void product64(const XrWork& w, const DirectLayout& L, int a0, int n) {
+// One warp: add(j, h) for the entries [beg, end) of a row, in the local column j (FP32 h). The images of one j
+// are adjacent and added one after the other, so the sums are the same on every call.
+template <class Add>
+__device__ inline void add_row(const XrWork& w, int a0, int n, int beg, int end, Add add) {
+  const int lane = threadIdx.x & 31;
+  int before = -1;
+  for (int e0 = beg; e0 < end; e0 += 128) {
+    int j[4];
+    float h[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int e = e0 + 32 * u + lane;
+      j[u] = e < end ? w.edge[e].x - a0 : n;
+      h[u] = e < end ? w.qch[e] : 0.0f;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      if (e0 + 32 * u >= end) break;  // uniform per warp
+      int prev = __shfl_up_sync(0xffffffffu, j[u], 1);
+      if (lane == 0) prev = before;
+      before = __shfl_sync(0xffffffffu, j[u], 31);
+      const unsigned first = __ballot_sync(0xffffffffu, j[u] != prev) & ((2u << lane) - 1u);
+      const int rank = j[u] < n ? (first ? lane - (31 - __clz(first)) : lane) : -1;  // images of j before this one
+      const int last = __reduce_max_sync(0xffffffffu, rank);
+      for (int q = 0; q <= last; ++q) {
+        if (rank == q) add(j[u], h[u]);
+        __syncwarp();
+      }
+    }
+  }
+}
+
+// G[q] = (H X)_row(q) in FP64 for q < m (the caller adds the diagonal and chi): a group of lanes per
+// row, X (of the whole system) in shared memory.
+template <class Row>
+__device__ inline void product64(const XrWork& w, const double* X, double* G, int a0, int m, Row row) {
   const int lane = threadIdx.x & 31, nw = blockDim.x >> 5, wid = threadIdx.x >> 5;
   int gs = 32;
-  while (gs > 4 && n * gs > 4 * (int)blockDim.x) gs >>= 1;
+  while (gs > 4 && m * gs > 4 * (int)blockDim.x) gs >>= 1;
   const int sub = lane & (gs - 1), gpw = 32 / gs;
-  for (int rb = wid * gpw; rb < n; rb += nw * gpw) {  // uniform per warp
-    const int r = rb + lane / gs;
+  for (int qb = wid * gpw; qb < m; qb += nw * gpw) {  // uniform per warp
+    const int q = qb + lane / gs;
     double s = 0.0;
-    if (r < n) {
-      const int ee = w.cnt[a0 + r + 1];
+    if (q < m) {
+      const int r = row(q), ee = w.cnt[a0 + r + 1];
       int e = w.cnt[a0 + r] + sub;
       for (; e + 3 * gs < ee; e += 4 * gs) {
         int j[4];
@@ -341,12 +374,12 @@ __device__ inline void product64(const XrWork& w, const DirectLayout& L, int a0,
           h[u] = w.hval[e + u * gs];
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) s += h[u] * L.X[j[u]];
+        for (int u = 0; u < 4; ++u) s += h[u] * X[j[u]];
       }
-      for (; e < ee; e += gs) s += w.hval[e] * L.X[w.edge[e].x - a0];
+      for (; e < ee; e += gs) s += w.hval[e] * X[w.edge[e].x - a0];
     }
     for (int o = gs / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-    if (sub == 0 && r < n) L.G[r] = s;
+    if (sub == 0 && q < m) G[q] = s;
   }
   __syncthreads();
 }
@@ -356,7 +389,7 @@ __global__ void __launch_bounds__(512, 1) k_qeq_direct(XrWork w, XrFF ff, const 
   extern __shared__ __align__(16) unsigned char dyn[];
   const int sys = list[blockIdx.x];
   const XrSystem& S = w.sys[sys];
-  const int a0 = S.atom_off, n = S.natoms, tid = threadIdx.x, lane = tid & 31, wid = tid >> 5, nw = blockDim.x >> 5;
+  const int a0 = S.atom_off, n = S.natoms, tid = threadIdx.x, wid = tid >> 5, nw = blockDim.x >> 5;
   const double* atab = xr_ff_at(ff, ff.nsets > 1 ? S.ff_set : 0).atom;
   const double Q = adjoint ? 0.0 : S.total_charge;
   const bool warm = !adjoint && S.has_guess != 0;
@@ -377,51 +410,25 @@ __global__ void __launch_bounds__(512, 1) k_qeq_direct(XrWork w, XrFF ff, const 
   if (r < rows) L.tiles[kTileSize * tile_at(r >> 5, r >> 5) + (kTile + 1) * (r & 31)] = row ? (float)eta : 1.0f;
   __syncthreads();
   // Row i's last entries, as many as it has half edges, are those with j > i and one direction of its
-  // self images; (j, i) lies in the lower triangle, whose rows j are contiguous. The images of one j
-  // are adjacent and add up one after the other, so the sums are the same on every call.
+  // self images; (j, i) lies in the lower triangle, whose rows j are contiguous.
   const int* const half = w.cnt + (w.A + 1) + a0;
   for (int i = wid; i < n; i += nw) {
-    const int end = w.cnt[a0 + i + 1], beg = end - (half[i + 1] - half[i]);
-    int before = -1;
-    for (int e0 = beg; e0 < end; e0 += 128) {
-      int j[4];
-      float h[4];
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int e = e0 + 32 * u + lane;
-        j[u] = e < end ? w.edge[e].x - a0 : n;
-        h[u] = e < end ? w.qch[e] : 0.0f;
+    add_row(w, a0, n, w.cnt[a0 + i + 1] - (half[i + 1] - half[i]), w.cnt[a0 + i + 1], [&](int j, float h) {
+      float* const t = L.tiles + kTileSize * tile_at(j >> 5, i >> 5);
+      if (j == i) {
+        t[(kTile + 1) * (i & 31)] += 2.0f * h;
+      } else {
+        t[kTile * (i & 31) + (j & 31)] += h;
+        if ((j >> 5) == (i >> 5)) t[kTile * (j & 31) + (i & 31)] += h;
       }
-#pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        if (e0 + 32 * u >= end) break;  // uniform per warp
-        int prev = __shfl_up_sync(0xffffffffu, j[u], 1);
-        if (lane == 0) prev = before;
-        before = __shfl_sync(0xffffffffu, j[u], 31);
-        const unsigned first = __ballot_sync(0xffffffffu, j[u] != prev) & ((2u << lane) - 1u);
-        const int rank = j[u] < n ? (first ? lane - (31 - __clz(first)) : lane) : -1;  // images of j before this one
-        const int last = __reduce_max_sync(0xffffffffu, rank);
-        for (int q = 0; q <= last; ++q) {
-          if (rank == q) {
-            float* const t = L.tiles + kTileSize * tile_at(j[u] >> 5, i >> 5);
-            if (j[u] == i) {
-              t[(kTile + 1) * (i & 31)] += 2.0f * h[u];
-            } else {
-              t[kTile * (i & 31) + (j[u] & 31)] += h[u];
-              if ((j[u] >> 5) == (i >> 5)) t[kTile * (j[u] & 31) + (i & 31)] += h[u];
-            }
-          }
-          __syncwarp();
-        }
-      }
-    }
+    });
   }
   // 2. The start gradient, projected: g - lambda with lambda = <D^-1, g> / <D^-1, 1>; the target is the
   //    tolerance times the norm <D^-1, g^2> at the uniform start, as in the CG solver.
   const bool product = warm || x0 != 0.0;
   if (product) {
     __syncthreads();
-    product64(w, L, a0, n);
+    product64(w, L.X, L.G, a0, n, [](int q) { return q; });
   } else {
     __syncthreads();
   }
@@ -434,7 +441,7 @@ __global__ void __launch_bounds__(512, 1) k_qeq_direct(XrWork w, XrFF ff, const 
       __syncthreads();
       if (row) L.X[r] = x0;
       __syncthreads();
-      product64(w, L, a0, n);
+      product64(w, L.X, L.G, a0, n, [](int q) { return q; });
       if (row) {
         gu = L.G[r] + eta * x0 + chi;
         L.X[r] = x;
@@ -493,7 +500,7 @@ __global__ void __launch_bounds__(512, 1) k_qeq_direct(XrWork w, XrFF ff, const 
     if (last) break;
     if (row) L.X[r] = x;
     __syncthreads();
-    product64(w, L, a0, n);
+    product64(w, L.X, L.G, a0, n, [](int q) { return q; });
     g = row ? L.G[r] + eta * x + chi : 0.0;
     double vl[1] = {di * g};
     block_sums<1>(sh, vl, n, [&](double* t) { t[0] /= s1; });
@@ -530,7 +537,437 @@ __global__ void __launch_bounds__(512, 1) k_qeq_direct(XrWork w, XrFF ff, const 
   w.a_e[(size_t)6 * w.A + a] = SELF_CONVERSION * (chi * q + 0.5 * eta * q * q);
 }
 
+// ------------------------------------------------------------------------------------ clusters
+// Larger systems: the same solve by the blocks of one thread-block cluster. Tile row i belongs to
+// block i mod nb; a block holds its rows' tiles (W_ik in place once known), a copy of the current
+// panel's tiles A_ik of every row, and the vectors whole. Step k of the factorization: the blocks send
+// their A_ik, and the owner of row k its D_k^-1, to every block; then each forms its W_ik and updates
+// its rows, the owner of row k + 1 inverting that row's diagonal tile meanwhile. A substitution sends
+// one tile of the vector a step (forward), or adds its product to the other rows' tiles at their
+// owners (backward). All control flow is the same in every block (it depends on cluster-wide sums
+// only), so the blocks meet at the hardware cluster barrier. Measured on 8 blocks, CG then direct: 396
+// atoms 537 -> 266 us (factorization 90, a substitution 26); on 16, 648 atoms warm-started 508 -> 427
+// us; a batch of 128 requests of up to 512 atoms, all classes side by side, 1165 -> 351 us.
+__device__ inline unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
+__device__ inline unsigned remote(const void* p, int rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(smem_u32(p)), "r"(rank));
+  return r;
+}
+__device__ inline void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ inline void send(const float* at, int rank, float v) {
+  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(remote(at, rank)), "f"(v) : "memory");
+}
+__device__ inline void send(const double* at, int rank, double v) {
+  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(remote(at, rank)), "d"(v) : "memory");
+}
+__device__ inline void send4(const float* at, int rank, const float4& v) {
+  asm volatile("st.shared::cluster.v4.f32 [%0], {%1, %2, %3, %4};" ::"r"(remote(at, rank)), "f"(v.x), "f"(v.y), "f"(v.z), "f"(v.w)
+               : "memory");
+}
+__device__ inline void send_add(const float* at, int rank, float v) {
+  asm volatile("red.relaxed.cluster.shared::cluster.add.f32 [%0], %1;" ::"r"(remote(at, rank)), "f"(v) : "memory");
+}
+
+// Tiles of block p's rows before its l-th one (row p + nb l).
+__host__ __device__ constexpr int row_offset(int p, int nb, int l) { return l * (p + 1) + nb * (l * (l - 1) / 2); }
+__host__ __device__ constexpr int rows_of(int p, int nb, int T) { return p < T ? (T - 1 - p) / nb + 1 : 0; }
+__host__ __device__ constexpr int most_tiles(int nb, int T) {
+  int m = 0;
+  for (int p = 0; p < nb; ++p) {
+    const int t = row_offset(p, nb, rows_of(p, nb, T));
+    m = t > m ? t : m;
+  }
+  return m;
+}
+__host__ __device__ constexpr size_t cluster_bytes(int n, int nb) {
+  const int T = (n + kTile - 1) / kTile;
+  return (size_t)4 * kTileSize * (most_tiles(nb, T) + T - 1 + 1) +
+         (size_t)kTile * (T * (sizeof(double) + 2 * sizeof(float)) + rows_of(0, nb, T) * sizeof(double));
+}
+
+struct ClusterShared {
+  DirectShared d;
+  double slots[2][16][4];  // partial sums by block, two exchanges' in turn
+};
+
+struct ClusterLayout {
+  int T, nb, rank, own;  // tile rows; blocks; this block and its number of rows (atoms, padding included)
+  float *tiles, *panel, *dinv;
+  double *X, *G;
+  float *b, *w1;
+  __device__ ClusterLayout(unsigned char* dyn, int n, int blocks, int p) {
+    T = (n + kTile - 1) / kTile;
+    nb = blocks;
+    rank = p;
+    own = kTile * rows_of(p, nb, T);
+    tiles = reinterpret_cast<float*>(dyn);  // the same offsets in every block: remote addresses are local ones
+    panel = tiles + kTileSize * most_tiles(nb, T);
+    dinv = panel + kTileSize * (T - 1);
+    X = reinterpret_cast<double*>(dinv + kTileSize);
+    b = reinterpret_cast<float*>(X + kTile * T);
+    w1 = b + kTile * T;
+    G = reinterpret_cast<double*>(w1 + kTile * T);
+  }
+  __device__ float* tile(int i, int j) const { return tiles + kTileSize * (row_offset(rank, nb, i / nb) + j); }  // i own
+  __device__ int owner(int i) const { return i % nb; }
+  __device__ int row(int q) const { return kTile * (rank + nb * (q >> 5)) + (q & 31); }  // atom of own row q
+};
+
+// Sums over the cluster of NV values of every thread with a row, in block order; post as in block_sums.
+template <int NV, class Post>
+__device__ inline void cluster_sums(const ClusterLayout& L, ClusterShared& sh, unsigned& parity, double (&v)[NV], Post post) {
+  static_assert(NV <= 4, "at most four values");
+  const int rows = L.own > 0 ? L.own : 1;
+  double (*slots)[4] = sh.slots[parity & 1];
+  ++parity;
+  block_sums<NV>(sh.d, v, rows, [](double*) {});
+  if ((int)threadIdx.x < L.nb)
+#pragma unroll
+    for (int k = 0; k < NV; ++k) send(&slots[L.rank][k], threadIdx.x, v[k]);
+  cluster_sync();
+  if (threadIdx.x == 0) {
+#pragma unroll
+    for (int k = 0; k < NV; ++k) {
+      v[k] = slots[0][k];
+      for (int q = 1; q < L.nb; ++q) v[k] += slots[q][k];
+    }
+    post(v);
+#pragma unroll
+    for (int k = 0; k < NV; ++k) sh.d.tot[k] = v[k];
+  }
+  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < NV; ++k) v[k] = sh.d.tot[k];
+}
+
+__device__ __noinline__ void cluster_factorize(const ClusterLayout& L, ClusterShared& sh) {
+  const int T = L.T, nb = L.nb, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  const int rg = threadIdx.x & 7, cg = (threadIdx.x >> 3) & 3;
+  if (L.rank == 0 && wid < 4) tile_inverse(L.tile(0, 0), nullptr, nullptr, sh.d);
+  for (int k = 0; k + 1 < T; ++k) {
+    cluster_sync();  // the last step's panel has been read everywhere
+    const int first = L.rank + nb * ((k + nb - L.rank) / nb);  // this block's first row past k
+    const int m = first < T ? (T - 1 - first) / nb + 1 : 0;    // and how many
+    for (int u = threadIdx.x; u < m * (kTileSize / 4); u += blockDim.x) {
+      const int i = first + nb * (u / (kTileSize / 4)), q = 4 * (u % (kTileSize / 4));
+      const float4 v = *reinterpret_cast<const float4*>(L.tile(i, k) + q);
+      for (int p = 0; p < nb; ++p) send4(L.panel + kTileSize * (i - 1) + q, p, v);
+    }
+    if (L.owner(k) == L.rank)
+      for (int u = threadIdx.x; u < kTileSize / 4; u += blockDim.x) {
+        const float4 v = *reinterpret_cast<const float4*>(L.tile(k, k) + 4 * u);
+        for (int p = 0; p < nb; ++p) send4(L.dinv + 4 * u, p, v);
+      }
+    cluster_sync();
+    for (int u = wid; u < 2 * m; u += nw) {  // W_ik = A_ik D_k^-1 in A_ik's place
+      const int i = first + nb * (u >> 1), c0 = 16 * (u & 1);
+      float c[4][4];
+      tile_product<4>(L.panel + kTileSize * (i - 1), L.dinv, c0, c);
+      float* o = L.tile(i, k) + kTile * c0;
+#pragma unroll
+      for (int q = 0; q < 4; ++q)
+        *reinterpret_cast<float4*>(o + kTile * (4 * cg + q) + 4 * rg) = make_float4(c[0][q], c[1][q], c[2][q], c[3][q]);
+    }
+    __syncthreads();
+    const bool next = L.owner(k + 1) == L.rank;  // this block inverts the next diagonal tile
+    if (next && wid < 4) {
+      tile_inverse(L.tile(k + 1, k + 1), L.tile(k + 1, k), L.panel + kTileSize * k, sh.d);
+    } else {
+      // the tiles (i, j), k < j <= i, of own rows i, numbered row by row
+      const int w0 = next ? wid - 4 : wid, ws = next ? nw - 4 : nw;
+      int u = w0, i = first;
+      for (;;) {
+        while (i < T && u >= i - k) {
+          u -= i - k;
+          i += nb;
+        }
+        if (i >= T) break;
+        const int j = k + 1 + u;
+        if (!(next && i == k + 1)) {
+          float c[4][8];
+          tile_product<8>(L.tile(i, k), L.panel + kTileSize * (j - 1), 0, c);
+          float* o = L.tile(i, j);
+#pragma unroll
+          for (int q = 0; q < 8; ++q) {
+            float4* d = reinterpret_cast<float4*>(o + kTile * (8 * cg + q) + 4 * rg);
+            float4 v = *d;
+            v.x -= c[0][q];
+            v.y -= c[1][q];
+            v.z -= c[2][q];
+            v.w -= c[3][q];
+            *d = v;
+          }
+        }
+        u += ws;
+      }
+    }
+  }
+  __syncthreads();
+}
+
+// H^-1 v for the NV vectors v[k], given and left in the owners' rows (a thread per own row).
+template <int NV>
+__device__ inline void cluster_substitute(const ClusterLayout& L, float* const (&v)[NV]) {
+  const int T = L.T, nb = L.nb, r = threadIdx.x;
+  const bool mine = r < L.own;
+  const int at = mine ? L.row(r) : 0, i = at >> 5;
+  auto publish = [&](int q) {  // this thread's row of every vector, to every block
+    for (int p = 0; p < nb; ++p) send(v[q] + at, p, v[q][at]);
+  };
+  if (mine && i == 0)
+    for (int q = 0; q < NV; ++q) publish(q);
+  cluster_sync();
+  for (int k = 0; k + 1 < T; ++k) {
+    if (mine && i > k) {
+      const float* w = L.tile(i, k) + (at & 31);
+      float s[NV][2];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) s[q][0] = s[q][1] = 0.0f;
+#pragma unroll 8
+      for (int c = 0; c < kTile; c += 2) {
+        const float w0 = w[kTile * c], w1 = w[kTile * c + kTile];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) {
+          s[q][0] += w0 * v[q][kTile * k + c];
+          s[q][1] += w1 * v[q][kTile * k + c + 1];
+        }
+      }
+#pragma unroll
+      for (int q = 0; q < NV; ++q) {
+        v[q][at] -= s[q][0] + s[q][1];
+        if (i == k + 1) publish(q);
+      }
+    }
+    cluster_sync();
+  }
+  float z[NV];
+  if (mine) {
+    const float* d = L.tile(i, i) + (at & 31);
+#pragma unroll
+    for (int q = 0; q < NV; ++q) z[q] = 0.0f;
+#pragma unroll 8
+    for (int c = 0; c < kTile; ++c) {
+      const float x = d[kTile * c];
+#pragma unroll
+      for (int q = 0; q < NV; ++q) z[q] += x * v[q][kTile * i + c];
+    }
+  }
+  __syncthreads();
+  if (mine)
+#pragma unroll
+    for (int q = 0; q < NV; ++q) v[q][at] = z[q];
+  cluster_sync();
+  for (int k = T - 1; k > 0; --k) {
+    if (L.owner(k) == L.rank)
+      for (int t = r; t < kTile * k; t += blockDim.x) {
+        const float* w = L.tile(k, t >> 5) + kTile * (t & 31);
+        float s[NV];
+#pragma unroll
+        for (int q = 0; q < NV; ++q) s[q] = 0.0f;
+#pragma unroll 8
+        for (int u = 0; u < kTile; ++u) {
+          const int c = (u + t) & 31;  // a lane starts at its own column: no two share a bank
+          const float x = w[c];
+#pragma unroll
+          for (int q = 0; q < NV; ++q) s[q] += x * v[q][kTile * k + c];
+        }
+#pragma unroll
+        for (int q = 0; q < NV; ++q) send_add(v[q] + t, L.owner(t >> 5), -s[q]);
+      }
+    cluster_sync();
+  }
+}
+
+__global__ void __launch_bounds__(512, 1) k_qeq_direct_cluster(XrWork w, XrFF ff, const int* list, int nb, int adjoint) {
+  __shared__ ClusterShared sh;
+  extern __shared__ __align__(16) unsigned char dyn[];
+  const int sys = list[blockIdx.x / nb];
+  const XrSystem& S = w.sys[sys];
+  const int a0 = S.atom_off, n = S.natoms, tid = threadIdx.x, wid = tid >> 5, nw = blockDim.x >> 5;
+  const double* atab = xr_ff_at(ff, ff.nsets > 1 ? S.ff_set : 0).atom;
+  const double Q = adjoint ? 0.0 : S.total_charge;
+  const bool warm = !adjoint && S.has_guess != 0;
+  const double x0 = Q == 0.0 ? 0.0 : Q / n;
+  const ClusterLayout L(dyn, n, nb, blockIdx.x % nb);
+  const int at = tid < L.own ? L.row(tid) : 0, m = min(L.own, max(0, L.own > 0 ? L.own - max(0, kTile * L.T - n) *
+                                                                              (L.owner(L.T - 1) == L.rank ? 1 : 0) : 0));
+  const bool row = tid < m;  // (only the last tile row has padding)
+  const int a = a0 + min(at, n - 1), type = w.type[a];
+  const double eta = atom_prm(atab, type, A_ETA), chi = adjoint ? w.qrhs[a] : atom_prm(atab, type, A_CHI);
+  unsigned parity = 0;
+  // 1. The own rows' tiles; the charges of every row.
+  const int ntiles = row_offset(L.rank, nb, L.own / kTile);
+  for (int k = tid; k < ntiles * kTileSize / 4; k += blockDim.x) reinterpret_cast<float4*>(L.tiles)[k] = make_float4(0, 0, 0, 0);
+  for (int k = tid; k < kTile * L.T; k += blockDim.x) L.X[k] = k < n ? (warm ? w.qguess[a0 + k] : x0) : 0.0;
+  __syncthreads();
+  if (tid < L.own) L.tile(at >> 5, at >> 5)[(kTile + 1) * (at & 31)] = row ? (float)eta : 1.0f;
+  __syncthreads();
+  // Row i's first entries, all but as many as it has half edges, are those with j < i and one direction of its
+  // self images.
+  const int* const half = w.cnt + (w.A + 1) + a0;
+  for (int q = wid; q < m; q += nw) {
+    const int i = L.row(q);
+    add_row(w, a0, n, w.cnt[a0 + i], w.cnt[a0 + i + 1] - (half[i + 1] - half[i]), [&](int j, float h) {
+      float* const t = L.tile(i >> 5, j >> 5);
+      if (j == i) {
+        t[(kTile + 1) * (i & 31)] += 2.0f * h;
+      } else {
+        t[kTile * (j & 31) + (i & 31)] += h;
+        if ((j >> 5) == (i >> 5)) t[kTile * (i & 31) + (j & 31)] += h;
+      }
+    });
+  }
+  __syncthreads();
+  auto product = [&]() { product64(w, L.X, L.G, a0, m, [&](int q) { return L.row(q); }); };
+  // 2. The start gradient and the target, as in k_qeq_direct.
+  const double di = row ? 1.0 / (double)L.tile(at >> 5, at >> 5)[(kTile + 1) * (at & 31)] : 0.0;
+  double x = row ? L.X[at] : 0.0, g = chi, gu = chi;
+  if (warm || x0 != 0.0) {
+    product();
+    g = gu = row ? L.G[tid] + eta * x + chi : 0.0;
+  }
+  if (warm) {
+    gu = chi;
+    if (x0 != 0.0) {
+      __syncthreads();
+      for (int k = tid; k < n; k += blockDim.x) L.X[k] = x0;
+      __syncthreads();
+      product();
+      gu = row ? L.G[tid] + eta * x0 + chi : 0.0;
+    }
+  }
+  if (!row) g = gu = 0.0;
+  double v3[3] = {di, di * g, di * gu}, vn[2] = {di * g * g, di * gu * gu};
+  cluster_sync();  // every block runs before the first remote write
+  cluster_sums<2>(L, sh, parity, vn, [](double*) {});
+  cluster_sums<3>(L, sh, parity, v3, [](double* t) {
+    t[1] /= t[0];
+    t[2] /= t[0];
+  });
+  const double s1 = v3[0], gfloor = 1e-28 * fmax(vn[0], vn[1]);
+  if (row) {
+    g -= v3[1];
+    gu -= v3[2];
+  }
+  double v2[2] = {di * g * g, di * gu * gu};
+  cluster_sums<2>(L, sh, parity, v2, [&](double* t) { t[1] *= w.cg_tol * w.cg_tol; });
+  double gz = v2[0];
+  const double target = v2[1];
+  // 3. Refinement steps, as in k_qeq_direct; y is made to sum to zero in FP64, so that one exchange gives its
+  //    multiplier and the constraint's shift.
+  int steps = 0;
+  bool failed = false, last = false, more = gz > target && gz > gfloor && n >= 2;
+  while (more) {
+    if (steps == 8 && !last) {
+      failed = true;
+      break;
+    }
+    if (tid < L.own) L.b[at] = row ? (float)-g : 0.0f;
+    if (steps == 0) {
+      if (tid < L.own) L.w1[at] = row ? 1.0f : 0.0f;
+      cluster_factorize(L, sh);
+      float* const both[2] = {L.b, L.w1};
+      cluster_substitute<2>(L, both);
+    } else {
+      float* const one[1] = {L.b};
+      cluster_substitute<1>(L, one);
+    }
+    ++steps;
+    const double b = row ? (double)L.b[at] : 0.0, w1 = row ? (double)L.w1[at] : 0.0;
+    double vs[3] = {b, w1, x};
+    cluster_sums<3>(L, sh, parity, vs, [&](double* t) {
+      t[0] /= t[1];
+      t[2] = (Q - t[2]) / n;
+    });
+    if (row) x += (b - vs[0] * w1) + vs[2];
+    if (last) break;
+    if (row)
+      for (int p = 0; p < nb; ++p) send(L.X + at, p, x);
+    cluster_sync();
+    product();
+    g = row ? L.G[tid] + eta * x + chi : 0.0;
+    double vl[1] = {di * g};
+    cluster_sums<1>(L, sh, parity, vl, [&](double* t) { t[0] /= s1; });
+    if (row) g -= vl[0];
+    double vg[2] = {di * g * g, 0.0};
+    const double before = gz;
+    cluster_sums<2>(L, sh, parity, vg, [&](double* t) { t[1] = t[0] / before; });
+    gz = vg[0];
+    if (!(vg[1] <= 1e-3) && !(gz <= target)) {
+      failed = true;
+      break;
+    }
+    last = gz <= target || vg[1] * gz <= 1e-2 * target;
+    more = last || gz > gfloor;
+  }
+  // 4. Final charges: the constraint restored exactly.
+  double sx[1] = {x};
+  cluster_sums<1>(L, sh, parity, sx, [&](double* t) { t[0] = (Q - t[0]) / n; });
+  cluster_sync();  // no block leaves while another may still write to it
+  if (failed) {
+    if (L.rank == 0 && tid == 0) {
+      int* const retry = w.qretry + (adjoint ? 2 : 0);
+      w.qretry[4 + (adjoint ? w.S : 0) + atomicAdd(retry, 1)] = sys;
+    }
+    return;
+  }
+  if (L.rank == 0 && tid == 0) {
+    atomicMax(w.counts + 4, steps);
+    w.qiters[sys] = max(w.qiters[sys], steps);
+  }
+  if (!row) return;
+  const double q = x + sx[0];
+  if (adjoint) {
+    w.qadj[a] = q;
+    return;
+  }
+  w.q[a] = q;
+  w.a_e[(size_t)6 * w.A + a] = SELF_CONVERSION * (chi * q + 0.5 * eta * q * q);
+}
+
+cudaLaunchConfig_t cluster_config(int nb, int count, size_t bytes, cudaStream_t st, cudaLaunchAttribute* attr) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(nb * count);
+  cfg.blockDim = dim3(512);
+  cfg.dynamicSmemBytes = bytes;
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = nb;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
 }  // namespace
+
+int xr_qeq_direct_cluster_max(int nb) {
+  const int largest = nb == 8 ? kQeqDirectCluster8 : kQeqDirectCluster16;
+  bool ok = cudaFuncSetAttribute(k_qeq_direct_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)std::max(cluster_bytes(kQeqDirectCluster8, 8), cluster_bytes(kQeqDirectCluster16, 16))) ==
+            cudaSuccess;
+  if (nb > 8)  // past the portable cluster size
+    ok = ok && cudaFuncSetAttribute(k_qeq_direct_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
+  int clusters = 0;
+  if (ok) {
+    cudaLaunchAttribute attr[1];
+    cudaLaunchConfig_t cfg = cluster_config(nb, 1, cluster_bytes(largest, nb), nullptr, attr);
+    ok = cudaOccupancyMaxActiveClusters(&clusters, (void*)k_qeq_direct_cluster, &cfg) == cudaSuccess;
+  }
+  if (!ok) cudaGetLastError();
+  return ok && clusters > 0 ? largest : 0;
+}
+
+int xr_launch_qeq_direct_cluster(const XrWork& w, const XrFF& ff, cudaStream_t st, const int* list, int count, int largest, int nb,
+                                 bool adjoint) {
+  cudaLaunchAttribute attr[1];
+  cudaLaunchConfig_t cfg = cluster_config(nb, count, cluster_bytes(largest, nb), st, attr);
+  return (int)cudaLaunchKernelEx(&cfg, k_qeq_direct_cluster, w, ff, list, nb, adjoint ? 1 : 0);
+}
 
 bool xr_qeq_direct_ready() {
   const bool ok = cudaFuncSetAttribute(k_qeq_direct, cudaFuncAttributeMaxDynamicSharedMemorySize,
