@@ -96,6 +96,9 @@ struct XrSystem {
   int cell_base;
   double cell_f0[3];
   double cell_scale[3];
+  // Slots per atom of the rows that k_scan_rows leaves in cand_edge's memory (0: none), and the system's first one
+  int row_cap;
+  long long row_off;
   double rc, rc2, bond_cut, hb_cut;     // cutoff, cutoff^2, min(5, rc), min(7.5, rc)
   double inv_rc;                        // 1 / rc
   float cellf[9];
@@ -187,7 +190,9 @@ struct XrWork {
   int* atom_slot;
   int* cell_cnt;
   int* cell_atoms;
+  float4* cell_pos;           // [A] wrapped FP32 positions in the order of cell_atoms, the atom in the fourth word
   int ncells;
+  int row_cap;                // slots per atom of the rows that k_cell_rows leaves in cand_edge's memory
   // edges
   int2* edge;                 // {j, code}
   int* edge_pair;             // pair id of every edge (its own or its reverse's)
@@ -326,6 +331,10 @@ void xr_launch_topology(const XrWork& w, cudaStream_t st);  // xr_launch_prep, t
 void xr_launch_prep(const XrWork& w, cudaStream_t st);      // wrapped FP32 coordinates (k_prep)
 void xr_launch_count(const XrWork& w, cudaStream_t st);     // all-pairs image scan, counts (k_neighbors<false>)
 void xr_launch_rows(const XrWork& w, cudaStream_t st);      // all-pairs image scan, rows (k_neighbors<true>)
+// The image scan with its rows kept (XrSystem::row_cap; counts[6] set when a row did not fit), then, after
+// xr_launch_scan, the rows, pairs and bonds.
+void xr_launch_scan_rows(const XrWork& w, cudaStream_t st);
+void xr_launch_emit_rows(const XrWork& w, cudaStream_t st);
 int xr_launch_scan(const XrWork& w, cudaStream_t st);  // (this and the next four: the kernels launched)
 void xr_launch_topology_fill(const XrWork& w, cudaStream_t st);
 // Candidate list at the cutoff of w.sys (descriptors at rc + 2 skin): fill=false counts into cand_cnt
@@ -340,6 +349,13 @@ int xr_launch_cells(const XrWork& w, cudaStream_t st);
 // fill=false counts into cand_cnt, scans it (total into counts[5]) and records the longest row in
 // counts[6]; fill=true writes cand_edge.
 int xr_launch_cell_candidates(const XrWork& w, bool fill, cudaStream_t st);
+// The edges straight from the cell list, where an atom has one image of another at most within the cutoff (systems of at
+// most XR_RANK_ATOMS atoms, fewer than 2^24 in the call): counts and unordered rows of row_cap slots in
+// cand_edge's memory (the longest row in counts[6]), then, after xr_launch_scan, the rows, pairs and bonds in order
+// (`natoms`: the largest system's atoms).
+int xr_launch_cell_rows(const XrWork& w, cudaStream_t st);
+void xr_launch_rank_rows(const XrWork& w, int natoms, cudaStream_t st);
+#define XR_RANK_ATOMS 65536
 // Sorts every candidate row into canonical (j, Sx, Sy, Sz) order; rows hold at most max_row entries
 // (at most XR_ROW_SORT_MAX).
 void xr_launch_row_sort(const XrWork& w, int max_row, cudaStream_t st);

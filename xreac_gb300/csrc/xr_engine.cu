@@ -115,6 +115,10 @@ struct xr_ctx {
   size_t ccell_cnt = 0;
   int* cell_atoms = nullptr;
   size_t ccell_atoms = 0;
+  float4* cell_pos = nullptr;
+  size_t ccell_pos = 0;
+  int row_longest = 0;  // the longest row that did not fit the slots its system's density suggested
+  double row_scale = 1.0;  // slots of k_scan_rows' periodic rows over what the density suggests: grows when one did not fit
   // Skin reuse (xr_ctx_set_skin): the list of the last call is reused by a call on the same systems
   // (atom counts, types, cells, pbc, cutoff) in which no atom moved more than `skin` from where it was
   // when the list was built; the list holds every image within rc + 2 skin then (ASE's convention).
@@ -800,7 +804,7 @@ void keep_skin_list(xr_ctx* c, int nsys, int A, double rc) {
   c->cache_valid = true;
 }
 
-enum ListMode { kScan = 0, kBuild = 1, kReuse = 2, kSupplied = 3, kCell = 4 };
+enum ListMode { kScan = 0, kBuild = 1, kReuse = 2, kSupplied = 3, kCell = 4, kCellRows = 5, kScanRows = 6 };
 
 // Cell-list choice of a call whose list comes from a search (an image scan, or a skin-list build at
 // rl): per system, the grid of cell_grid stored in both descriptor sets; used when the searches'
@@ -844,6 +848,57 @@ long long plan_cells(xr_ctx* c, int nsys, const xr_system* sys, double rl, XrSys
     }
   }
   return use ? total : 0;
+}
+
+// Slots per row for a call whose rows come straight from the cell list (k_cell_rows): a third above what each
+// system's mean density gives, at least the longest row that exceeded that before; 0 where the call's systems do
+// not allow it (several images of an atom within the cutoff, too many atoms).
+int plan_cell_rows(const xr_ctx* c, int nsys, const xr_system* sys, int A, double rc) {
+  if (A >= 1 << 24) return 0;
+  double most = 0.0;
+  int largest = 0;
+  for (int s = 0; s < nsys; ++s) {
+    const XrSystem& S = c->host_sys[s];
+    if (S.cell_n[0] <= 0 || S.reach[0] || S.reach[1] || S.reach[2] || sys[s].natoms > XR_RANK_ATOMS) return 0;
+    const double* m = S.cell;
+    double volume = m[0] * (m[4] * m[8] - m[5] * m[7]) + m[1] * (m[5] * m[6] - m[3] * m[8]) + m[2] * (m[3] * m[7] - m[4] * m[6]);
+    for (int k = 0; k < 3; ++k)
+      if (!S.periodic[k]) volume *= S.cell_n[k] / S.cell_scale[k];  // the range of the positions
+    const double mean = sys[s].natoms / volume * (4.0 / 3.0 * 3.14159265) * rc * rc * rc;
+    most = std::max(most, std::min<double>(sys[s].natoms, 1.35 * mean + 64.0));
+    largest = std::max(largest, sys[s].natoms);
+  }
+  const double cap = std::min<double>(largest, std::max<double>(most, c->row_longest * 1.1));
+  return cap * A > 1e9 ? 0 : ((int)cap + 3) / 4 * 4;
+}
+
+// Slots of the image scan's rows (k_scan_rows): every atom of a small open system, a third above what the mean density
+// gives in a periodic cell, else nearly twice a liquid's row; rows of up to 900 words lie within a reservation of 450
+// directed edges per atom. Returns the entries in all, 0 where the call's systems do not allow it (too many atoms or
+// images).
+constexpr int kScanImages = 64;
+long long plan_scan_rows(xr_ctx* c, int nsys, const xr_system* sys, double rc) {
+  long long total = 0;
+  for (int s = 0; s < nsys; ++s) {
+    XrSystem& S = c->host_sys[s];
+    const int n = sys[s].natoms;
+    const long long images = (2ll * S.reach[0] + 1) * (2ll * S.reach[1] + 1) * (2ll * S.reach[2] + 1);
+    if (n > 65535 || images > kScanImages) return 0;
+    long long cap = n * images;
+    if (S.periodic[0] && S.periodic[1] && S.periodic[2]) {
+      const double* m = S.cell;
+      const double volume = m[0] * (m[4] * m[8] - m[5] * m[7]) + m[1] * (m[5] * m[6] - m[3] * m[8]) + m[2] * (m[3] * m[7] - m[4] * m[6]);
+      const double mean = n / volume * (4.0 / 3.0 * 3.14159265) * rc * rc * rc;
+      cap = std::min(cap, (long long)std::min(1e9, c->row_scale * 1.35 * mean + 64.0));
+    } else if (n > 896 || images > 1) {
+      cap = std::min(cap, (long long)(c->row_scale * 768.0));
+    }
+    S.row_cap = (int)cap;
+    S.row_off = total;
+    total += n * cap;
+    if (total > 1ll << 29) return 0;
+  }
+  return total;
 }
 
 // Everything the launch sequence after the list count depends on, other than data in device memory:
@@ -1011,14 +1066,31 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     }
   }
   long long ncells = 0;
+  int row_cap = 0;
   if (mode == kScan || mode == kBuild) {
     ncells = plan_cells(c, nsys, sys, mode == kBuild ? rc + 2.0 * c->skin : rc, mode == kBuild ? c->h_sys_list : nullptr);
     if (ncells > 0) {
       if (!grow(c, &c->atom_cell, &c->catom_cell, (size_t)A) || !grow(c, &c->atom_slot, &c->catom_slot, (size_t)A) ||
           !grow(c, &c->cell_atoms, &c->ccell_atoms, (size_t)A) || !grow(c, &c->cell_cnt, &c->ccell_cnt, (size_t)ncells + 1) ||
-          !grow(c, &c->cand_cnt, &c->ccand_cnt, (size_t)A + 1))
+          !grow(c, &c->cell_pos, &c->ccell_pos, (size_t)A) || !grow(c, &c->cand_cnt, &c->ccand_cnt, (size_t)A + 1))
         return cuda_fail(c, cudaErrorMemoryAllocation, "allocation");
-      if (mode == kScan) mode = kCell;
+      if (mode == kScan) {
+        mode = kCell;
+        row_cap = plan_cell_rows(c, nsys, sys, A, rc);
+        if (row_cap > 0) {
+          if (!grow(c, &c->cand_edge, &c->ccand_edge, ((size_t)A * row_cap + 1) / 2))
+            return cuda_fail(c, cudaErrorMemoryAllocation, "allocation");
+          mode = kCellRows;
+        }
+      }
+    }
+  }
+  if (mode == kScan) {
+    const long long slots = plan_scan_rows(c, nsys, sys, rc);
+    if (slots > 0) {
+      if (!grow(c, &c->cand_edge, &c->ccand_edge, (size_t)(slots + 1) / 2))
+        return cuda_fail(c, cudaErrorMemoryAllocation, "allocation");
+      mode = kScanRows;
     }
   }
   // energy-reduction chunks: each system's atoms in runs of XR_CHUNK_ATOMS, numbered in system order
@@ -1082,12 +1154,17 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     w.atom_slot = c->atom_slot;
     w.cell_cnt = c->cell_cnt;
     w.cell_atoms = c->cell_atoms;
+    w.cell_pos = c->cell_pos;
     w.ncells = (int)ncells;
+    w.row_cap = row_cap;
   }
   stage(c, 0, st);
   xr_launch_prep(w, st);  // also assigns every atom its cell when the call uses the cell list
   launches += 1;
-  if (mode == kScan || mode == kSupplied) {
+  if (mode == kScanRows) {
+    xr_launch_scan_rows(w, st);
+    launches += 1;
+  } else if (mode == kScan || mode == kSupplied) {
     // the image scan; for a supplied list only its coincident-atom check counts (xreac checks every
     // pair's minimum image whatever list it is given), and the filter's counts replace its own
     xr_launch_count(w, st);
@@ -1098,6 +1175,22 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     const long long m = c->h_cand_cnt[A];
     if (m > 0) cudaMemcpyAsync(c->cand_edge, c->h_cand_edge, sizeof(int2) * (size_t)m, cudaMemcpyHostToDevice, st);
     h2d += sizeof(int) * ((long long)A + 1) + sizeof(int2) * m;
+  }
+  if (mode == kCellRows) {
+    launches += xr_launch_cells(w, st);
+    launches += xr_launch_cell_rows(w, st);
+    launches += xr_launch_scan(w, st);
+    cudaMemcpyAsync(c->h_small, c->counts, 8 * sizeof(int), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(c->h_small + 8, c->status, sizeof(int), cudaMemcpyDeviceToHost, st);
+    d2h += 9 * sizeof(int);
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(c, e, "neighbour count");
+    if (int code = status_to_code(c, c->h_small[8])) return code;
+    if (c->h_small[6] > row_cap) {  // a row is longer than its slots: this call takes the candidate rows
+      c->row_longest = std::max(c->row_longest, c->h_small[6]);
+      cudaMemsetAsync(c->cnt, 0, sizeof(int) * 4 * ((size_t)A + 1), st);
+      cudaMemsetAsync(c->counts, 0, 8 * sizeof(int), st);
+      mode = kCell;
+    }
   }
   if (mode == kBuild || mode == kCell) {
     // every image within the list cutoff (rc + 2 skin for a skin list, with its descriptors; rc for
@@ -1137,21 +1230,27 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     }
     if (mode == kBuild) ++c->list_builds;
   }
-  if (mode != kScan) {
-    w.cand_cnt = c->cand_cnt;
-    w.cand_edge = c->cand_edge;
-    xr_launch_filter(w, false, st);
-    launches += 1;
+  if (mode != kCellRows) {  // (whose counts the host has)
+    if (mode != kScan && mode != kScanRows) {
+      w.cand_cnt = c->cand_cnt;
+      w.cand_edge = c->cand_edge;
+      xr_launch_filter(w, false, st);
+      launches += 1;
+    }
+    launches += xr_launch_scan(w, st);
+    cudaMemcpyAsync(c->h_small, c->counts, 8 * sizeof(int), cudaMemcpyDeviceToHost, st);
+    cudaMemcpyAsync(c->h_small + 8, c->status, sizeof(int), cudaMemcpyDeviceToHost, st);
+    d2h += 9 * sizeof(int);
+    if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(c, e, "neighbour count");
+    if (int code = status_to_code(c, c->h_small[8])) return code;
+    if (mode == kScanRows && c->h_small[6] != 0) {  // a row is longer than its slots: scan again for the rows
+      c->row_scale = std::min(64.0, c->row_scale * 1.5);
+      mode = kScan;
+    }
   }
-  launches += xr_launch_scan(w, st);
-  cudaMemcpyAsync(c->h_small, c->counts, 4 * sizeof(int), cudaMemcpyDeviceToHost, st);
-  cudaMemcpyAsync(c->h_small + 4, c->status, sizeof(int), cudaMemcpyDeviceToHost, st);
-  d2h += 5 * sizeof(int);
-  if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(c, e, "neighbour count");
   const int nE = c->h_small[0], nP = c->h_small[1], nB = c->h_small[2], nD = c->h_small[3];
-  if (int code = status_to_code(c, c->h_small[4])) return code;
   if (mode == kBuild) keep_skin_list(c, nsys, A, rc);
-  c->list_mode = mode == kBuild && ncells > 0 ? 5 : (int)mode;
+  c->list_mode = mode == kBuild && ncells > 0 ? 5 : mode == kCellRows ? (int)kCell : mode == kScanRows ? (int)kScan : (int)mode;
   if (!ensure_lists(c, nE, nP, nB)) return cuda_fail(c, cudaErrorMemoryAllocation, "list allocation");
   attach_lists(c, w);
   w.nE = nE;
@@ -1181,6 +1280,8 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     if (nlist > 0) std::memcpy(c->h_qsmall_p, c->h_qsmall.data(), sizeof(int) * nlist);
     h2d += sizeof(int4) * (long long)qteam + sizeof(int) * (long long)nlist;
   }
+  int largest_system = 0;
+  for (int s = 0; s < nsys; ++s) largest_system = std::max(largest_system, sys[s].natoms);
   const ResultLayout RL = result_layout(A, nsys, nB);
   if (!grow(c, &c->outbuf, &c->coutbuf, RL.end) || !host_grow(&c->h_out, &c->ch_out, RL.end))
     return cuda_fail(c, cudaErrorMemoryAllocation, "result block");
@@ -1240,6 +1341,10 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     stage(c, 1, st);
     if (mode == kScan)
       xr_launch_rows(w, st);
+    else if (mode == kCellRows)
+      xr_launch_rank_rows(w, largest_system, st);
+    else if (mode == kScanRows)
+      xr_launch_emit_rows(w, st);
     else
       xr_launch_filter(w, true, st);
     xr_launch_reverse(w, st);
@@ -1297,7 +1402,8 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
   bool done = false;
   if (c->graphs && !c->profile && qteam == 0) {
     const int ints[] = {(int)mode, qcluster ? 1 : 0, qcsize, qblocks, qteam, qsmall, qbig, nlist, nE > 0, nP > 0, nB > 0,
-                        (int)flags, dcount[0], dcount[1], dcount[2], dlargest[0], dlargest[1], dlargest[2], qd.nb};
+                        (int)flags, dcount[0], dcount[1], dcount[2], dlargest[0], dlargest[1], dlargest[2], qd.nb,
+                        largest_system};
     const void* ptrs[] = {c->h_qmap_p, c->h_qsmall_p, c->qmap, c->qsmall, c->outbuf};
     const int nptrs = (int)(sizeof(ptrs) / sizeof(ptrs[0]));
     const std::vector<unsigned char> kv = launch_key(w, ff->d, ints, (int)(sizeof(ints) / sizeof(int)), ptrs, nptrs);
@@ -1800,7 +1906,7 @@ void xr_ctx_destroy(xr_ctx* c) {
                   c->bond_i, c->bond_j, c->b_r, c->b_v, c->b_fwd, c->b_adj, c->b_e, c->dbrow, c->sys, c->energy,
                   c->props, c->status, c->counts, c->barrier, c->qmap, c->qsmall, c->qiters, c->qretry, c->red, c->qguess, c->qrhs, c->qadj, c->pgrad, c->bx_count,
                   c->arow, c->nact, c->nzrow, c->nnz, c->qb_first, c->qb_last, c->chunk_part, c->mids, c->nmids, c->mlist,
-                  c->cand_cnt, c->cand_edge, c->sys_list, c->atom_cell, c->atom_slot, c->cell_cnt, c->cell_atoms,
+                  c->cand_cnt, c->cand_edge, c->sys_list, c->atom_cell, c->atom_slot, c->cell_cnt, c->cell_atoms, c->cell_pos,
                   c->mid_tiles, c->qsplit};
   for (void* p : bufs)
     if (p) cudaFree(p);
@@ -2041,7 +2147,7 @@ int xr_ctx_reserve(xr_ctx* c, int atoms, int systems, long long edges, long long
       !grow(c, &c->cand_cnt, &c->ccand_cnt, (size_t)atoms + 1) ||
       !grow(c, &c->cand_edge, &c->ccand_edge, (size_t)std::max<long long>(edges, 1)) ||
       !grow(c, &c->atom_cell, &c->catom_cell, (size_t)atoms) || !grow(c, &c->atom_slot, &c->catom_slot, (size_t)atoms) ||
-      !grow(c, &c->cell_atoms, &c->ccell_atoms, (size_t)atoms) ||
+      !grow(c, &c->cell_atoms, &c->ccell_atoms, (size_t)atoms) || !grow(c, &c->cell_pos, &c->ccell_pos, (size_t)atoms) ||
       !grow(c, &c->cell_cnt, &c->ccell_cnt, 2 * (size_t)atoms + 64 * (size_t)systems + 1))
     return cuda_fail(c, cudaErrorMemoryAllocation, "reservation");
   return XR_OK;
@@ -2066,7 +2172,8 @@ long long xr_footprint_bytes(int atoms, int systems, long long edges, long long 
   const long long per_pair = 3 * sizeof(int) + 6 * sizeof(double);
   const long long per_bond = kBondBytes + 32;  // + the exported-bond record of the result block
   const long long chunks = (long long)systems + atoms / XR_CHUNK_ATOMS + 1;
-  const long long per_cells = 4 * sizeof(int) + 2 * sizeof(int);  // cand_cnt, atom_cell, atom_slot, cell_atoms, cell_cnt
+  // cand_cnt, atom_cell, atom_slot, cell_atoms, cell_cnt, cell_pos
+  const long long per_cells = 4 * sizeof(int) + 2 * sizeof(int) + sizeof(float4);
   const long long base = (long long)atoms * (per_atom + per_cells) + (long long)systems * (per_system + 64 * sizeof(int)) +
                          edges * (per_edge + sizeof(int2)) + (edges / 2) * per_pair + bonds * per_bond +
                          chunks * XR_PART_N * sizeof(double);
