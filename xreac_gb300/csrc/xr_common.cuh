@@ -314,7 +314,7 @@ enum AF { AF_DELTAP = 0, AF_TOTAL, AF_NLP, AF_VLPEX, AF_DLP, AF_DLPT, AF_SUMPI, 
 // sensitivities of the energy terms to total, d = total - valency, db = total - valency_boc and
 // sbo2; the rest are filled by the chain kernels.
 enum AJ { AJ_TOTAL = 0, AJ_D, AJ_DB, AJ_SBO2, AJ_OV1, AJ_OV2, AJ_DLPT, AJ_DLP, AJ_SUMPI, AJ_PRODSUM,
-          AJ_TOTAL_ALL, AJ_DELTAP, AJ_N };
+          AJ_TOTAL_ALL, AJ_N };
 // Per-bond forward slots in b_fwd.
 enum BF { BF_BO0 = 0, BF_PI0, BF_PP0, BF_DSIG, BF_DPI, BF_DPP, BF_BO, BF_PI, BF_PP, BF_SIG, BF_F1, BF_F4, BF_F5,
           BF_CORR, BF_MASK, BF_DF1I, BF_DF1J, BF_N };
@@ -380,13 +380,13 @@ int xr_launch_qeq_cluster(const XrWork& w, const XrFF& ff, cudaStream_t st, int 
                           int nbig, int nsmall, bool adjoint = false);
 // The streams of a call's launch sequence after the lists. The bonded terms need the lists and the
 // positions only, and the charges the pair kernel only, so the bond orders and bonded terms run beside
-// the pair kernel and the QEq solve, and the torsions and hydrogen bonds beside the angles; the parts
+// the pair kernel and the QEq solve, and the torsions, hydrogen bonds and per-atom and per-bond terms beside the angles; the parts
 // join before the bond-order chain's radial terms (which add to the pair kernel's) and the force
 // assembly. Without a fork (timed stages) every member is the call's own stream.
 struct XrFork {
   bool on;
-  cudaStream_t main, bonded, torsion, hbond;
-  cudaEvent_t lists, pairs, orders, atoms, torsions, hbonds, done;
+  cudaStream_t main, bonded, torsion, hbond, atom;
+  cudaEvent_t lists, pairs, orders, atoms, torsions, hbonds, done, atoms2;
   void record(cudaEvent_t e, cudaStream_t s) const {
     if (on) cudaEventRecord(e, s);
   }

@@ -101,8 +101,8 @@ struct xr_ctx {
   static constexpr size_t kGraphSeen = 4096;
   int last_graph = 0;  // of the last call: 0 launched directly, 1 recorded, 2 replayed
   // Side streams and events of the launch sequence (XrFork).
-  cudaStream_t side[6] = {};     // bonded, torsions, hydrogen bonds; the direct QEq solves' classes
-  cudaEvent_t fork_ev[11] = {};
+  cudaStream_t side[7] = {};     // bonded, torsions, hydrogen bonds; the direct QEq solves' classes; per-atom terms
+  cudaEvent_t fork_ev[12] = {};
   bool qeq_direct = false;       // the direct QEq solver fits the device's shared memory
   int direct8 = 0, direct16 = 0;  // the largest systems of its clusters of 8 and 16 blocks (0: not available)
   // Cell list (xr_ctx_set_cell_list): 0 chooses per call, 1 always, -1 never.
@@ -1288,7 +1288,8 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
   w.bx_rec = reinterpret_cast<XrBondRecord*>(c->outbuf + RL.bonds);
   const bool forked = !c->profile;
   const XrFork fork = {forked, st, forked ? c->side[0] : st, forked ? c->side[1] : st, forked ? c->side[2] : st,
-                       c->fork_ev[0], c->fork_ev[1], c->fork_ev[2], c->fork_ev[3], c->fork_ev[4], c->fork_ev[5], c->fork_ev[6]};
+                       forked ? c->side[6] : st, c->fork_ev[0], c->fork_ev[1], c->fork_ev[2], c->fork_ev[3], c->fork_ev[4],
+                       c->fork_ev[5], c->fork_ev[6], c->fork_ev[11]};
   // The charges: the CG solvers on the call's stream, each class of direct solves beside them on a stream of
   // its own (the first class takes the call's when there is no CG), then what those left to CG. The CG
   // launch comes first: its teams need whole SMs.
@@ -1380,7 +1381,7 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     launches += 3;
     stage(c, 6, st);
     if (!fork.on) xr_launch_bonded(w, ff->d, fork);
-    launches += 13;
+    launches += 12;
     stage(c, 7, st);
     fork.wait(st, fork.done);
     if (w.full_derivative) {  // adds to the pairs' radial terms, as the bond-order chain does

@@ -2281,7 +2281,7 @@ __global__ void k_pair_forces(XrWork w) {
 // warp instruction takes 64 cycles of the FP64 pipe), so chunks are small enough to spread over the
 // SMs, and the block's partials are summed slot by slot (a few adds per lane, then five shuffles)
 // rather than each warp reducing all 23 slots.
-constexpr int kReduceThreads = 128;
+constexpr int kReduceThreads = 256;  // (48 KB of partials)
 
 // Partial slots: 0..13 components, 14 mass, 15..17 mass * x, 18 charge, 19..21 charge * x, 22 finite.
 __global__ void __launch_bounds__(kReduceThreads) k_reduce_chunk(XrWork w, XrFF ff) {
@@ -2343,7 +2343,7 @@ __global__ void __launch_bounds__(kReduceThreads) k_reduce_chunk(XrWork w, XrFF 
 #pragma unroll
   for (int k = 0; k < XR_PART_N; ++k) part[k][tid] = v[k];
   __syncthreads();
-  // slot k by warp k % 4: four partials per lane in thread order, then the warp's butterfly (finite
+  // slot k by warp k % 8: eight partials per lane in thread order, then the warp's butterfly (finite
   // combines by min)
   const int lane = tid & 31, wid = tid >> 5;
   for (int k = wid; k < XR_PART_N; k += kReduceThreads / 32) {
