@@ -363,7 +363,7 @@ void xr_launch_row_sort(const XrWork& w, int max_row, cudaStream_t st);
 void xr_launch_reverse(const XrWork& w, cudaStream_t st);
 void xr_launch_pairs(const XrWork& w, const XrFF& ff, cudaStream_t st);
 int xr_launch_qeq(const XrWork& w, const XrFF& ff, cudaStream_t st, int nblocks, const int4* map, int nteam,
-                  const int* small, int nsmall, bool adjoint = false);
+                  int team_rows, const int* small, int nsmall, bool adjoint = false);
 void xr_launch_charge_response(const XrWork& w, const XrFF& ff, cudaStream_t st, int stage);
 // Parameter gradient of the QEq parameters from the charges and the adjoint solution (qadj):
 // chi and eta of every atom's type, the pair table's gamma of every pair's type.

@@ -248,6 +248,7 @@ struct xr_ctx {
   int* qsmall = nullptr;
   size_t cqsmall = 0;
   std::vector<int4> h_qmap;
+  int qteam_rows = 0;  // the most rows a block of the teams in h_qmap owns, before the splits move to molecules
   std::vector<int> h_qsmall;
   double* red = nullptr;
   size_t cred = 0;
@@ -677,7 +678,9 @@ void plan_qeq(xr_ctx* c, const xr_system* sys, int nsys, const std::vector<int>&
       std::sort(small.begin(), small.end(), [&](int a, int b) { return sys[a].natoms > sys[b].natoms; });
       c->h_qsmall.assign(small.begin(), small.end());
       c->h_qmap.clear();
+      c->qteam_rows = 0;
       for (size_t k = 0; k < large.size(); ++k) {
+        c->qteam_rows = std::max(c->qteam_rows, (sys[large[k]].natoms + team[k] - 1) / team[k]);
         const int first = (int)c->h_qmap.size();
         for (int r = 0; r < team[k]; ++r) c->h_qmap.push_back(make_int4(large[k], r, team[k], first));
       }
@@ -1313,7 +1316,7 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     }
     if (cg) {
       const int le = qcluster ? xr_launch_qeq_cluster(w, ff->d, st, qcsize, qblocks, c->qsmall, qbig, qsmall, adjoint)
-                              : xr_launch_qeq(w, ff->d, st, qblocks, c->qmap, qteam, c->qsmall, qsmall, adjoint);
+                              : xr_launch_qeq(w, ff->d, st, qblocks, c->qmap, qteam, c->qteam_rows, c->qsmall, qsmall, adjoint);
       launches += (qcluster ? qbig > 0 : qteam > 0) ? 2 : 1;  // the teams' row splits, then the solver
       if (le) return le;
     }

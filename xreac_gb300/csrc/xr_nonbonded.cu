@@ -223,14 +223,27 @@ __device__ bool grid_barrier(unsigned* bar, unsigned target, const XrWork& w, bo
 constexpr int kRedSmem = 8 * 32 + 16;
 __device__ inline double* result_slot(double* smem, int slot) { return smem + 256 + 8 * (slot & 1); }
 
+// Threads of a block that solves by conjugate gradients, and of one in a grid team whose blocks own at most
+// kTeamRows rows: half as many with twice the registers there, because the pipelined solver spills at
+// 64, and what 1,024 threads spill is more than the solver's shared memory leaves of the L1 cache; the
+// first warp's few instructions between an iteration's sums and its packets took 2,400 cycles instead
+// of 950 (QEq of the 4,608-atom water box 534 instead of 688 us). Blocks with more rows stream them
+// from L2 and want the warps: the 36,864-atom water box takes 2.5 ms with 1,024 threads, 3.1 ms with 512.
+constexpr int kQeqThreads = 1024, kTeamThreads = 512, kTeamRows = 64;
+
+template <int T>
 struct GridTeam {
+  static constexpr int kThreads = T;
   unsigned* bar;                // arrival counter of this team (zeroed before the launch)
   double* red;                  // the team's reduction slots: [slot][value][rank]
   int nb, rank;                 // blocks in the team and this block's rank
   mutable unsigned target = 0;  // barrier episodes so far times nb
+  mutable unsigned tag = 0;     // packet exchanges so far
+  // number of the team's current wait, barriers and packet exchanges together
+  __device__ unsigned episode() const { return target / nb + tag; }
   __device__ bool sync(const XrWork& w) const {
     target += nb;
-    return grid_barrier(bar, target, w, wait_poisoned(w, target / nb));
+    return grid_barrier(bar, target, w, wait_poisoned(w, episode()));
   }
   // Team-wide sum of NV block totals held by lane 0 of warp 0, fused with the barrier: lane 0
   // publishes the block's values into a fixed slot and arrives (release); after the bounded wait
@@ -238,7 +251,7 @@ struct GridTeam {
   // totals (scalar work that then costs no extra synchronisation), and every thread receives them.
   template <int NV, class Post>
   __device__ bool reduce(const XrWork& w, double* v, double* smem, int slot, Post post) const {
-    static_assert(NV <= 8, "at most eight values per reduction");
+    static_assert(NV <= 6, "at most six values per reduction: GridPackets keeps its packets in the last two");
     __shared__ int ok;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     target += nb;
@@ -297,77 +310,217 @@ struct GridTeam {
     for (int k = 0; k < NV; ++k) v[k] = res[k];
     return ok;
   }
-  // The same for NV <= 4 floats (the FP32 sweeps' scalars): slots of four floats per rank, one
-  // 16-byte load per rank, and FP32 sums. An FP64 add occupies this part's FP64 pipe for 64
-  // cycles per warp instruction, so the double form's 30 dependent adds for three values took
-  // about 1 us of the reduction.
-  template <int NV, class Post>
-  __device__ bool reducef(const XrWork& w, float* v, double* smem, int slot, Post post) const {
-    static_assert(NV <= 4, "at most four values per reduction");
-    __shared__ int ok;
+};
+
+// A grid team's exchange of rows and scalars by packets: values that carry the number of their exchange, so
+// that a reader needs no barrier, only the value. A row's packet is 8 bytes (value, tag), a rank's scalars
+// 16 (three floats, tag), each written and read by one relaxed access of its size. Exchanges alternate two
+// buffers: a rank writes for exchange k after it has read every rank's packets of k - 1, which each
+// sent after it had read those of k - 2.
+// The object lies in shared memory. In registers it was spilled, and the spilled values of 1024 threads
+// are more than what the solver's shared memory leaves of the L1 cache: the first warp's few
+// instructions between the sums and the packets then took 1,200 cycles instead of 360.
+//
+// The teams of 1,024 threads a block, whose systems are large, send their rows as plain floats: published by a
+// fence before the scalars' packet and read, four to a load, after every rank's has come. Packets
+// are twice the bytes in every block, and from some 10,000 rows on that costs more than the second trip to the L2 cache
+// (the 36,864-atom water box: 9 us for the packets of an iteration, 4 us for the floats).
+struct GridPackets {
+  uint4* scalars;  // rank 0's packet of even exchanges: the last two words of the team's reduction slots 1 and 2
+  float* rows[2];  // of the system's atoms, even and odd exchanges: packets, or plain floats
+  int nb, rank, n;
+  int odd;        // the system starts at an odd atom: 16-byte loads of row pairs begin half a pair early
+  unsigned fail;  // the exchange a test made unsatisfiable
+  template <int T>
+  __device__ void init(const XrWork& w, const GridTeam<T>& team, float* F, int a0, int n_) {
+    scalars = reinterpret_cast<uint4*>(team.red + 8 * (size_t)team.nb + 6);
+    constexpr bool plain = T > kTeamThreads;
+    for (int k = 0; k < 2; ++k) rows[k] = rows_of(w, F, k) + (plain ? 1 : 2) * (size_t)a0;
+    nb = team.nb;
+    rank = team.rank;
+    n = n_;
+    odd = a0 & 1;
+    fail = w.wait_fail_at > 0 ? w.wait_fail_at - team.target / team.nb : 0u;
+  }
+  // 8 bytes per atom and buffer, among the FP32 vectors that only the solver over global rows uses
+  static __device__ float* rows_of(const XrWork& w, float* F, int k) { return F + (k ? 6 : 2) * (size_t)w.A; }
+  __device__ uint4* scalar(unsigned tag, int r) const { return scalars + 4 * ((tag & 1u) * nb + r); }
+  // Once per solve, before a barrier: the rank's packets carry no tag of an earlier solve.
+  template <int T>
+  static __device__ void clear(const XrWork& w, const GridTeam<T>& team, float* F, int a0, int r0, int r1) {
+    for (int r = 2 * r0 + (int)threadIdx.x; r < 2 * r1; r += blockDim.x)
+      rows_of(w, F, 0)[2 * a0 + r] = rows_of(w, F, 1)[2 * a0 + r] = 0.0f;
+    if (threadIdx.x < 2)
+      *reinterpret_cast<uint4*>(team.red + ((1 + threadIdx.x) * (size_t)team.nb + team.rank) * 8 + 6) = make_uint4(0u, 0u, 0u, 0u);
+  }
+  template <bool plain>
+  __device__ void send_row(unsigned tag, int r, float v) const {
+    if constexpr (plain) {
+      rows[tag & 1u][r] = v;
+      return;
+    }
+    const unsigned long long x = (unsigned long long)tag << 32 | __float_as_uint(v);
+    asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(rows[tag & 1u] + 2 * r), "l"(x) : "memory");
+  }
+  // After a poll that found too little: whether the wait has run out.
+  static __device__ __noinline__ bool give_up(const XrWork& w, long long it) {
+    if (it > 256) __nanosleep(32);
+    if (it <= wait_cap(w, 1ll << 24) && ((it & 255) != 0 || !(*(volatile int*)w.status & XR_S_BARRIER))) return false;
+    atomicOr(w.status, XR_S_BARRIER);
+    return true;
+  }
+  // Exchange number `tag` (from 1, the rows sent before it): the sums over the team of the
+  // rows' acc (held by the first warp alone, or by the threads below m), added in rank order and so bit-identical
+  // in every block, to post(t, lane) on the first warp, and the system's n rows into yt. False when a
+  // wait ran out. Counting the blocks in on one word, then loading their sums, then the rows, took 5.2 of
+  // an iteration's 8.4 us on the 4,608-atom water box.
+  template <int kThreads, class Post>
+  __device__ __forceinline__ bool exchange(const XrWork& w, unsigned tag, float* acc, float* smem, bool one_warp, int m, float* yt,
+                                           Post post) const {
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    target += nb;
-    float* res = reinterpret_cast<float*>(result_slot(smem, slot));
-    float* rs = reinterpret_cast<float*>(red + (size_t)slot * 8 * nb);  // [rank][4]
+    constexpr bool plain = kThreads > kTeamThreads;
+    const unsigned want = tag == fail ? ~0u : tag;
+    bool good = true;
+    auto sums = [](float* v) {
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) {
+        const float x = __shfl_xor_sync(0xffffffffu, v[0], o), y = __shfl_xor_sync(0xffffffffu, v[1], o),
+                    z = __shfl_xor_sync(0xffffffffu, v[2], o);
+        v[0] += x;
+        v[1] += y;
+        v[2] += z;
+      }
+    };
+    if (!one_warp) {
+      const int rw = min((m + 31) >> 5, kThreads / 32);  // warps with rows
+      if (wid < rw) {
+        sums(acc);
+        if (lane < 3) smem[32 * lane + wid] = lane == 0 ? acc[0] : lane == 1 ? acc[1] : acc[2];
+      }
+      __syncthreads();
+      if (wid == 0)
+#pragma unroll
+        for (int k = 0; k < 3; ++k) acc[k] = lane < rw ? smem[32 * k + lane] : 0.0f;
+    }
     if (wid == 0) {
-      int good = 1;
-      __syncwarp();  // orders warp 0's row writes before lane 0's release
+      sums(acc);
+      if (plain) {
+        __syncwarp();
+        __threadfence();
+      }
       if (lane == 0) {
-        float4 o = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        if (NV > 0) o.x = v[0];
-        if (NV > 1) o.y = v[1];
-        if (NV > 2) o.z = v[2];
-        if (NV > 3) o.w = v[3];
-        reinterpret_cast<float4*>(rs)[rank] = o;
-        asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
-        const long long cap = wait_cap(w, 1ll << 24);
-        const bool poisoned = wait_poisoned(w, target / nb);
-        long long it = 0;
-        while (poisoned || ld_acquire(bar) < target) {
-          if (++it > cap || ((it & 255) == 0 && (*(volatile int*)w.status & XR_S_BARRIER))) {
-            atomicOr(w.status, XR_S_BARRIER);
-            good = 0;
+        const unsigned long long lo = (unsigned long long)__float_as_uint(acc[1]) << 32 | __float_as_uint(acc[0]);
+        const unsigned long long hi = (unsigned long long)tag << 32 | __float_as_uint(acc[2]);
+        asm volatile("{ .reg .b128 p; mov.b128 p, {%1, %2}; st.relaxed.gpu.global.b128 [%0], p; }" ::"l"(scalar(tag, rank)),
+                     "l"(lo), "l"(hi) : "memory");
+      }
+      if (one_warp && !plain) asm volatile("bar.arrive 1, %0;" ::"n"(kThreads) : "memory");
+      // each lane adds its ranks in order, then a fixed shuffle tree: deterministic
+      float t[3] = {0.0f, 0.0f, 0.0f};
+      for (int base = 0; base < nb && good; base += 5 * 32) {
+        unsigned long long lo[5], hi[5];
+        unsigned pend = 0;
+#pragma unroll
+        for (int u = 0; u < 5; ++u) {
+          lo[u] = hi[u] = 0;
+          if (base + lane + 32 * u < nb) pend |= 1u << u;
+        }
+        for (long long it = 0; pend;) {
+#pragma unroll
+          for (int u = 0; u < 5; ++u)
+            if (pend >> u & 1u)
+              asm volatile("{ .reg .b128 p; ld.relaxed.gpu.global.b128 p, [%2]; mov.b128 {%0, %1}, p; }"
+                           : "=l"(lo[u]), "=l"(hi[u]) : "l"(scalar(tag, base + lane + 32 * u)) : "memory");
+#pragma unroll
+          for (int u = 0; u < 5; ++u)
+            if ((pend >> u & 1u) && unsigned(hi[u] >> 32) == want) pend &= ~(1u << u);
+          if (pend && give_up(w, ++it)) {
+            good = false;
             break;
           }
-          if (it > 256) __nanosleep(32);
         }
-        ok = good;
+#pragma unroll
+        for (int u = 0; u < 5; ++u) {
+          t[0] += __uint_as_float(unsigned(lo[u]));
+          t[1] += __uint_as_float(unsigned(lo[u] >> 32));
+          t[2] += __uint_as_float(unsigned(hi[u]));
+        }
       }
+      if (plain) __threadfence();
       __syncwarp();
-      // each lane adds its ranks in order, then a fixed shuffle tree: deterministic
-      float t[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-      for (int base = 0; base < nb; base += 5 * 32) {
-        float4 x[5];
+      sums(t);
+      post(t, lane);
+    } else if (!plain) {
+      // the first warp's row phases run alone: polls before its packets left only took issue slots from it
+      if (one_warp) asm volatile("bar.sync 1, %0;" ::"n"(kThreads) : "memory");
+      // two rows per 16-byte load (each row's packet is whole by itself), five loads in flight
+      constexpr int kLoads = 5, kStep = 2 * (kThreads - 32);
+      for (int r = 2 * (int)(threadIdx.x - 32) - odd; r < n && good; r += kLoads * kStep) {
+        const unsigned long long* const p = reinterpret_cast<const unsigned long long*>(rows[tag & 1u]) + r;
+        unsigned pend = 0;
 #pragma unroll
-        for (int u = 0; u < 5; ++u) {
-          const int q = base + lane + 32 * u;
-          x[u] = q < nb ? __ldcg(reinterpret_cast<const float4*>(rs) + q) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        for (int u = 0; u < kLoads; ++u) {
+          const int q = r + u * kStep;
+          if (q >= 0 && q < n) pend |= 1u << 2 * u;
+          if (q + 1 < n) pend |= 2u << 2 * u;
         }
+        for (long long it = 0; pend;) {
+          unsigned long long x[kLoads], y[kLoads];
 #pragma unroll
-        for (int u = 0; u < 5; ++u) {
-          t[0] += x[u].x;
-          t[1] += x[u].y;
-          t[2] += x[u].z;
-          t[3] += x[u].w;
+          for (int u = 0; u < kLoads; ++u) {
+            const unsigned both = pend >> 2 * u & 3u;
+            x[u] = y[u] = 0;
+            if (both == 3u)
+              asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(x[u]), "=l"(y[u]) : "l"(p + u * kStep) : "memory");
+            else if (both == 1u)
+              asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(x[u]) : "l"(p + u * kStep) : "memory");
+            else if (both == 2u)
+              asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(y[u]) : "l"(p + u * kStep + 1) : "memory");
+          }
+#pragma unroll
+          for (int u = 0; u < kLoads; ++u) {
+            if ((pend >> 2 * u & 1u) && unsigned(x[u] >> 32) == want) {
+              yt[r + u * kStep] = __uint_as_float(unsigned(x[u]));
+              pend &= ~(1u << 2 * u);
+            }
+            if ((pend >> 2 * u & 2u) && unsigned(y[u] >> 32) == want) {
+              yt[r + u * kStep + 1] = __uint_as_float(unsigned(y[u]));
+              pend &= ~(2u << 2 * u);
+            }
+          }
+          if (pend && give_up(w, ++it)) {
+            good = false;
+            break;
+          }
         }
-      }
-#pragma unroll
-      for (int k = 0; k < NV; ++k) {
-        float s = t[k];
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        t[k] = s;
-      }
-      if (lane == 0) {
-        for (int k = 0; k < NV; ++k) res[k] = t[k];
-        post(res);
       }
     }
+    if (!plain) return __syncthreads_and(good);
+    if (!__syncthreads_and(good)) return false;
+    const float* const src = rows[tag & 1u];
+    // 16-byte loads from the first 16-byte boundary on, the few rows before it and after the last whole vector one by one
+    const int head = min(n, int((16 - (reinterpret_cast<uintptr_t>(src) & 15)) & 15) / 4), nv = (n - head) / 4;
+    const float4* const src4 = reinterpret_cast<const float4*>(src + head);
+    for (int q = threadIdx.x; q < nv; q += kThreads) {
+      const float4 v = __ldcg(src4 + q);
+      float* d = yt + head + 4 * q;
+      d[0] = v.x;
+      d[1] = v.y;
+      d[2] = v.z;
+      d[3] = v.w;
+    }
+    const int rest = head + 4 * nv;
+    if ((int)threadIdx.x < head) yt[threadIdx.x] = __ldcg(src + threadIdx.x);
+    if ((int)threadIdx.x < n - rest) yt[rest + threadIdx.x] = __ldcg(src + rest + threadIdx.x);
     __syncthreads();
-    for (int k = 0; k < NV; ++k) v[k] = res[k];
-    return ok;
+    return true;
   }
 };
+
+template <class Team>
+constexpr bool is_grid = false;
+template <int T>
+constexpr bool is_grid<GridTeam<T>> = true;
 
 struct BlockTeam {
   __device__ bool sync(const XrWork&) const {
@@ -597,7 +750,7 @@ struct QeqRows {
 struct QeqShared {
   double red[kRedSmem];
   double sc_lam, sc_alpha, sc_step, sc_beta;
-  float sf_lam, sf_alpha, sf_step, sf_beta, sf_gz, sf_stop, sf_shift, sf_aold;
+  float sf_lam, sf_alpha, sf_step, sf_beta, sf_gz, sf_stop, sf_shift, sf_rgz, sf_raold;
   double sd_s1w;  // <1, M^-1 1> of the FP32 row solver's block-Jacobi preconditioner
   // Scalars of the solve formed once, by the thread that runs a reduction's post hook (a division
   // done by every warp would cost the FP64 pipe once per warp): the start multipliers, the target,
@@ -608,6 +761,9 @@ struct QeqShared {
   double cred[2][8][8];  // cluster team: partials pushed by the blocks of the cluster
   unsigned cseq[2][8];   // cluster team: exchange number of each pushed entry
   int sc_state;  // 0 iterate, 1 converged, 2 stop
+  GridPackets link;            // grid team: the row solver's exchanges and what else its first warp reads alone
+  float sf_rs1;
+  int sc_budget;
   union {
     double d[32][33];
     float f[32][33];
@@ -740,24 +896,26 @@ __device__ int qeq_cg(const XrWork& w, const double* atab, const Team& team, Qeq
     }
     T php0 = T(0), php1 = T(0);  // lane partials in warp 0: p'Hp and <D^-1, Hp>
     for (int tb = r0; tb < r1; tb += 32) {
-      const int r = tb + wid;
-      T hz = T(0);
-      if (wid < 32 && r < r1) {
-        const int a = a0 + r;
-        const int eb = w.cnt[a], ee = w.cnt[a + 1];
-        if (M.cached && M.gstage) {
-          for (int e = eb + lane; e < ee; e += 32) hz += M.cache_h[e - M.ebeg] * M.gstage[M.cache_j[e - M.ebeg]];
-        } else if (M.cached) {
-          for (int e = eb + lane; e < ee; e += 32) hz += M.cache_h[e - M.ebeg] * __ldcg(G + a0 + M.cache_j[e - M.ebeg]);
-        } else {
-          for (int e = eb + lane; e < ee; e += 32) {
-            const int j = w.edge[e].x;
-            const double h = M.scaled ? w.hval[e] : w.hval[e] * __ldcg(DI + j);
-            hz += T(h) * __ldcg(G + j);
+      for (int k = wid; k < 32; k += blockDim.x >> 5) {
+        const int r = tb + k;
+        T hz = T(0);
+        if (r < r1) {
+          const int a = a0 + r;
+          const int eb = w.cnt[a], ee = w.cnt[a + 1];
+          if (M.cached && M.gstage) {
+            for (int e = eb + lane; e < ee; e += 32) hz += M.cache_h[e - M.ebeg] * M.gstage[M.cache_j[e - M.ebeg]];
+          } else if (M.cached) {
+            for (int e = eb + lane; e < ee; e += 32) hz += M.cache_h[e - M.ebeg] * __ldcg(G + a0 + M.cache_j[e - M.ebeg]);
+          } else {
+            for (int e = eb + lane; e < ee; e += 32) {
+              const int j = w.edge[e].x;
+              const double h = M.scaled ? w.hval[e] : w.hval[e] * __ldcg(DI + j);
+              hz += T(h) * __ldcg(G + j);
+            }
           }
         }
+        part[k][lane] = hz;
       }
-      if (wid < 32) part[wid][lane] = hz;
       __syncthreads();
       if (wid < 4) {  // lane = row of the tile; warp k adds lanes 8k .. 8k+7 of the row's partials
         T s = part[lane][8 * wid];
@@ -894,9 +1052,8 @@ __device__ inline int row_group(int m, int entries = 0) {
 // runs post(t) on the totals t[0..NV) (bit-identical in every block) and the block waits for it.
 // Returns false when a team exchange gave up.
 template <int NV, class Team, class Post>
-__device__ inline bool team_sumf(const Team& team, const XrWork& w, float* v, float* smem, Post post, int* slot) {
+__device__ inline bool team_sumf(const Team& team, const XrWork& w, float* v, float* smem, Post post) {
   constexpr bool kCluster = std::is_same<Team, ClusterTeam>::value;
-  constexpr bool kGrid = std::is_same<Team, GridTeam>::value;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
 #pragma unroll
   for (int k = 0; k < NV; ++k) v[k] = warp_total_t<float>(v[k]);
@@ -904,14 +1061,6 @@ __device__ inline bool team_sumf(const Team& team, const XrWork& w, float* v, fl
 #pragma unroll
     for (int k = 0; k < NV; ++k) smem[32 * k + wid] = v[k];
   __syncthreads();
-  if constexpr (kGrid) {
-    float f[NV];
-#pragma unroll
-    for (int k = 0; k < NV; ++k) f[k] = wid == 0 ? warp_total_t<float>(lane < nw ? smem[32 * k + lane] : 0.0f) : 0.0f;
-    const bool ok = team.template reducef<NV>(w, f, reinterpret_cast<double*>(smem), *slot, post);
-    *slot = *slot == 1 ? 2 : 1;
-    return ok;
-  }
   bool good = true;
   if (wid == 0) {
     float x[NV];
@@ -941,9 +1090,9 @@ __device__ inline bool team_sumf(const Team& team, const XrWork& w, float* v, fl
 // for a system of n atoms of which this block owns m rows (r0 .. r1):
 //   yt[n4]  D v for every row of the system (v = M^-1 of the vector being multiplied), the vector the
 //           product gathers; n4 = n rounded up to a multiple of 4; two such buffers for a cluster
+//   binv[8m] row r of its group's inverse block (columns: the group's rows in order, zeros past them)
 //   own rows, a record each: the constants D_ii, eta D^-1, c = H w1, w1 = M^-1 1, then the solver's
 //           x (the correction), p, s, r, u, and for the pipelined solver of grid teams q, z, w, m~, hv
-//   binv[8m] row r of its group's inverse block (columns: the group's rows in order)
 //   rp[m + 1] row starts relative to the cache; first[m], size[m] the group of each row (16-bit)
 // M is block-Jacobi: groups of at most 8 consecutive own rows whose atoms are joined by distances
 // below 1.3 A (molecules), each block H restricted to the group. One-row groups are Jacobi.
@@ -952,7 +1101,7 @@ __device__ inline bool team_sumf(const Team& team, const XrWork& w, float* v, fl
 // 1e-7 (about 3e-4) for the pipelined CG of grid teams.
 template <class Team>
 __host__ __device__ constexpr double sweep_ratio32() {
-  return std::is_same<Team, GridTeam>::value ? 1e-7 : 1e-10;
+  return is_grid<Team> ? 1e-7 : 1e-10;
 }
 
 // A team splits a system's rows between its blocks, and each block forms its block-Jacobi groups from
@@ -996,7 +1145,7 @@ __host__ __device__ constexpr int rows32_yt_buffers() {
 // the row stride odd (a thread per row then meets no bank conflict).
 template <class Team>
 __host__ __device__ constexpr int rows32_vectors() {
-  return std::is_same<Team, GridTeam>::value ? 15 : 9;
+  return is_grid<Team> ? 15 : 9;
 }
 
 // One record of consecutive values per row: a row's values lie at constant offsets from one address (a
@@ -1012,9 +1161,9 @@ struct Rows32 {
     float* f = reinterpret_cast<float*>(base);
     n4 = (n + 3) / 4 * 4;
     yt = f;
-    rec = f + rows32_yt_buffers<Team>() * n4;
-    binv = rec + kStride * m;
-    rp = reinterpret_cast<int*>(binv + kGroupMax * m);
+    binv = f + rows32_yt_buffers<Team>() * n4;
+    rec = binv + kGroupMax * m;
+    rp = reinterpret_cast<int*>(rec + kStride * m);
     first = reinterpret_cast<unsigned short*>(rp + m + 1);
     size = first + m;
   }
@@ -1035,6 +1184,26 @@ struct Rows32 {
   __device__ float& hv(int i) const { return at(13, i); }
   // FP32 scratch of the setup, 8 per row over the records
   __device__ float* scratch32() const { return rec; }
+  // Row i of M^-1 v: its row of the group's inverse block times value v of the group's rows. All loads at once (a
+  // row alone on its thread waits for each: a loop over the group took 0.8 us).
+  __device__ float group_apply(int v, int i) const {
+    static_assert(kGroupMax == 8, "two 16-byte loads of the inverse's row");
+    const int f = first[i], k = size[i];
+    const float4* bi = reinterpret_cast<const float4*>(binv + kGroupMax * i);
+    const float4 b0 = bi[0], b1 = bi[1];
+    float x[kGroupMax];
+#pragma unroll
+    for (int b = 0; b < kGroupMax; ++b) x[b] = b < k ? at(v, f + b) : 0.0f;
+    float t = b0.x * x[0];
+    t += b0.y * x[1];
+    t += b0.z * x[2];
+    t += b0.w * x[3];
+    t += b1.x * x[4];
+    t += b1.y * x[5];
+    t += b1.z * x[6];
+    t += b1.w * x[7];
+    return t;
+  }
   // buffer k of the gathered vector (a cluster team alternates two)
   __device__ float* ytb(int k) const { return yt + (k & 1) * n4; }
 };
@@ -1103,7 +1272,7 @@ __device__ __noinline__ bool qeq_rows32_setup(const XrWork& w, const double* ata
                                               int n, int r0, int r1, const QeqMatrix<float>& M, float* gyt) {
   extern __shared__ __align__(16) unsigned char qeq_dyn[];
   constexpr bool kCluster = std::is_same<Team, ClusterTeam>::value;
-  constexpr bool kGrid = std::is_same<Team, GridTeam>::value;
+  constexpr bool kGrid = is_grid<Team>;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, tid = threadIdx.x;
   const int m = r1 - r0;
   const Rows32<Team> R(qeq_dyn, n, m);
@@ -1247,6 +1416,15 @@ __device__ __noinline__ bool qeq_rows32_setup(const XrWork& w, const double* ata
     for (int q = tid; q < n; q += blockDim.x) R.yt[q] = __ldcg(gyt + a0 + q);
     __syncthreads();
   }
+  if constexpr (kGrid) {
+    if (!__isShared(M.cache_h)) {
+      stream_rows(M.cache_h, M.cache_j, M.ebeg, R.rp, m, R.yt, &R.cw(0), R.kStride);
+      __syncthreads();
+      for (int i = tid; i < m; i += blockDim.x) R.cw(i) += R.etadi(i) * R.yt[r0 + i];
+      __syncthreads();
+      return true;
+    }
+  }
   for (int ib = wid * gpw; ib < m; ib += nw * gpw) {
     const int i = ib + lane / gs;
     float t = 0.0f;
@@ -1274,7 +1452,7 @@ __device__ __noinline__ bool qeq_rows32_setup(const XrWork& w, const double* ata
 // layout's r, s and u). The correction x of the own rows is written to y_out (global, by atom).
 template <class Team>
 __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, QeqShared& sh, int a0, int n, int r0,
-                                          int r1, const QeqMatrix<float>& M, float* y_out, double ratio, int max_it, int* slot) {
+                                          int r1, const QeqMatrix<float>& M, float* y_out, double ratio, int max_it) {
   extern __shared__ __align__(16) unsigned char qeq_dyn[];
   constexpr bool kCluster = std::is_same<Team, ClusterTeam>::value;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, tid = threadIdx.x;
@@ -1304,13 +1482,6 @@ __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, Qeq
         if (r != team.rank) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_map(remote, r)), "f"(v) : "memory");
     }
   };
-  auto group_apply = [&](int i) {  // (M^-1 g)_i over the group of row i
-    const int f = R.first[i], k = R.size[i];
-    const float* bi = R.binv + kGroupMax * i;
-    float t = 0.0f;
-    for (int b = 0; b < k; ++b) t += bi[b] * R.rr(f + b);
-    return t;
-  };
   for (int i = tid; i < m; i += blockDim.x) {
     R.rr(i) = float(__ldcg(G + a0 + r0 + i));
     R.p(i) = 0.0f;
@@ -1320,7 +1491,7 @@ __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, Qeq
   __syncthreads();
   float u0 = 0.0f, u1 = 0.0f;
   for (int i = tid; i < m; i += blockDim.x) {
-    const float y = group_apply(i);
+    const float y = R.group_apply(7, i);
     R.u(i) = y;
     publish(i, y * R.dd(i));
     u0 += R.wv(i) * R.rr(i);
@@ -1336,7 +1507,7 @@ __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, Qeq
         sh.sf_gz = gz;
         sh.sf_stop = float(ratio) * gz;
         sh.sc_state = (!(gz > 0.0f) || n < 2) ? 1 : 0;
-      }, slot))
+      }))
     return -1;
   const float* yt = yt_of(buf);
   const float fstop = sh.sf_stop;
@@ -1393,7 +1564,7 @@ __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, Qeq
             sh.sf_alpha = gz / t[0];
             sh.sf_step = sh.sf_alpha * t[1] / s1;
           }
-        }, slot))
+        }))
       return -1;
     if (sh.sc_state != 0) break;
     const float alpha = sh.sf_alpha, step = sh.sf_step;
@@ -1406,7 +1577,7 @@ __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, Qeq
     u1 = 0.0f;
     buf ^= 1;
     for (int i = tid; i < m; i += blockDim.x) {
-      const float y = group_apply(i);
+      const float y = R.group_apply(7, i);
       R.u(i) = y;
       publish(i, y * R.dd(i));
       u0 += R.wv(i) * R.rr(i);
@@ -1421,7 +1592,7 @@ __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, Qeq
           sh.sf_beta = gzn / sh.sf_gz;
           sh.sf_gz = gzn;
           if (gzn <= fstop) sh.sc_state = 1;
-        }, slot))
+        }))
       return -1;
     yt = yt_of(buf);
   }
@@ -1452,24 +1623,21 @@ __device__ __noinline__ int qeq_cg_rows32(const XrWork& w, const Team& team, Qeq
 //
 // The product gathers yt = D m~ over the pre-scaled rows (H'_ij = H_ij / D_jj). A group of lanes
 // per row forms the product and its first lane the updates; a thread per row the partial sums and
-// the group products M^-1 w. Every block writes its rows' D m~ to global memory before the
-// reduction and stages the whole vector after it, alternating two global buffers (gyt0, gyt1): a
-// block writes buffer k & 1 for exchange k only after exchange k - 1, which every block entered
-// after staging exchange k - 2's buffer. (Written for any team: a cluster alternates two shared
-// buffers the same way.) The iteration stops when gamma falls to `ratio` times its start value.
+// the group products M^-1 w. The rows' D m~ and the scalars travel as tagged packets
+// (GridPackets). The iteration stops when gamma falls to
+// `ratio` times its start value.
 // The correction y of the own rows is written to y_out (global, indexed by atom).
 // kStream: the rows stream from global memory (stream_rows) instead of lying in this block's shared
 // memory; two instances, so that neither spills for the other's sake.
-template <class Team, bool kStream>
-__device__ __noinline__ int qeq_cg_rows32_pipelined(const XrWork& w, const Team& team, QeqShared& sh, int a0, int n,
+template <bool kStream, int kThreads>
+__device__ __noinline__ int qeq_cg_rows32_pipelined(const XrWork& w, const GridTeam<kThreads>& team, QeqShared& sh, int a0, int n,
                                                     int r0, int r1, const QeqMatrix<float>& M, float* y_out,
-                                                    double ratio, int max_it, float* gyt0, float* gyt1, int* slot) {
+                                                    double ratio, int max_it, float* F) {
   extern __shared__ __align__(16) unsigned char qeq_dyn[];
-  constexpr bool kCluster = std::is_same<Team, ClusterTeam>::value;
-  constexpr bool kGrid = std::is_same<Team, GridTeam>::value;
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, tid = threadIdx.x;
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, tid = threadIdx.x;
+  constexpr int nw = kThreads / 32;
   const int m = r1 - r0;
-  const Rows32<Team> R(qeq_dyn, n, m);
+  const Rows32<GridTeam<kThreads>> R(qeq_dyn, n, m);
   // the row cache in this block's shared memory (offsets from the dynamic base: shared-memory loads)
   const float* const ch_s = reinterpret_cast<const float*>(
       qeq_dyn + (kStream ? 0 : reinterpret_cast<const unsigned char*>(M.cache_h) - qeq_dyn));
@@ -1477,89 +1645,59 @@ __device__ __noinline__ int qeq_cg_rows32_pipelined(const XrWork& w, const Team&
       qeq_dyn + (kStream ? 0 : reinterpret_cast<const unsigned char*>(M.cache_j) - qeq_dyn));
   const double* G = &QW(Q_G, 0);
   float* red = reinterpret_cast<float*>(sh.red);
-  const float s1 = float(sh.sd_s1w);
-  // exchange parity: the setup's product gathered buffer 0, so the first exchange writes buffer 1
-  int buf = 1;
-  auto yt_of = [&](int k) -> float* { return kCluster ? R.ytb(k) : R.yt; };
-  auto publish = [&](int i, float v) {  // D m~ of own row i, here and in the other blocks
-    float* yt = yt_of(buf);
-    yt[r0 + i] = v;
-    if constexpr (kCluster) {
-      const unsigned remote = smem_u32(yt + r0 + i);
-      for (int r = 0; r < team.nb; ++r)
-        if (r != team.rank) asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(cluster_map(remote, r)), "f"(v) : "memory");
-    }
-    if constexpr (kGrid) (buf ? gyt1 : gyt0)[a0 + r0 + i] = v;  // the other blocks stage it after the reduction
+  GridPackets& link = sh.link;
+  unsigned tag = team.tag;
+  if (tid == 0) {
+    link.init(w, team, F, a0, n);
+    sh.sf_rs1 = 1.0f / float(sh.sd_s1w);
+    sh.sc_budget = max_it;
+  }
+  float* const yt = R.yt;
+  // The phases of one row per thread: by the first warp alone up to two rows a lane (a block barrier between two
+  // of them costs more than the second row), else by all threads.
+  const bool one_warp = m <= 64;
+  const int row0 = one_warp && wid > 0 ? m : tid, row_step = one_warp ? 32 : kThreads;
+  auto rows_sync = [&]() {
+    if (one_warp) __syncwarp();
+    else __syncthreads();
   };
-  auto stage = [&]() {  // a grid team's whole yt from global memory, after the reduction that published it
-    if constexpr (kGrid) {
-      const float* src = (buf ? gyt1 : gyt0) + a0;
-      // 16-byte loads from the first 16-byte boundary on; the few elements before it and after the
-      // last whole vector one by one
-      const int head = min(n, int((16 - (reinterpret_cast<uintptr_t>(src) & 15)) & 15) / 4);
-      const int nv4 = (n - head) / 4;
-      const float4* src4 = reinterpret_cast<const float4*>(src + head);
-      for (int q = tid; q < nv4; q += blockDim.x) {
-        const float4 v = __ldcg(src4 + q);
-        float* d = R.yt + head + 4 * q;
-        d[0] = v.x;
-        d[1] = v.y;
-        d[2] = v.z;
-        d[3] = v.w;
-      }
-      const int rest = head + 4 * nv4;
-      if (tid < head) R.yt[tid] = __ldcg(src + tid);
-      if (tid < n - rest) R.yt[rest + tid] = __ldcg(src + rest + tid);
-      __syncthreads();
-    }
-  };
-  auto group_apply = [&](int v, int i) {  // M^-1 of the rows' value v, row i: over its group
-    const int f = R.first[i], k = R.size[i];
-    const float* bi = R.binv + kGroupMax * i;
-    float t = 0.0f;
-    for (int b = 0; b < k; ++b) t += bi[b] * R.at(v, f + b);
-    return t;
-  };
-  // lanes per row: the fewest that take the block's rows in one pass over its warps (a block of 33
-  // rows would otherwise give its first warp a second row, and the team waits for that block)
+  // lanes per row: those that take the block's rows in the fewest steps
   int gs = 32;
-  while (gs > 4 && m * gs > (int)blockDim.x) gs >>= 1;
+  for (int g = 16; g >= 4; g >>= 1)
+    if ((m * g + kThreads - 1) / kThreads * 32 < (m * gs + kThreads - 1) / kThreads * (32 * g / gs)) gs = g;
   const int sub = lane & (gs - 1), gpw = 32 / gs;
-  // The product H'yt over the cached rows (gs lanes per row, four entries per lane in flight: the rows
-  // may stream from L2 rather than shared memory); the first lane of the row's group then runs
-  // epi(i, sum) with the off-diagonal sum (the diagonal term is etadi * yt).
-  auto product = [&](auto epi) {
-    const float* yt = yt_of(buf);
-    auto row_dot = [&](const float* ch, const unsigned short* cj, int e, int ee) {
-      float t = 0.0f;
-      for (; e + 3 * gs < ee; e += 4 * gs) {
-        const float h0 = ch[e], h1 = ch[e + gs], h2 = ch[e + 2 * gs], h3 = ch[e + 3 * gs];
-        const int j0 = cj[e], j1 = cj[e + gs], j2 = cj[e + 2 * gs], j3 = cj[e + 3 * gs];
-        t += h0 * yt[j0];
-        t += h1 * yt[j1];
-        t += h2 * yt[j2];
-        t += h3 * yt[j3];
-      }
-      for (; e < ee; e += gs) t += ch[e] * yt[cj[e]];
-      return t;
-    };
+  // The off-diagonal sums of H'yt over the cached rows into hv, gs lanes per row with four entries per lane in
+  // flight; the diagonal term (etadi yt) and the updates follow with a thread per row (by the lanes that
+  // hold the sums, one per row, they cost every warp's issue and shared-memory slots).
+  auto product = [&]() {
     if constexpr (!kStream) {
       for (int ib = wid * gpw; ib < m; ib += nw * gpw) {
         const int i = ib + lane / gs;
         float t = 0.0f;
-        if (i < m) t = row_dot(ch_s, cj_s, R.rp[i] + sub, R.rp[i + 1]);
+        if (i < m) {
+          int e = R.rp[i] + sub;
+          const int ee = R.rp[i + 1];
+          for (; e + 3 * gs < ee; e += 4 * gs) {
+            const float h0 = ch_s[e], h1 = ch_s[e + gs], h2 = ch_s[e + 2 * gs], h3 = ch_s[e + 3 * gs];
+            const int j0 = cj_s[e], j1 = cj_s[e + gs], j2 = cj_s[e + 2 * gs], j3 = cj_s[e + 3 * gs];
+            t += h0 * yt[j0];
+            t += h1 * yt[j1];
+            t += h2 * yt[j2];
+            t += h3 * yt[j3];
+          }
+          for (; e < ee; e += gs) t += ch_s[e] * yt[cj_s[e]];
+        }
         for (int o = gs / 2; o > 0; o >>= 1) t += __shfl_xor_sync(0xffffffffu, t, o);
-        if (sub == 0 && i < m) epi(i, t + R.etadi(i) * yt[r0 + i]);
+        if (sub == 0 && i < m) R.hv(i) = t;
       }
     } else {
       stream_rows(M.cache_h, M.cache_j, M.ebeg, R.rp, m, yt, &R.hv(0), R.kStride);
-      __syncthreads();
-      for (int i = tid; i < m; i += blockDim.x) epi(i, R.hv(i) + R.etadi(i) * yt[r0 + i]);
     }
+    __syncthreads();
   };
   // start: r = -g0, u~ = M^-1 r exchanged with the reduction of <w1, r> and <r, u~>; then
   // u = u~ - w1 <w1, r>/s1 and w = H u = H u~ - c <w1, r>/s1
-  for (int i = tid; i < m; i += blockDim.x) {
+  for (int i = row0; i < m; i += row_step) {
     R.rr(i) = -float(__ldcg(G + a0 + r0 + i));
     R.x(i) = 0.0f;
     R.p(i) = 0.0f;
@@ -1569,87 +1707,101 @@ __device__ __noinline__ int qeq_cg_rows32_pipelined(const XrWork& w, const Team&
   }
   __syncthreads();
   float acc[3] = {0.0f, 0.0f, 0.0f};
-  for (int i = tid; i < m; i += blockDim.x) {
-    const float t = group_apply(7, i);
+  ++tag;
+  for (int i = row0; i < m; i += row_step) {
+    const float t = R.group_apply(7, i);
     R.u(i) = t;
-    publish(i, t * R.dd(i));
+    link.template send_row<(kThreads > kTeamThreads)>(tag, r0 + i, t * R.dd(i));
     acc[0] += R.wv(i) * R.rr(i);
     acc[1] += R.rr(i) * t;
   }
-  if (!team_sumf<2>(team, w, acc, red, [&](const float* t) {
-        const float shift = t[0] / s1;
+  if (!link.template exchange<kThreads>(w, tag, acc, red, one_warp, m, yt, [&](const float* t, int l) {
+        const float shift = t[0] * sh.sf_rs1;
         const float gam = t[1] - shift * t[0];  // <r, P r>
-        sh.sf_shift = shift;
-        sh.sf_stop = float(ratio) * gam;
-        sh.sc_state = (!(gam > 0.0f) || n < 2) ? 1 : 0;
-      }, slot))
+        if (l == 0) {
+          sh.sf_shift = shift;
+          sh.sf_stop = float(ratio) * gam;
+          sh.sc_state = (!(gam > 0.0f) || link.n < 2) ? 1 : 0;
+        }
+      }))
     return -1;
-  stage();
-  if (sh.sc_state == 0) {
+  acc[0] = acc[1] = acc[2] = 0.0f;
+  int state = sh.sc_state;  // (read between the exchange's barrier and the product's: warp 0 may be first to the next)
+  if (state == 0) {
+    product();
     const float shift = sh.sf_shift;
-    product([&](int i, float hv) {
-      R.wq(i) = hv - shift * R.cw(i);
-      R.u(i) -= shift * R.wv(i);
-    });
-    __syncthreads();  // the group products read the other rows of the group
-  }
-  const float fstop = sh.sf_stop;
-  int it = 0;
-  while (sh.sc_state == 0) {
-    buf ^= 1;
-    acc[0] = acc[1] = acc[2] = 0.0f;
-    for (int i = tid; i < m; i += blockDim.x) {
-      const float t = group_apply(11, i);
-      R.mt(i) = t;
-      publish(i, t * R.dd(i));
-      acc[0] += R.rr(i) * R.u(i);
-      acc[1] += R.wq(i) * R.u(i);
-      acc[2] += R.wv(i) * R.wq(i);
+    for (int i = row0; i < m; i += row_step) {
+      const float wv = R.hv(i) + R.etadi(i) * yt[r0 + i] - shift * R.cw(i);
+      const float uv = R.u(i) - shift * R.wv(i), rv = R.rr(i);
+      R.wq(i) = wv;
+      R.u(i) = uv;
+      acc[0] += rv * uv;
+      acc[1] += wv * uv;
+      acc[2] += R.wv(i) * wv;
     }
-    const bool more = it < max_it;
-    if (!team_sumf<3>(team, w, acc, red, [&](const float* t) {
+    rows_sync();  // the group products read the other rows of the group
+  }
+  int it = 0;
+  while (state == 0) {
+    ++tag;
+    for (int i = row0; i < m; i += row_step) {
+      const float t = R.group_apply(11, i);
+      R.mt(i) = t;
+      link.template send_row<(kThreads > kTeamThreads)>(tag, r0 + i, t * R.dd(i));
+    }
+    if (!link.template exchange<kThreads>(w, tag, acc, red, one_warp, m, yt, [&](const float* t, int l) {
+          // (one division: the first lane's 1 / p'Hp and the second's 1 / gamma, which the next iteration reads)
           const float gam = t[0], dlt = t[1];
-          if (gam <= fstop || !more) {
-            sh.sc_state = 1;
-            return;
+          const float beta = it == 0 ? 0.0f : gam * sh.sf_rgz;
+          const float php = it == 0 ? dlt : dlt - beta * gam * sh.sf_raold;  // p'Hp
+          const float inv = 1.0f / (l == 0 ? php : gam);
+          const float rgz = __shfl_sync(0xffffffffu, inv, 1);
+          if (l == 0) {
+            if (gam <= sh.sf_stop || it >= sh.sc_budget) {
+              sh.sc_state = 1;
+            } else if (!(fabsf(php) > 0.0f) || !isfinite(php) || !isfinite(gam)) {
+              sh.sc_state = 2;  // breakdown: the FP64 residual of the sweep decides what follows
+            } else {
+              sh.sf_beta = beta;
+              sh.sf_alpha = gam * inv;
+              sh.sf_raold = php * rgz;
+              sh.sf_rgz = rgz;
+              sh.sf_shift = t[2] * sh.sf_rs1;
+            }
           }
-          const float beta = it == 0 ? 0.0f : gam / sh.sf_gz;
-          const float php = it == 0 ? dlt : dlt - beta * gam / sh.sf_aold;  // p'Hp
-          if (!(fabsf(php) > 0.0f) || !isfinite(php) || !isfinite(gam)) {
-            sh.sc_state = 2;  // breakdown: the FP64 residual of the sweep decides what follows
-            return;
-          }
-          const float alpha = gam / php;
-          sh.sf_beta = beta;
-          sh.sf_alpha = alpha;
-          sh.sf_aold = alpha;
-          sh.sf_gz = gam;
-          sh.sf_shift = t[2] / s1;
-        }, slot))
+        }))
       return -1;
-    if (sh.sc_state != 0) break;
-    stage();
+    state = sh.sc_state;
+    if (state != 0) break;
+    product();
     const float alpha = sh.sf_alpha, beta = sh.sf_beta, shift = sh.sf_shift;
-    product([&](int i, float hv) {
-      const float nv = hv - shift * R.cw(i);
-      const float mv = R.mt(i) - shift * R.wv(i);
+    acc[0] = acc[1] = acc[2] = 0.0f;
+    for (int i = row0; i < m; i += row_step) {
+      const float w1 = R.wv(i), wo = R.wq(i), uo = R.u(i);
+      const float nv = R.hv(i) + R.etadi(i) * yt[r0 + i] - shift * R.cw(i);
+      const float mv = R.mt(i) - shift * w1;
       const float zv = nv + beta * R.z(i);
       const float qv = mv + beta * R.q(i);
-      const float sv = R.wq(i) + beta * R.s(i);
-      const float pv = R.u(i) + beta * R.p(i);
+      const float sv = wo + beta * R.s(i);
+      const float pv = uo + beta * R.p(i);
+      const float rv = R.rr(i) - alpha * sv, uv = uo - alpha * qv, wv = wo - alpha * zv;
       R.z(i) = zv;
       R.q(i) = qv;
       R.s(i) = sv;
       R.p(i) = pv;
       R.x(i) += alpha * pv;
-      R.rr(i) -= alpha * sv;
-      R.u(i) -= alpha * qv;
-      R.wq(i) -= alpha * zv;
-    });
-    __syncthreads();  // the group products read the other rows of the group
+      R.rr(i) = rv;
+      R.u(i) = uv;
+      R.wq(i) = wv;
+      acc[0] += rv * uv;
+      acc[1] += wv * uv;
+      acc[2] += w1 * wv;
+    }
+    rows_sync();  // the group products read the other rows of the group
     ++it;
   }
-  for (int i = tid; i < m; i += blockDim.x) y_out[a0 + r0 + i] = R.x(i);
+  team.tag = tag;
+  for (int i = row0; i < m; i += row_step) y_out[a0 + r0 + i] = R.x(i);
   __syncthreads();
   return it;
 }
@@ -1659,12 +1811,15 @@ __device__ __noinline__ int qeq_cg_rows32_pipelined(const XrWork& w, const Team&
 // <D^-1, G^2> (from the projected values, so free of cancellation). Two team reductions.
 template <class Team>
 __device__ bool qeq_residual(const XrWork& w, const double* atab, const Team& team, QeqShared& sh, int a0, int r0, int r1,
-                             double s1, double target, double* gz_out, int& slot, bool adjoint) {
+                             double s1, double target, double* gz_out, int& slot, bool adjoint, const unsigned short* cols,
+                             int ebeg) {
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   double* X = &QW(Q_X, 0);
   double* G = &QW(Q_G, 0);
   const double* DI = &QW(Q_DINV, 0);
   const int gs = row_group(r1 - r0, w.cnt[a0 + r1] - w.cnt[a0 + r0]), sub = lane & (gs - 1), gpw = 32 / gs;
+  // loads in flight: a grid team's blocks have half the warps
+  constexpr int kLoads = is_grid<Team> ? 8 : 4;
   double acc[1] = {0.0};
   for (int rb = r0 + wid * gpw; rb < r1; rb += nw * gpw) {
     const int r = rb + lane / gs, a = a0 + r;
@@ -1672,20 +1827,21 @@ __device__ bool qeq_residual(const XrWork& w, const double* atab, const Team& te
     if (r < r1) {
       const int ee = w.cnt[a + 1];
       int e = w.cnt[a] + sub;
-      for (; e + 3 * gs < ee; e += 4 * gs) {
-        int j[4];
-        double h[4], x[4];
+      auto column = [&](int k) { return cols != nullptr ? a0 + cols[k - ebeg] : w.edge[k].x; };
+      for (; e + (kLoads - 1) * gs < ee; e += kLoads * gs) {
+        int j[kLoads];
+        double h[kLoads], x[kLoads];
 #pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          j[u] = w.edge[e + u * gs].x;
+        for (int u = 0; u < kLoads; ++u) {
+          j[u] = column(e + u * gs);
           h[u] = w.hval[e + u * gs];
         }
 #pragma unroll
-        for (int u = 0; u < 4; ++u) x[u] = __ldcg(X + j[u]);
+        for (int u = 0; u < kLoads; ++u) x[u] = __ldcg(X + j[u]);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) hx += h[u] * x[u];
+        for (int u = 0; u < kLoads; ++u) hx += h[u] * x[u];
       }
-      for (; e < ee; e += gs) hx += w.hval[e] * __ldcg(X + w.edge[e].x);
+      for (; e < ee; e += gs) hx += w.hval[e] * __ldcg(X + column(e));
     }
     for (int o = gs / 2; o > 0; o >>= 1) hx += __shfl_xor_sync(0xffffffffu, hx, o);
     if (sub == 0 && r < r1) G[a] = hx;  // finished one row per thread below
@@ -1763,7 +1919,7 @@ __device__ void qeq_solve(const XrWork& w, const double* atab, const Team& team,
   constexpr bool kBlock = std::is_same<Team, BlockTeam>::value;
   constexpr bool kCluster = std::is_same<Team, ClusterTeam>::value;
   // (the same for every block of a team: it depends on the system only)
-  constexpr bool kGridTeam = std::is_same<Team, GridTeam>::value;
+  constexpr bool kGridTeam = is_grid<Team>;
   int team_rows = n;  // the most rows any block of the team owns (the same value in every block)
   if constexpr (kGridTeam) team_rows = min(n, ((n + team.nb - 1) / team.nb + 31) / 32 * 32 + kGroupMax);
   // A grid team takes the row solver while that layout fits at all (up to about 45,000 atoms on 152
@@ -1818,6 +1974,8 @@ __device__ void qeq_solve(const XrWork& w, const double* atab, const Team& team,
     if (sub == 0 && r < r1) DI[a] = d;  // the shield sum; the diagonal follows one row per thread
   }
   __syncthreads();
+  if constexpr (kGridTeam)
+    if (small_rows) GridPackets::clear(w, team, F, a0, r0, r1);
   for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) {
     const int a = a0 + r;
     const double di = 1.0 / (atom_prm(atab, w.type[a], A_ETA) + DI[a]);
@@ -2009,12 +2167,10 @@ __device__ void qeq_solve(const XrWork& w, const double* atab, const Team& team,
       int it = 0;
       if (small_rows) {
         if constexpr (kGridTeam)
-          it = fits32 ? qeq_cg_rows32_pipelined<Team, false>(w, team, sh, a0, n, r0, r1, M32, v32.y, sh.sd_ratio, budget, v32.g,
-                                                             v32.g2, &slot)
-                      : qeq_cg_rows32_pipelined<Team, true>(w, team, sh, a0, n, r0, r1, M32, v32.y, sh.sd_ratio, budget, v32.g,
-                                                            v32.g2, &slot);
+          it = fits32 ? qeq_cg_rows32_pipelined<false, Team::kThreads>(w, team, sh, a0, n, r0, r1, M32, v32.y, sh.sd_ratio, budget, F)
+                      : qeq_cg_rows32_pipelined<true, Team::kThreads>(w, team, sh, a0, n, r0, r1, M32, v32.y, sh.sd_ratio, budget, F);
         else
-          it = qeq_cg_rows32(w, team, sh, a0, n, r0, r1, M32, v32.y, sh.sd_ratio, budget, &slot);
+          it = qeq_cg_rows32(w, team, sh, a0, n, r0, r1, M32, v32.y, sh.sd_ratio, budget);
       } else {
         it = qeq_cg<Team, float>(w, atab, team, sh, a0, n, r0, r1, v32, M32, s1, gz, fmax(1e-10 * gz, 0.01 * target), 0.0,
                                  budget, false, slot);
@@ -2037,7 +2193,7 @@ __device__ void qeq_solve(const XrWork& w, const double* atab, const Team& team,
       for (int r = r0 + threadIdx.x; r < r1; r += blockDim.x) X[a0 + r] += shift;
       if (!team.sync(w)) return;
       double gz_new = 0.0;
-      if (!qeq_residual(w, atab, team, sh, a0, r0, r1, s1, target, &gz_new, slot, adjoint)) return;
+      if (!qeq_residual(w, atab, team, sh, a0, r0, r1, s1, target, &gz_new, slot, adjoint, M32.cache_j, ebeg)) return;
       const bool stalled = gz_new > 1e-3 * gz;
       gz = gz_new;
       if (stalled && gz > target) {
@@ -2124,7 +2280,8 @@ __device__ void qeq_small_systems(const XrWork& w, const XrFF& ff, const int* sm
 // and synchronises through its own bounded counter. The remaining blocks each solve a share of the
 // small systems (small[k], k = b - nteam, b - nteam + (gridDim.x - nteam), ...) alone, with block
 // barriers only. All blocks are co-resident (cooperative launch, one block per SM).
-__global__ void __launch_bounds__(1024, 1) k_qeq_grid(XrWork w, XrFF ff, const int4* map, int nteam, const int* small,
+template <int T>
+__global__ void __launch_bounds__(T, 1) k_qeq_grid(XrWork w, XrFF ff, const int4* map, int nteam, const int* small,
                                                       int nsmall, int adjoint) {
   __shared__ QeqShared sh;
   extern __shared__ __align__(16) unsigned char dyn[];
@@ -2133,12 +2290,19 @@ __global__ void __launch_bounds__(1024, 1) k_qeq_grid(XrWork w, XrFF ff, const i
     const XrSystem& S = w.sys[m.x];
     // the rows of this block (k_qeq_splits: equal shares, no molecule cut)
     const int r0 = w.qsplit[2 * blockIdx.x], r1 = max(r0, w.qsplit[2 * blockIdx.x + 1]);
-    GridTeam team{w.barrier + m.w, w.red + (size_t)32 * m.w, m.z, m.y};
+    GridTeam<T> team{w.barrier + m.w, w.red + (size_t)32 * m.w, m.z, m.y};
     qeq_solve(w, atoms_of_system(ff, S), team, S.atom_off, S.natoms, r0, r1, adjoint ? 0.0 : S.total_charge,
               !adjoint && S.has_guess != 0, sh, dyn, kQeqMaxDyn, adjoint != 0);
     __syncthreads();
   }
   qeq_small_systems(w, ff, small, nsmall, w.barrier + nteam, adjoint, sh, dyn);
+}
+
+// The same for a batch without teams.
+__global__ void __launch_bounds__(kQeqThreads, 1) k_qeq_small(XrWork w, XrFF ff, const int* small, int nsmall, int adjoint) {
+  __shared__ QeqShared sh;
+  extern __shared__ __align__(16) unsigned char dyn[];
+  qeq_small_systems(w, ff, small, nsmall, w.barrier, adjoint, sh, dyn);
 }
 
 // Row splits of the QEq teams, one warp per split, before the solver (so that its registers stay with
@@ -2189,7 +2353,7 @@ __global__ void k_qeq_splits(XrWork w, const int* big, int nbig, int csize, cons
 // reductions through distributed shared memory; then every block takes systems of `small` alone.
 // A cluster's leader draws the next big system from a counter and the draw reaches the other
 // blocks through an exchange. Ordinary launch: no block waits on a block of another cluster.
-__global__ void __launch_bounds__(1024, 1) k_qeq_cluster(XrWork w, XrFF ff, const int* big, int nbig, const int* small,
+__global__ void __launch_bounds__(kQeqThreads, 1) k_qeq_cluster(XrWork w, XrFF ff, const int* big, int nbig, const int* small,
                                                          int nsmall, int adjoint) {
   __shared__ QeqShared sh;
   extern __shared__ __align__(16) unsigned char dyn[];
@@ -2221,7 +2385,7 @@ __global__ void __launch_bounds__(1024, 1) k_qeq_cluster(XrWork w, XrFF ff, cons
 }
 
 // The systems that the direct solver left (usually none), one block each.
-__global__ void __launch_bounds__(1024, 1) k_qeq_retry(XrWork w, XrFF ff, int adjoint) {
+__global__ void __launch_bounds__(kQeqThreads, 1) k_qeq_retry(XrWork w, XrFF ff, int adjoint) {
   __shared__ QeqShared sh;
   extern __shared__ __align__(16) unsigned char dyn[];
   int* const retry = w.qretry + (adjoint ? 2 : 0);
@@ -2231,7 +2395,7 @@ __global__ void __launch_bounds__(1024, 1) k_qeq_retry(XrWork w, XrFF ff, int ad
 }
 
 // Fallback without cooperative launch: one block per system, no shared-memory row cache.
-__global__ void __launch_bounds__(1024, 1) k_qeq_block(XrWork w, XrFF ff, int adjoint) {
+__global__ void __launch_bounds__(kQeqThreads, 1) k_qeq_block(XrWork w, XrFF ff, int adjoint) {
   __shared__ QeqShared sh;
   const XrSystem& S = w.sys[blockIdx.x];
   BlockTeam team;
@@ -2471,18 +2635,21 @@ void xr_launch_pairs(const XrWork& w, const XrFF& ff, cudaStream_t st) {
 }
 
 int xr_qeq_coop_blocks_per_sm() {
-  cudaFuncSetAttribute(k_qeq_grid, cudaFuncAttributeMaxDynamicSharedMemorySize, kQeqMaxDyn);
+  cudaFuncSetAttribute(k_qeq_grid<kTeamThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQeqMaxDyn);
+  cudaFuncSetAttribute(k_qeq_grid<kQeqThreads>, cudaFuncAttributeMaxDynamicSharedMemorySize, kQeqMaxDyn);
+  cudaFuncSetAttribute(k_qeq_small, cudaFuncAttributeMaxDynamicSharedMemorySize, kQeqMaxDyn);
   cudaFuncSetAttribute(k_qeq_retry, cudaFuncAttributeMaxDynamicSharedMemorySize, kQeqMaxDyn);
-  int nb = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_qeq_grid, 1024, kQeqMaxDyn);
-  return nb;
+  int nb = 0, few = 0;
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_qeq_grid<kQeqThreads>, kQeqThreads, kQeqMaxDyn);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&few, k_qeq_grid<kTeamThreads>, kTeamThreads, kQeqMaxDyn);
+  return std::min(nb, few);
 }
 
 namespace {
 cudaLaunchConfig_t cluster_config(int csize, int nblocks, cudaStream_t st, cudaLaunchAttribute* attr) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3(nblocks);
-  cfg.blockDim = dim3(1024);
+  cfg.blockDim = dim3(kQeqThreads);
   cfg.dynamicSmemBytes = kQeqMaxDyn;
   cfg.stream = st;
   attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -2526,28 +2693,31 @@ int xr_launch_qeq_cluster(const XrWork& w, const XrFF& ff, cudaStream_t st, int 
 
 // Returns 0 on success or a CUDA error code from the launch. With nblocks > 0 the cooperative
 // solver runs nblocks blocks (nteam team blocks described by map, the rest over the small list);
-// nblocks = 0 selects the one-block-per-system fallback.
+// nblocks = 0 selects the one-block-per-system fallback. team_rows: the most rows a team's block owns.
 int xr_launch_qeq(const XrWork& w, const XrFF& ff, cudaStream_t st, int nblocks, const int4* map, int nteam,
-                  const int* small, int nsmall, bool adjoint) {
+                  int team_rows, const int* small, int nsmall, bool adjoint) {
   int adj = adjoint ? 1 : 0;
   if (nblocks > 0) {
     // team barrier counters, then the small-system counter
     cudaMemsetAsync(w.barrier, 0, sizeof(unsigned) * (size_t)(nteam + 1), st);
     if (nteam > 0) k_qeq_splits<<<(2 * nteam + 3) / 4, 128, 0, st>>>(w, nullptr, 0, 0, map, nteam);
     if (nteam == 0) {  // no block waits on another: an ordinary launch, which may overlap other streams' work
-      k_qeq_grid<<<nblocks, 1024, kQeqMaxDyn, st>>>(w, ff, map, nteam, small, nsmall, adj);
+      k_qeq_small<<<nblocks, kQeqThreads, kQeqMaxDyn, st>>>(w, ff, small, nsmall, adj);
       return (int)cudaGetLastError();
     }
     void* args[] = {(void*)&w, (void*)&ff, (void*)&map, (void*)&nteam, (void*)&small, (void*)&nsmall, (void*)&adj};
-    cudaError_t e = cudaLaunchCooperativeKernel((const void*)k_qeq_grid, dim3(nblocks), dim3(1024), args, kQeqMaxDyn, st);
+    const bool few = team_rows <= kTeamRows;
+    const void* kernel = few ? (const void*)k_qeq_grid<kTeamThreads> : (const void*)k_qeq_grid<kQeqThreads>;
+    cudaError_t e = cudaLaunchCooperativeKernel(kernel, dim3(nblocks), dim3(few ? kTeamThreads : kQeqThreads), args,
+                                                kQeqMaxDyn, st);
     return (int)e;
   }
-  k_qeq_block<<<w.S, 1024, 0, st>>>(w, ff, adj);
+  k_qeq_block<<<w.S, kQeqThreads, 0, st>>>(w, ff, adj);
   return (int)cudaGetLastError();
 }
 
 int xr_launch_qeq_retry(const XrWork& w, const XrFF& ff, cudaStream_t st, int count, bool adjoint) {
-  k_qeq_retry<<<count, 1024, kQeqMaxDyn, st>>>(w, ff, adjoint ? 1 : 0);
+  k_qeq_retry<<<count, kQeqThreads, kQeqMaxDyn, st>>>(w, ff, adjoint ? 1 : 0);
   return (int)cudaGetLastError();
 }
 
