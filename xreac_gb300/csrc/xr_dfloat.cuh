@@ -37,10 +37,45 @@ __device__ inline xr_df xr_df_fast_two_sum(float a, float b) {
   return {s, __fsub_rn(b, __fsub_rn(s, a))};
 }
 
-__device__ inline xr_df xr_df_from_double(double x) {
-  const float h = __double2float_rn(x);
-  return {h, __double2float_rn(x - (double)h)};
+// Conversions between double and float are FP64 instructions here, each as long on the FP64 pipe as an FMA (64
+// cycles for a warp), and they were three quarters of an exponential's FP64 issue. Both directions are
+// exact or correctly rounded with integer instructions, without a branch to the FP64 ones (which the
+// compiler predicates, and a predicated instruction takes the pipe all the same): magnitudes below float's
+// normal range become zero, which is below 2^-48 of whatever they are added to here, and doubles beyond
+// its range NaN, which the domain checks of exp and log reject. FP64 instructions before and after:
+// xr_exp 11 and 3, xr_log 11 and 2.
+__device__ inline double xr_f2d(float f) {
+  const unsigned u = __float_as_uint(f), t = u & 0x7fffffffu;
+  unsigned hi = (t >> 3) + 0x38000000u, lo = u << 29;
+  if (t < 0x00800000u) hi = lo = 0u;
+  if (t >= 0x7f800000u) hi |= 0x7ff00000u;  // infinite or NaN
+  return __hiloint2double((int)(hi | (u & 0x80000000u)), (int)lo);
 }
+
+// hi: x rounded to the nearest float (halves away from zero), lo: the rest of x, rounded to float.
+__device__ inline xr_df xr_df_from_double(double x) {
+  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x), e = h & 0x7ff00000u;
+  // the significand's low 29 bits go to lo: add half a unit of the 30th, cut there, keep the signed rest
+  const unsigned lr = l + 0x10000000u, hr = h + (lr < l ? 1u : 0u), sign = h & 0x80000000u;
+  unsigned hi = ((__funnelshift_l(lr, hr, 3) + 0x40000000u) & 0x7fffffffu) | sign;
+  unsigned scale = ((e << 3) + 0x40000000u) | sign;  // +-2^exponent of x
+  if (e < 897u << 20) hi = scale = 0u;
+  if (e > 1150u << 20) hi = 0x7fffffffu;
+  const float rest = __int2float_rn((int)(lr & 0x1fffffffu) - 0x10000000);
+  return {__uint_as_float(hi), __fmul_rn(__fmul_rn(rest, 0x1p-52f), __uint_as_float(scale))};
+}
+
+// x rounded to float (halves away from zero).
+__device__ inline float xr_d2f(double x) {
+  const unsigned h = (unsigned)__double2hiint(x), l = (unsigned)__double2loint(x), e = h & 0x7ff00000u;
+  const unsigned lr = l + 0x10000000u, hr = h + (lr < l ? 1u : 0u);
+  unsigned hi = ((__funnelshift_l(lr, hr, 3) + 0x40000000u) & 0x7fffffffu) | (h & 0x80000000u);
+  if (e < 897u << 20) hi = 0u;
+  if (e > 1150u << 20) hi = 0x7fffffffu;
+  return __uint_as_float(hi);
+}
+
+__device__ inline double xr_df_to_double(xr_df a) { return xr_f2d(a.hi) + xr_f2d(a.lo); }
 
 __device__ inline xr_df xr_df_add(xr_df a, xr_df b) {
   xr_df s = xr_df_two_sum(a.hi, b.hi);
@@ -126,15 +161,15 @@ __device__ inline xr_df xr_df_exp_float(float x, int* n) {
 // significant bits so that k hi is exact): a double-float input would lose the bits of x beyond 48,
 // 1e-13 of exp(x) at |x| = 70.
 __device__ inline double xr_exp(double x) {
-  const float xf = __double2float_rn(x);
+  const float xf = xr_d2f(x);
   if (!(fabsf(xf) < 80.0f)) return exp(x);
   const float kf = rintf(__fmul_rn(xf, 0x1.715476p+6f));  // round(x 64 / ln2), |kf| < 2^13
-  const double kd = (double)kf;
+  const double kd = xr_f2d(kf);
   double r = fma(-kd, 0x1.62e42fefa4000p-7, x);
   r = fma(-kd, -0x1.8432a1b0e2634p-49, r);
   int n;
   const xr_df m = xr_df_exp_finish(xr_df_from_double(r), (int)kf, &n);
-  const double v = (double)m.hi + (double)m.lo;
+  const double v = xr_df_to_double(m);
   return __longlong_as_double(__double_as_longlong(v) + ((long long)n << 52));  // v 2^n: both normal
 }
 
@@ -186,5 +221,5 @@ __device__ inline double xr_log(double a) {
   e.lo = __fmul_rn(e.lo, s);
   const xr_df t = xr_df_add_f(xr_df_mul(ad, e), -1.0f);  // a exp(-y0) - 1
   const xr_df l = xr_df_add_f(t, y0);
-  return (double)l.hi + ((double)l.lo - 0.5 * (double)t.hi * (double)t.hi);
+  return xr_f2d(l.hi) + fma(xr_f2d(__fmul_rn(-0.5f, t.hi)), xr_f2d(t.hi), xr_f2d(l.lo));
 }

@@ -42,6 +42,19 @@ __device__ inline void edge_vector(const XrSystem& S, const double4_32a& xi, con
     return;
   }
   const int sx = xr_sx(code), sy = xr_sy(code), sz = xr_sz(code);
+  // nearest images: a product with -1, 0 or 1 needs no multiplication and no converted factor, both of which would be
+  // FP64 instructions (15 of the 24 that an offset takes; a warp of pairs nearly always has one)
+  if (abs(sx) <= 1 && abs(sy) <= 1 && abs(sz) <= 1) {
+    auto times = [](int s, double a) {
+      const int hi = __double2hiint(a);
+      return s == 0 ? 0.0 : __hiloint2double(s < 0 ? hi ^ (int)0x80000000 : hi, __double2loint(a));
+    };
+    for (int c = 0; c < 3; ++c) {
+      const double off = __dadd_rn(__dadd_rn(times(sx, S.cell[c]), times(sy, S.cell[3 + c])), times(sz, S.cell[6 + c]));
+      v[c] = __dadd_rn(__dsub_rn(xb[c], xa[c]), off);
+    }
+    return;
+  }
   for (int c = 0; c < 3; ++c) {
     const double off = __dadd_rn(__dadd_rn(__dmul_rn((double)sx, S.cell[c]), __dmul_rn((double)sy, S.cell[3 + c])),
                                  __dmul_rn((double)sz, S.cell[6 + c]));
@@ -49,17 +62,16 @@ __device__ inline void edge_vector(const XrSystem& S, const double4_32a& xi, con
   }
 }
 
-// t^(-1/3) for t in the float range: an FP32 seed, then two Newton-Raphson steps on f(z) = z^-3 - t,
-// z <- z (4 - t z^3) / 3, each of which squares the relative error (about 1e-7, 1e-14, then FP64
-// rounding). Multiplies only: it replaces a double cube root and the divisions by it. It stays FP64:
-// the shield builds the QEq matrix, whose solve amplifies an entry's error by the matrix's condition
-// (a double-float version, about 1e-14, moved the Coulomb energy of an ill-conditioned fixture by 2e-12
-// of its value, beyond the parity tolerance).
+// t^(-1/3) for t in the float range: an FP32 seed z of relative error about 1e-7, then with e = 1 - t z^3
+// the series z (1 - e)^(-1/3) = z (1 + e / 3 + 2 e^2 / 9 + ...), whose next term is below 1e-19. Multiplies
+// only: it replaces a double cube root and the divisions by it. It stays FP64: the shield builds the
+// QEq matrix, whose solve amplifies an entry's error by the matrix's condition (a double-float version, about
+// 1e-14, moved the Coulomb energy of an ill-conditioned fixture by 2e-12 of its value, beyond the
+// parity tolerance). Two Newton steps took 12 FP64 instructions with the seed's conversions, this takes 6.
 __device__ inline double inv_cbrt(double t) {
-  double z = (double)rcbrtf((float)t);
-  z = z * (4.0 - t * z * z * z) * (1.0 / 3.0);
-  z = z * (4.0 - t * z * z * z) * (1.0 / 3.0);
-  return z;
+  const double z = xr_f2d(rcbrtf(xr_d2f(t)));
+  const double e = fma(-t, z * z * z, 1.0);
+  return fma(z * e, fma(e, 2.0 / 9.0, 1.0 / 3.0), z);
 }
 
 // The QEq block-Jacobi groups: runs of at most kGroupMax consecutive atoms, each within kGroupBond of
@@ -87,9 +99,9 @@ __device__ inline void pair_one(const XrWork& w, const XrFF& ff0, int p) {
   double taper = 0.0, dtaper = 0.0;
   if (r < rc) {
     const double u = r * S.inv_rc;
-    taper = 1 + u * u * u * u * (-35 + u * (84 + u * (-70 + 20 * u)));
-    const double um = u - 1;
-    dtaper = 140.0 * S.inv_rc * u * u * u * um * um * um;
+    const double u2 = u * u, t = fma(u, u, -u);  // u (u - 1)
+    taper = 1 + u2 * u2 * (-35 + u * (84 + u * (-70 + 20 * u)));
+    dtaper = 140.0 * S.inv_rc * t * t * t;
   }
   const double gam = pair_prm(ff, pt, P_GAMMA);
   const double z = inv_cbrt(r * r * r + gam);  // (r^3 + gamma)^(-1/3), FP64: the QEq matrix is built from it
@@ -107,8 +119,8 @@ __device__ inline void pair_one(const XrWork& w, const XrFF& ff0, int p) {
     const xr_df f = xr_df_exp_df(xr_df_mul(ls, {ff.vdw_invp.x, ff.vdw_invp.y}));
     const xr_df d = xr_df_exp_df(xr_df_add(xr_df_mul(lr, {ff.vdw_p_m1.x, ff.vdw_p_m1.y}),
                                            xr_df_mul(ls, {ff.vdw_invp_m1.x, ff.vdw_invp_m1.y})));
-    f13 = (double)f.hi + (double)f.lo;
-    df13 = (double)d.hi + (double)d.lo;
+    f13 = xr_df_to_double(f);
+    df13 = xr_df_to_double(d);
   }
   // reciprocals of the pair's radii from the table: multiplies instead of FP64 divisions
   const double D = pair_prm(ff, pt, P_D), alpha = pair_prm(ff, pt, P_ALPHA);
@@ -158,7 +170,7 @@ __global__ void k_hval(XrWork w) {
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ne; e += gridDim.x * blockDim.x) {
     const double h = QEQ_COULOMB * w.p_shield[w.edge_pair[e]];
     w.hval[e] = h;
-    w.qch[e] = float(h);  // FP32 copy for the solver's row cache (which may overwrite it, scaled)
+    w.qch[e] = xr_d2f(h);  // FP32 copy for the solver's row cache (which may overwrite it, scaled)
   }
 }
 
