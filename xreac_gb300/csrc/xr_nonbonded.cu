@@ -80,6 +80,9 @@ constexpr int kGroupMax = 8;
 constexpr double kGroupBond = 1.3;
 
 // ------------------------------------------------------------------------------ pair kernel
+// Bound by the FP64 pipe (84 % of its issue): 69 instructions there per pair, 97 before conversions, comparisons
+// and the products of nearest images' offsets became integer instructions and the vdW term was
+// factored. Pairs stage of the 36,864-atom water box 1,727 -> 1,133 us, of 4,608 atoms 243 -> 160.
 __device__ inline void pair_one(const XrWork& w, const XrFF& ff0, int p) {
   const int e = w.pair_edge[p], i = w.pair_i[p];
   const int2 ed = w.edge[e];
@@ -88,8 +91,11 @@ __device__ inline void pair_one(const XrWork& w, const XrFF& ff0, int p) {
   const XrFF ff = xr_ff_at(ff0, ff0.nsets > 1 ? S.ff_set : 0);
   double v[3];
   edge_vector(S, w.x[i], w.x[j], (uint32_t)ed.y, v);
-  const double r = __dsqrt_rn(__dadd_rn(__dadd_rn(__dmul_rn(v[0], v[0]), __dmul_rn(v[1], v[1])), __dmul_rn(v[2], v[2])));
-  if (r < kGroupBond && i != j && abs(i - j) < kGroupMax) {  // a bond for the QEq preconditioner's groups
+  const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(v[0], v[0]), __dmul_rn(v[1], v[1])), __dmul_rn(v[2], v[2]));
+  const double r = __dsqrt_rn(r2);
+  // (distances compare as integers, being positive: a comparison of doubles is an FP64 instruction too)
+  auto below = [&](double limit) { return __double_as_longlong(r) < __double_as_longlong(limit); };
+  if (below(kGroupBond) && i != j && abs(i - j) < kGroupMax) {  // a bond for the QEq preconditioner's groups
     const int lo = min(i, j), hi = max(i, j);
     atomicMin(w.qb_first + hi, lo);
     atomicMax(w.qb_last + hi, lo);
@@ -97,17 +103,17 @@ __device__ inline void pair_one(const XrWork& w, const XrFF& ff0, int p) {
   const double rc = S.rc;
   const int T = ff.ntypes, pt = w.type[i] * T + w.type[j];
   double taper = 0.0, dtaper = 0.0;
-  if (r < rc) {
+  if (below(rc)) {
     const double u = r * S.inv_rc;
     const double u2 = u * u, t = fma(u, u, -u);  // u (u - 1)
     taper = 1 + u2 * u2 * (-35 + u * (84 + u * (-70 + 20 * u)));
     dtaper = 140.0 * S.inv_rc * t * t * t;
   }
   const double gam = pair_prm(ff, pt, P_GAMMA);
-  const double z = inv_cbrt(r * r * r + gam);  // (r^3 + gamma)^(-1/3), FP64: the QEq matrix is built from it
+  const double z = inv_cbrt(r2 * r + gam);  // (r^3 + gamma)^(-1/3), FP64: the QEq matrix is built from it
   const double z2 = z * z;
   const double shield = taper * z;
-  const double dshield = dtaper * z - taper * r * r * (z2 * z2);
+  const double dshield = dtaper * z - taper * r2 * (z2 * z2);
   double f13 = r, df13 = 1.0;
   // exponentials and logarithms in double-float arithmetic on the FP32 pipe (xr_dfloat.cuh): they
   // were most of this kernel's FP64 issue. The shielding chain stays in double-floats from r to
@@ -125,10 +131,11 @@ __device__ inline void pair_one(const XrWork& w, const XrFF& ff0, int p) {
   // reciprocals of the pair's radii from the table: multiplies instead of FP64 divisions
   const double D = pair_prm(ff, pt, P_D), alpha = pair_prm(ff, pt, P_ALPHA);
   const double2 inv = __ldg(reinterpret_cast<const double2*>(ff.pair_inv) + pt);  // 1/r_vdW, 1/rcore
-  const double ev = xr_exp(0.5 * alpha * (1 - f13 * inv.x));
-  const double dev = ev * (-0.5 * alpha * inv.x) * df13;
-  double E = taper * D * (ev * ev - 2 * ev);
-  double G = dtaper * D * (ev * ev - 2 * ev) + taper * D * (2 * ev - 2) * dev;
+  const double ax = alpha * inv.x;
+  const double ev = xr_exp(0.5 * (alpha - ax * f13));
+  const double Dq = D * (ev * (ev - 2));
+  double E = taper * Dq;
+  double G = dtaper * Dq - taper * ((ev - 1) * (ev * df13 * (D * ax)));
   if (ff.vdw_type == 2 || ff.vdw_type == 3) {
     const double ecore = pair_prm(ff, pt, P_ECORE), acore = pair_prm(ff, pt, P_ACORE);
     const double ec = ecore * xr_exp(acore * (1 - r * inv.y));
@@ -2423,28 +2430,58 @@ __global__ void k_pairs(XrWork w, XrFF ff0) {
 // ------------------------------------------------------------------------ force assembly
 // The pair's shielded Coulomb energy 332.06371 q_i q_j shield(r) is formed here, with the final
 // charges, and its dE/dr joins the pair's radial sensitivity (vdW, charge response, bond-order
-// chain): dE/dx_j += G v/r, dE/dx_i -= G v/r.
-__device__ inline void pair_force_one(const XrWork& w, int p) {
+// chain): dE/dx_j += G v/r, dE/dx_i -= G v/r. Returns false when no force comes of it.
+__device__ inline bool pair_force(const XrWork& w, int p, int* i_out, int* j_out, double f[3]) {
   const int i = w.pair_i[p];
   const int2 ed = w.edge[w.pair_edge[p]];
   const int j = ed.x;
   const double qq = C_ELE * w.q[i] * w.q[j];
   w.p_ecoul[p] = qq * w.p_shield[p];
   const double G = w.p_g[p] + qq * w.p_dshield[p];
-  if (G == 0.0 || i == j) return;  // a self-image pair moves both ends together: no net force
+  if (G == 0.0 || i == j) return false;  // a self-image pair moves both ends together: no net force
   const XrSystem& S = w.sys[w.sys_of[i]];
   double v[3];
   edge_vector(S, w.x[i], w.x[j], (uint32_t)ed.y, v);
   const double s = G / w.p_r[p];
-  for (int c = 0; c < 3; ++c) {
-    atomicAdd(w.f + 3 * j + c, s * v[c]);
-    atomicAdd(w.f + 3 * i + c, -s * v[c]);
-  }
+  for (int c = 0; c < 3; ++c) f[c] = s * v[c];
+  *i_out = i;
+  *j_out = j;
+  return true;
 }
 
+// A warp takes 32 kForcePairs consecutive pairs. Pairs are stored by their first atom, so a lane adds up what its
+// pairs give that atom and passes it on when the atom changes: bound by the FP64 atomics, of which the three to
+// the first atom met the same address from every lane of the warp. The force stage of the
+// 36,864-atom water box takes 872 us with 1 pair a lane, 593 with 4, 608 with 8 and 635 with 16, that of 1,000 C/H/O
+// atoms 82, 80, 91 and 98 (too few warps).
+constexpr int kForcePairs = 4;
 __global__ void k_pair_forces(XrWork w) {
   const int np = xr_num_pairs(w);
-  for (int p = blockIdx.x * blockDim.x + threadIdx.x; p < np; p += gridDim.x * blockDim.x) pair_force_one(w, p);
+  const int warp = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5), nw = (int)(gridDim.x * blockDim.x >> 5);
+  const int lane = threadIdx.x & 31;
+  for (long long base = (long long)warp * 32 * kForcePairs; base < np; base += (long long)nw * 32 * kForcePairs) {
+    double g[3] = {0.0, 0.0, 0.0};
+    int at = -1;
+    auto flush = [&]() {
+      if (at >= 0)
+        for (int c = 0; c < 3; ++c) atomicAdd(w.f + 3 * at + c, -g[c]);
+    };
+    const int end = (int)min((long long)np, base + 32 * kForcePairs);
+    for (int p = (int)base + lane; p < end; p += 32) {
+      int i, j;
+      double f[3];
+      if (!pair_force(w, p, &i, &j, f)) continue;
+      for (int c = 0; c < 3; ++c) atomicAdd(w.f + 3 * j + c, f[c]);
+      if (i != at) {
+        flush();
+        at = i;
+        for (int c = 0; c < 3; ++c) g[c] = f[c];
+      } else {
+        for (int c = 0; c < 3; ++c) g[c] += f[c];
+      }
+    }
+    flush();
+  }
 }
 
 // ------------------------------------------------------------------------ reductions
@@ -2745,7 +2782,10 @@ int xr_launch_qeq_retry(const XrWork& w, const XrFF& ff, cudaStream_t st, int co
 
 void xr_launch_forces(const XrWork& w, const XrFF& ff, cudaStream_t st) {
   (void)ff;
-  if (w.nP > 0) k_pair_forces<<<(w.nP + 255) / 256, 256, 0, st>>>(w);
+  if (w.nP > 0) {
+    const int threads = (w.nP + kForcePairs - 1) / kForcePairs;
+    k_pair_forces<<<(threads + 255) / 256, 256, 0, st>>>(w);
+  }
 }
 
 void xr_launch_reduce(const XrWork& w, const XrFF& ff, cudaStream_t st) {
