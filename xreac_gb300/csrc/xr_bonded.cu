@@ -433,9 +433,23 @@ __global__ void k_bond_energy(XrWork w, XrFF ff) {
 // would spend most of the pipe on idle lanes. Per-unit sums (energies, the unit's own adjoints and
 // force) are formed by a segmented warp reduction over the contiguous items of each unit, in lane
 // and pass order, so energies are deterministic; contributions to other atoms and bonds use atomics.
-constexpr int kUnits = 8;          // units per warp chunk
+constexpr int kUnits = 8;          // units per warp chunk, at most
 constexpr int kItemBuf = 64;       // per-warp item buffer: at most 31 left over + 32 new
 constexpr int kBondedWarps = 4;    // warps per block of the item kernels
+constexpr int kWarpsWanted = 1216;
+
+// Units per warp chunk for `count` units in all. A warp works through its batches one after another, so the chunks
+// are no longer than two warps per scheduler ask for (608 schedulers); where there is more work than that, longer chunks
+// fill the batches better. Bonded stage with chunks of 8 throughout, and for one, two and four warps per scheduler:
+// a 288-atom slab 333, 234, 237 and 238 us; 192 atoms of water 181, 156, 156 and 156; 24 slabs with parameter
+// gradients 517, 516, 471 and 556; 4,608 atoms of water 328, 330, 321 and 359; 36,864 atoms 1,349 to 1,344 (8 units).
+// A call of a few small molecules keeps the long chunks: the angles of each lie in one warp, or two, so that what they
+// add to an atom, a bond or a parameter comes in one order and repeats bit for bit, and there is little to gain
+// (9 atoms: 112 and 109 us).
+__host__ __device__ inline int chunk_units(int count) {
+  const int n = (count + kWarpsWanted - 1) / kWarpsWanted;
+  return count <= 4 * kUnits || n > kUnits ? kUnits : n;
+}
 
 __device__ inline uint32_t pack_item(int u, int a, int c) { return ((uint32_t)u << 28) | ((uint32_t)a << 14) | (uint32_t)c; }
 __device__ inline int item_unit(uint32_t it) { return (int)(it >> 28); }
@@ -485,7 +499,7 @@ __device__ inline void push_items(uint32_t* buf, int& nbuf, bool ok, uint32_t it
 
 // Valence angle, penalty and coalition terms (src/xreac/energy.py:278-318 with the angle rule of
 // src/xreac/energy.py:49-55): units are centres j, items the pairs of j's active bonds.
-__global__ void __launch_bounds__(32 * kBondedWarps) k_angles(XrWork w, XrFF ff0) {
+__global__ void __launch_bounds__(32 * kBondedWarps) k_angles(XrWork w, XrFF ff0, int units) {
   constexpr int NC = 8, NV = 10;
   __shared__ double ucon[kBondedWarps][kUnits][NC];
   __shared__ double uacc[kBondedWarps][kUnits][NV];
@@ -493,9 +507,9 @@ __global__ void __launch_bounds__(32 * kBondedWarps) k_angles(XrWork w, XrFF ff0
   __shared__ uint32_t buf[kBondedWarps][kItemBuf];
   const int lane = threadIdx.x & 31, wl = threadIdx.x >> 5;
   const int chunk = (int)((blockIdx.x * (unsigned)blockDim.x + threadIdx.x) >> 5);
-  const int j0 = chunk * kUnits;
+  const int j0 = chunk * units;
   if (j0 >= w.A) return;
-  const int nu = min(kUnits, w.A - j0);
+  const int nu = min(units, w.A - j0);
   const int L = w.A + 1, T = ff0.ntypes;
   const double* g = ff0.g;
   const bool lammps = !w.full_derivative;
@@ -814,8 +828,9 @@ __global__ void __launch_bounds__(32 * kBondedWarps) k_torsions(XrWork w, XrFF f
   const double* g = ff0.g;
   const int nm = *w.nmids;
   double* acc = &uacc[wl][0][0];
-  for (int q0 = warp * kUnits; q0 < nm; q0 += nwarps * kUnits) {
-    const int nu = min(kUnits, nm - q0);
+  const int units = chunk_units(nm);
+  for (int q0 = warp * units; q0 < nm; q0 += nwarps * units) {
+    const int nu = min(units, nm - q0);
     if (lane < nu) {
       UnitInt& ui = uint_[wl][lane];
       const int m = w.mids[q0 + lane];
@@ -1368,7 +1383,7 @@ void xr_launch_bonded(const XrWork& w, const XrFF& ff, const XrFork& fork) {
     k_mid_scan<<<1, 1024, 0, st_t>>>(w);
     k_mid_fill<<<gT, kMidTile, 0, st_t>>>(w);
     fork.wait(st_t, fork.atoms);
-    const int chunks = (w.nB + kUnits - 1) / kUnits;
+    const int units = chunk_units(w.nB), chunks = (w.nB + units - 1) / units;  // (there are at most nB middles)
     const int blocks = std::min((chunks + kBondedWarps - 1) / kBondedWarps, 152 * 16);
     k_torsions<<<blocks, 32 * kBondedWarps, 0, st_t>>>(w, ff);
     fork.record(fork.torsions, st_t);
@@ -1381,8 +1396,8 @@ void xr_launch_bonded(const XrWork& w, const XrFF& ff, const XrFork& fork) {
   if (w.nB > 0) k_bond_energy<<<gM, tb, 0, st_a>>>(w, ff);
   fork.record(fork.atoms2, st_a);
   {
-    const int chunks = (w.A + kUnits - 1) / kUnits;
-    k_angles<<<(chunks + kBondedWarps - 1) / kBondedWarps, 32 * kBondedWarps, 0, st>>>(w, ff);
+    const int units = chunk_units(w.A), chunks = (w.A + units - 1) / units;
+    k_angles<<<(chunks + kBondedWarps - 1) / kBondedWarps, 32 * kBondedWarps, 0, st>>>(w, ff, units);
   }
   if (w.nB > 0) fork.wait(st, fork.torsions);
   fork.wait(st, fork.hbonds);
