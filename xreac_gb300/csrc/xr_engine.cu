@@ -731,6 +731,11 @@ bool plan_qeq_cluster(xr_ctx* c, const xr_system* sys, int nsys, const std::vect
 // others (for the CG plans). A caller that bounds the CG iterations, or the test that makes a team wait
 // run out, gets the CG solver whose iterations and waits those are.
 constexpr int kQeqDirectIterations = 400;
+// The largest system alone in its call that one block solves. A cluster pays two cluster barriers a tile step and has
+// eight blocks' FP64 for the products of periodic systems' long rows: with eight tile rows a block takes 152 us
+// for 240 atoms of water, open, and 197 in a cell, a cluster 168 and 182; with nine (288 atoms) a block 192 and 283, a cluster 191 and
+// 217.
+constexpr int kQeqDirectBlockAlone = 256;
 
 struct DirectPlan {
   std::vector<int> cluster, block, small;  // clusters of `nb` blocks; single blocks; single blocks of small systems
@@ -745,7 +750,7 @@ void plan_qeq_direct(const xr_ctx* c, const xr_system* sys, int nsys, DirectPlan
       rest.push_back(s);
     else if (n <= kQeqDirectSmall)
       d.small.push_back(s);
-    else if (n <= kQeqDirectMax)
+    else if (n <= (nsys == 1 && c->direct8 > 0 ? kQeqDirectBlockAlone : kQeqDirectMax))
       d.block.push_back(s);
     else if (n <= c->direct8)
       d.cluster.push_back(s);
