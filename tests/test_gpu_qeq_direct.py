@@ -1,4 +1,4 @@
-"""The direct QEq solvers (one block up to 288 atoms, a cluster of blocks up to 736) against the oracle's dense KKT solve of src/xreac/energy.py:89-103.
+"""The direct QEq solvers (one block up to 288 atoms, a cluster of blocks up to 608) against the oracle's dense KKT solve of src/xreac/energy.py:89-103.
 
 Sizes lie on both sides of their 32-row tiles, of their launch classes (32, 96, 288, 608 atoms) and of their end; the
 next size takes the CG solver. Cells so small that an atom sees its own images, net charges, warm starts, adjoint solves
@@ -56,7 +56,7 @@ def test_cluster_charges(n):
     r = calc.evaluate(symbols, x, total_charge=1.0 if n % 2 else 0.0)
     np.testing.assert_allclose(r.charges, _dense(symbols, x, charge=1.0 if n % 2 else 0.0), atol=1e-10, rtol=0)
     steps = calc.qeq_work()[0]
-    assert steps <= 8 if n <= 736 else steps > 8  # refinement steps, or CG iterations
+    assert steps <= 8 if n <= 608 else steps > 8  # refinement steps, or CG iterations
     warm = calc.evaluate(symbols, x + 1e-3, total_charge=1.0 if n % 2 else 0.0, initial_charges=r.charges + 0.01)
     np.testing.assert_allclose(warm.charges, r.charges, atol=1e-10, rtol=0)
 
@@ -69,7 +69,7 @@ def test_small_cells_with_self_images(n_mol, side):
     s = water_box(n_mol=n_mol, box=side, min_oo=2.4, seed=6)
     calc = Calculator(ForceField.bundled(FF), max_expanded_atoms=100000)
     r = calc.evaluate(s.symbols, s.positions, cell=s.cell, pbc=True)
-    assert calc.qeq_work()[0] <= 8
+    assert calc.qeq_work()[0] <= 8 or 3 * n_mol > 608  # (larger systems take the CG solver)
     np.testing.assert_allclose(r.charges, _dense(s.symbols, s.positions, s.cell), atol=1e-10, rtol=0)
 
 

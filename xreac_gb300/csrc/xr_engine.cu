@@ -104,7 +104,7 @@ struct xr_ctx {
   cudaStream_t side[7] = {};     // bonded, torsions, hydrogen bonds; the direct QEq solves' classes; per-atom terms
   cudaEvent_t fork_ev[12] = {};
   bool qeq_direct = false;       // the direct QEq solver fits the device's shared memory
-  int direct8 = 0, direct16 = 0;  // the largest systems of its clusters of 8 and 16 blocks (0: not available)
+  int direct_cluster = 0;    // the largest system of its clusters of blocks (0: not available)
   // Cell list (xr_ctx_set_cell_list): 0 chooses per call, 1 always, -1 never.
   int cell_mode = 0;
   int* atom_cell = nullptr;
@@ -641,7 +641,7 @@ int status_to_code(xr_ctx* c, int st) {
 }
 
 // QEq work plan of a batch for the solver kernel (at most kQeqBlocks co-resident blocks). A team
-// of ceil(n / 32) blocks (32 rows per 1024-thread block) solves a large system with grid-level
+// of blocks (32 rows each in a batch; qeq_alone_blocks for a single system) solves a large system with grid-level
 // reductions, which shortens one solve; a single block solves a system with block barriers only,
 // which costs the fewest SM-cycles. So a single-system call gives a team to a system above
 // kQeqSmall atoms, and a batch (throughput) only to systems above kQeqBatchBlock atoms. Teams are
@@ -651,7 +651,17 @@ constexpr int kQeqSmall = 160;
 #ifndef XR_QEQ_TEAM_ROWS
 #define XR_QEQ_TEAM_ROWS 32
 #endif
-constexpr int kQeqTeamRows = XR_QEQ_TEAM_ROWS;  // rows per block of a grid-wide team (a multiple of 32)
+constexpr int kQeqTeamRows = XR_QEQ_TEAM_ROWS;  // rows per block of a grid-wide team of a batch
+// A single system's team: a block for every 12 rows up to two thirds of the chip, which leaves the bonded branch
+// multiprocessors to run beside the solve, and more blocks once those would have over 48 rows. Evaluations with blocks of
+// 32 rows, and as here: 740 atoms of water in a cell 711 and 597 us, 1,000 780 and 655, 2,400 986 and 909, 4,608 1,492 and
+// 1,346 (and 1,513 with 144 blocks, 1,525 with 152), 9,000 2,604 and 2,373.
+constexpr int kQeqAloneRows = 12, kQeqAloneMost = 48;
+int qeq_alone_blocks(int natoms, int budget) {
+  const int some = std::max(1, budget * 2 / 3);
+  if (natoms > kQeqAloneMost * some) return std::min(budget, (natoms + kQeqAloneMost - 1) / kQeqAloneMost);
+  return std::min(some, (natoms + kQeqAloneRows - 1) / kQeqAloneRows);
+}
 constexpr int kQeqBatchBlock = 1024;
 
 void plan_qeq(xr_ctx* c, const xr_system* sys, int nsys, const std::vector<int>& ids, int* nblocks, int* nteam, int* nsmall) {
@@ -665,11 +675,15 @@ void plan_qeq(xr_ctx* c, const xr_system* sys, int nsys, const std::vector<int>&
     const int small_blocks = small.empty() ? 0 : (large.empty() ? std::min<int>((int)small.size(), budget)
                                                                  : std::min<int>((int)small.size(), std::max(1, budget / 4)));
     const int avail = budget - small_blocks;
+    auto blocks = [&](size_t k) {
+      const int n = sys[large[k]].natoms;
+      return nsys == 1 ? qeq_alone_blocks(n, avail) : (n + kQeqTeamRows - 1) / kQeqTeamRows;
+    };
     long long want = 0;
-    for (size_t k = 0; k < large.size(); ++k) want += (sys[large[k]].natoms + kQeqTeamRows - 1) / kQeqTeamRows;
+    for (size_t k = 0; k < large.size(); ++k) want += blocks(k);
     long long have = 0;
     for (size_t k = 0; k < large.size(); ++k) {
-      const long long d = (sys[large[k]].natoms + kQeqTeamRows - 1) / kQeqTeamRows;
+      const long long d = blocks(k);
       team[k] = (int)std::max<long long>(2, want > avail ? d * avail / std::max<long long>(want, 1) : d);
       have += team[k];
     }
@@ -738,8 +752,7 @@ constexpr int kQeqDirectIterations = 400;
 constexpr int kQeqDirectBlockAlone = 256;
 
 struct DirectPlan {
-  std::vector<int> cluster, block, small;  // clusters of `nb` blocks; single blocks; single blocks of small systems
-  int nb = 8;
+  std::vector<int> cluster, block, small;  // clusters of blocks; single blocks; single blocks of small systems
 };
 
 void plan_qeq_direct(const xr_ctx* c, const xr_system* sys, int nsys, DirectPlan& d, std::vector<int>& rest) {
@@ -750,16 +763,12 @@ void plan_qeq_direct(const xr_ctx* c, const xr_system* sys, int nsys, DirectPlan
       rest.push_back(s);
     else if (n <= kQeqDirectSmall)
       d.small.push_back(s);
-    else if (n <= (nsys == 1 && c->direct8 > 0 ? kQeqDirectBlockAlone : kQeqDirectMax))
+    else if (n <= (nsys == 1 && c->direct_cluster > 0 ? kQeqDirectBlockAlone : kQeqDirectMax))
       d.block.push_back(s);
-    else if (n <= c->direct8)
+    else if (n <= c->direct_cluster)
       d.cluster.push_back(s);
-    else if (nsys == 1 && n <= c->direct16) {  // a system alone also takes the wider clusters
-      d.cluster.push_back(s);
-      d.nb = 16;
-    } else {
+    else
       rest.push_back(s);
-    }
   }
   auto larger = [&](int a, int b) { return sys[a].natoms > sys[b].natoms; };
   for (std::vector<int>* v : {&d.cluster, &d.block, &d.small}) std::sort(v->begin(), v->end(), larger);
@@ -1328,7 +1337,7 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     const int* list = c->qsmall + (nlist - nd);
     for (int k = 0; k < 3; ++k) {
       if (dcount[k] == 0) continue;
-      const int le = k == 0 ? xr_launch_qeq_direct_cluster(w, ff->d, dst[0], list, dcount[0], dlargest[0], qd.nb, adjoint)
+      const int le = k == 0 ? xr_launch_qeq_direct_cluster(w, ff->d, dst[0], list, dcount[0], dlargest[0], adjoint)
                             : xr_launch_qeq_direct(w, ff->d, dst[k], list, dcount[k], dlargest[k], adjoint);
       if (le) return le;
       list += dcount[k];
@@ -1411,7 +1420,7 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
   bool done = false;
   if (c->graphs && !c->profile && qteam == 0) {
     const int ints[] = {(int)mode, qcluster ? 1 : 0, qcsize, qblocks, qteam, qsmall, qbig, nlist, nE > 0, nP > 0, nB > 0,
-                        (int)flags, dcount[0], dcount[1], dcount[2], dlargest[0], dlargest[1], dlargest[2], qd.nb,
+                        (int)flags, dcount[0], dcount[1], dcount[2], dlargest[0], dlargest[1], dlargest[2],
                         largest_system};
     const void* ptrs[] = {c->h_qmap_p, c->h_qsmall_p, c->qmap, c->qsmall, c->outbuf};
     const int nptrs = (int)(sizeof(ptrs) / sizeof(ptrs[0]));
@@ -1879,8 +1888,7 @@ int xr_ctx_create(int device, void* stream, xr_ctx** out) {
   c->coop_per_sm = xr_qeq_coop_blocks_per_sm();
   c->qeq_direct = xr_qeq_direct_ready();
   if (c->qeq_direct) {
-    c->direct8 = xr_qeq_direct_cluster_max(8);
-    c->direct16 = xr_qeq_direct_cluster_max(16);
+    c->direct_cluster = xr_qeq_direct_cluster_max();
   }
   c->max_clusters = xr_qeq_max_clusters(kQeqClusterSingle);
   c->max_clusters_batch = xr_qeq_max_clusters(kQeqClusterBatch);

@@ -2356,10 +2356,7 @@ __global__ void k_qeq_splits(XrWork w, const int* big, int nbig, int csize, cons
     const int4 m = map[t >> 1];
     sys = m.x;
     const int n = w.sys[sys].natoms;
-    // whole tiles of 32 rows for a team that has about one a block (fewer rows would leave lanes idle),
-    // equal shares above that (256 rows for 242 would leave 8 of 152 blocks without any)
-    int per = (n + m.z - 1) / m.z;
-    if (per <= 64) per = (per + 31) / 32 * 32;
+    const int per = (n + m.z - 1) / m.z;  // equal shares
     r = min(n, (m.y + (t & 1)) * per);
   }
   const XrSystem& S = w.sys[sys];

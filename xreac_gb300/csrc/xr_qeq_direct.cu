@@ -545,9 +545,10 @@ __global__ void __launch_bounds__(512, 1) k_qeq_direct(XrWork w, XrFF ff, const 
 // its rows, the owner of row k + 1 inverting that row's diagonal tile meanwhile. A substitution sends
 // one tile of the vector a step (forward), or adds its product to the other rows' tiles at their
 // owners (backward). All control flow is the same in every block (it depends on cluster-wide sums
-// only), so the blocks meet at the hardware cluster barrier. Measured on 8 blocks, CG then direct: 396
-// atoms 537 -> 266 us (factorization 90, a substitution 26); on 16, 648 atoms warm-started 508 -> 427
-// us; a batch of 128 requests of up to 512 atoms, all classes side by side, 1165 -> 351 us.
+// only), so the blocks meet at the hardware cluster barrier. Measured, CG then direct: 396 atoms 537 -> 266 us
+// (factorization 90, a substitution 26); a batch of 128 requests of up to 512 atoms, all classes side
+// by side, 1165 -> 351 us. Larger systems' chain of diagonal blocks is longer than a grid-wide team's CG: 648
+// atoms, warm-started, took 424 us on a cluster of 16 blocks and take 277 on a team.
 __device__ inline unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ inline unsigned remote(const void* p, int rank) {
   unsigned r;
@@ -590,17 +591,17 @@ __host__ __device__ constexpr size_t cluster_bytes(int n, int nb) {
 
 struct ClusterShared {
   DirectShared d;
-  double slots[2][16][4];  // partial sums by block, two exchanges' in turn
+  double slots[2][kQeqDirectBlocks][4];  // partial sums by block, two exchanges' in turn
 };
 
 struct ClusterLayout {
-  int T, nb, rank, own;  // tile rows; blocks; this block and its number of rows (atoms, padding included)
+  static constexpr int nb = kQeqDirectBlocks;
+  int T, rank, own;  // tile rows; this block and its number of rows (atoms, padding included)
   float *tiles, *panel, *dinv;
   double *X, *G;
   float *b, *w1;
-  __device__ ClusterLayout(unsigned char* dyn, int n, int blocks, int p) {
+  __device__ ClusterLayout(unsigned char* dyn, int n, int p) {
     T = (n + kTile - 1) / kTile;
-    nb = blocks;
     rank = p;
     own = kTile * rows_of(p, nb, T);
     tiles = reinterpret_cast<float*>(dyn);  // the same offsets in every block: remote addresses are local ones
@@ -644,7 +645,8 @@ __device__ inline void cluster_sums(const ClusterLayout& L, ClusterShared& sh, u
 }
 
 __device__ __noinline__ void cluster_factorize(const ClusterLayout& L, ClusterShared& sh) {
-  const int T = L.T, nb = L.nb, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
+  constexpr int nb = ClusterLayout::nb;
+  const int T = L.T, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
   const int rg = threadIdx.x & 7, cg = (threadIdx.x >> 3) & 3;
   if (L.rank == 0 && wid < 4) tile_inverse(L.tile(0, 0), nullptr, nullptr, sh.d);
   for (int k = 0; k + 1 < T; ++k) {
@@ -711,7 +713,8 @@ __device__ __noinline__ void cluster_factorize(const ClusterLayout& L, ClusterSh
 // H^-1 v for the NV vectors v[k], given and left in the owners' rows (a thread per own row).
 template <int NV>
 __device__ inline void cluster_substitute(const ClusterLayout& L, float* const (&v)[NV]) {
-  const int T = L.T, nb = L.nb, r = threadIdx.x;
+  constexpr int nb = ClusterLayout::nb;
+  const int T = L.T, r = threadIdx.x;
   const bool mine = r < L.own;
   const int at = mine ? L.row(r) : 0, i = at >> 5;
   auto publish = [&](int q) {  // this thread's row of every vector, to every block
@@ -781,9 +784,10 @@ __device__ inline void cluster_substitute(const ClusterLayout& L, float* const (
   }
 }
 
-__global__ void __launch_bounds__(512, 1) k_qeq_direct_cluster(XrWork w, XrFF ff, const int* list, int nb, int adjoint) {
+__global__ void __launch_bounds__(512, 1) k_qeq_direct_cluster(XrWork w, XrFF ff, const int* list, int adjoint) {
   __shared__ ClusterShared sh;
   extern __shared__ __align__(16) unsigned char dyn[];
+  constexpr int nb = kQeqDirectBlocks;
   const int sys = list[blockIdx.x / nb];
   const XrSystem& S = w.sys[sys];
   const int a0 = S.atom_off, n = S.natoms, tid = threadIdx.x, wid = tid >> 5, nw = blockDim.x >> 5;
@@ -791,7 +795,7 @@ __global__ void __launch_bounds__(512, 1) k_qeq_direct_cluster(XrWork w, XrFF ff
   const double Q = adjoint ? 0.0 : S.total_charge;
   const bool warm = !adjoint && S.has_guess != 0;
   const double x0 = Q == 0.0 ? 0.0 : Q / n;
-  const ClusterLayout L(dyn, n, nb, blockIdx.x % nb);
+  const ClusterLayout L(dyn, n, blockIdx.x % nb);
   const int at = tid < L.own ? L.row(tid) : 0, m = min(L.own, max(0, L.own > 0 ? L.own - max(0, kTile * L.T - n) *
                                                                               (L.owner(L.T - 1) == L.rank ? 1 : 0) : 0));
   const bool row = tid < m;  // (only the last tile row has padding)
@@ -928,14 +932,14 @@ __global__ void __launch_bounds__(512, 1) k_qeq_direct_cluster(XrWork w, XrFF ff
   w.a_e[(size_t)6 * w.A + a] = SELF_CONVERSION * (chi * q + 0.5 * eta * q * q);
 }
 
-cudaLaunchConfig_t cluster_config(int nb, int count, size_t bytes, cudaStream_t st, cudaLaunchAttribute* attr) {
+cudaLaunchConfig_t cluster_config(int count, size_t bytes, cudaStream_t st, cudaLaunchAttribute* attr) {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(nb * count);
+  cfg.gridDim = dim3(kQeqDirectBlocks * count);
   cfg.blockDim = dim3(512);
   cfg.dynamicSmemBytes = bytes;
   cfg.stream = st;
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = nb;
+  attr[0].val.clusterDim.x = kQeqDirectBlocks;
   attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
@@ -945,28 +949,26 @@ cudaLaunchConfig_t cluster_config(int nb, int count, size_t bytes, cudaStream_t 
 
 }  // namespace
 
-int xr_qeq_direct_cluster_max(int nb) {
-  const int largest = nb == 8 ? kQeqDirectCluster8 : kQeqDirectCluster16;
+int xr_qeq_direct_cluster_max() {
+  constexpr int largest = kQeqDirectCluster;
   bool ok = cudaFuncSetAttribute(k_qeq_direct_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)std::max(cluster_bytes(kQeqDirectCluster8, 8), cluster_bytes(kQeqDirectCluster16, 16))) ==
+                                 (int)cluster_bytes(largest, kQeqDirectBlocks)) ==
             cudaSuccess;
-  if (nb > 8)  // past the portable cluster size
-    ok = ok && cudaFuncSetAttribute(k_qeq_direct_cluster, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) == cudaSuccess;
   int clusters = 0;
   if (ok) {
     cudaLaunchAttribute attr[1];
-    cudaLaunchConfig_t cfg = cluster_config(nb, 1, cluster_bytes(largest, nb), nullptr, attr);
+    cudaLaunchConfig_t cfg = cluster_config(1, cluster_bytes(largest, kQeqDirectBlocks), nullptr, attr);
     ok = cudaOccupancyMaxActiveClusters(&clusters, (void*)k_qeq_direct_cluster, &cfg) == cudaSuccess;
   }
   if (!ok) cudaGetLastError();
   return ok && clusters > 0 ? largest : 0;
 }
 
-int xr_launch_qeq_direct_cluster(const XrWork& w, const XrFF& ff, cudaStream_t st, const int* list, int count, int largest, int nb,
+int xr_launch_qeq_direct_cluster(const XrWork& w, const XrFF& ff, cudaStream_t st, const int* list, int count, int largest,
                                  bool adjoint) {
   cudaLaunchAttribute attr[1];
-  cudaLaunchConfig_t cfg = cluster_config(nb, count, cluster_bytes(largest, nb), st, attr);
-  return (int)cudaLaunchKernelEx(&cfg, k_qeq_direct_cluster, w, ff, list, nb, adjoint ? 1 : 0);
+  cudaLaunchConfig_t cfg = cluster_config(count, cluster_bytes(largest, kQeqDirectBlocks), st, attr);
+  return (int)cudaLaunchKernelEx(&cfg, k_qeq_direct_cluster, w, ff, list, adjoint ? 1 : 0);
 }
 
 bool xr_qeq_direct_ready() {
