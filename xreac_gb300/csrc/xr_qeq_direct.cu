@@ -18,7 +18,7 @@
 // the others update the rest. A tile product is bound by shared-memory loads: each lane forms 4 x 8
 // entries, so that 12 load wavefronts feed 32 multiply-adds.
 //
-// What bounds it: the chain of diagonal blocks (32 dependent pivots each), and for the gradients the
+// What bounds it: the chain of diagonal blocks (16 dependent pairs of pivots each), and for the gradients the
 // FP64 pipe (an entry is one of its multiply-adds, two a clock).
 #include <algorithm>
 
@@ -38,7 +38,7 @@ struct DirectShared {
   double red[8][16];  // warp partials of a block sum
   double tot[8];
   float redf[2][16], totf[2];
-  float column[2][kTile];  // the pivot column of an inversion, two steps' in turn
+  float column[4][kTile];  // the two pivot columns of an inversion, two steps' in turn
   unsigned short map[kMaxTiles * (kMaxTiles + 1) / 2 + kMaxTiles];  // tile (i, j) -> slot; then the scratch slots
 };
 
@@ -129,10 +129,11 @@ __device__ inline void tile_product(const float* a, const float* b, int c0, floa
 }
 
 // Warps 0 to 3: tile t less the product of w and a (null: of nothing), replaced by its inverse. Gauss-Jordan
-// without pivoting, lane = row, warp q holds columns 8 q .. 8 q + 7; the pivot column goes through shared
-// memory, one barrier of the four warps a pivot. A vanishing pivot gives non-finite entries, which
-// the refinement notices. (By one warp, all 32 columns unrolled, it took 11 us: 4,000 instructions do
-// not fit the instruction cache.)
+// without pivoting, two pivots at a time, lane = row, warp q holds columns 8 q .. 8 q + 7; the pivot columns go through
+// shared memory, one barrier of the four warps and one reciprocal (of the 2 x 2 block's determinant) a pair. With one
+// pivot at a time QEq took 234 us for 375 atoms (224), 174 for a 288-atom slab (167) and 116 for 192 atoms (112).
+// A vanishing determinant gives non-finite entries, which the refinement notices. (By one warp, all 32 columns
+// unrolled, an inversion took 11 us: 4,000 instructions do not fit the instruction cache.)
 __device__ __noinline__ void tile_inverse(float* t, const float* w, const float* a, DirectShared& sh) {
   const int lane = threadIdx.x & 31, q = threadIdx.x >> 5;
   float v[8];
@@ -156,20 +157,31 @@ __device__ __noinline__ void tile_inverse(float* t, const float* w, const float*
   }
   for (int cb = 0; cb < 4; ++cb) {
 #pragma unroll
-    for (int ci = 0; ci < 8; ++ci) {
+    for (int ci = 0; ci < 8; ci += 2) {
       const int c = 8 * cb + ci;
-      float* const col = sh.column[ci & 1];
-      if (q == cb) col[lane] = v[ci];
+      float* const ca = sh.column[ci & 2];
+      float* const cd = sh.column[(ci & 2) + 1];
+      if (q == cb) {
+        ca[lane] = v[ci];
+        cd[lane] = v[ci + 1];
+      }
       asm volatile("bar.sync 1, 128;" ::: "memory");
-      const float inv = __fdividef(1.0f, col[c]);
-      const bool own = lane == c;
-      const float f = own ? -inv : col[lane] * inv;
+      // the pivot block's rows times its inverse (p11 -p01; -p10 p00) / det
+      const float2 pa = *reinterpret_cast<const float2*>(ca + c), pb = *reinterpret_cast<const float2*>(cd + c);
+      const float inv = __fdividef(1.0f, pa.x * pb.y - pb.x * pa.y);
+      const float x = ca[lane], y = cd[lane];
+      const bool first = lane == c, second = lane == c + 1, own = first || second;
+      const float fa = (first ? -pb.y : second ? pa.y : x * pb.y - y * pa.y) * inv;
+      const float fb = (first ? pb.x : second ? -pa.x : y * pa.x - x * pb.x) * inv;
 #pragma unroll
       for (int j = 0; j < 8; ++j) {
-        const float p = __shfl_sync(0xffffffffu, v[j], c);
-        v[j] = (own ? 0.0f : v[j]) - f * p;
+        const float p0 = __shfl_sync(0xffffffffu, v[j], c), p1 = __shfl_sync(0xffffffffu, v[j], c + 1);
+        v[j] = (own ? 0.0f : v[j]) - fa * p0 - fb * p1;
       }
-      if (q == cb) v[ci] = own ? inv : -f;
+      if (q == cb) {
+        v[ci] = -fa;
+        v[ci + 1] = -fb;
+      }
     }
   }
 #pragma unroll
