@@ -149,18 +149,17 @@ __device__ inline void pair_one(const XrWork& w, const XrFF& ff0, int p) {
   w.p_g[p] = G;
   if (w.pgrad && taper != 0.0) {
     // dE/d(D, alpha, r_vdW, gamma_w) of this pair's tapered vdW term (and the inner core's)
-    const double rvdw = pair_prm(ff, pt, P_RVDW);
     double* gp = xr_pgrad(w, i) + (size_t)pt * XR_NPAIR_COLS;
     const double m = taper * D * (2 * ev - 2) * ev;  // dE/d(log ev) per unit of the exponent's argument
     atomicAdd(gp + P_D, taper * (ev * ev - 2 * ev));
-    atomicAdd(gp + P_ALPHA, m * 0.5 * (1 - f13 / rvdw));
-    atomicAdd(gp + P_RVDW, m * 0.5 * alpha * f13 / (rvdw * rvdw));
+    atomicAdd(gp + P_ALPHA, m * 0.5 * (1 - f13 * inv.x));
+    atomicAdd(gp + P_RVDW, m * 0.5 * ax * f13 * inv.x);
     if (ff.vdw_type == 1 || ff.vdw_type == 3) {
       // f13 = (r^p + gw)^(1/p) with gw = gamma_w^-p: d f13 / d gamma_w = -f13 gw / (sum gamma_w)
       const double pw = ff.g[28], gw = __ldg(ff.pair_gw + pt);
       const double sum = exp(pw * log(r)) + gw;
       const double gamw = pair_prm(ff, pt, P_GAMMA_W);
-      atomicAdd(gp + P_GAMMA_W, m * (-0.5 * alpha / rvdw) * (-f13 * gw / (sum * gamw)));
+      atomicAdd(gp + P_GAMMA_W, m * 0.5 * ax * (f13 * gw / (sum * gamw)));
     }
     if (ff.vdw_type == 2 || ff.vdw_type == 3) {
       const double ecore = pair_prm(ff, pt, P_ECORE), acore = pair_prm(ff, pt, P_ACORE), rcore = pair_prm(ff, pt, P_RCORE);
