@@ -738,15 +738,15 @@ def main():
                        "max": float(lat.max()), "queue_p50": float(np.percentile(qwait, 50)),
                        "queue_p99": float(np.percentile(qwait, 99)), "arrival_rate_per_s": 2000,
                        "batches": replay_batches, "requests": int(len(lat)), "max_atoms_per_request": 512},
-        "roofline": {"bound": "hbm", "kernel": "k_qeq_cluster (QEq solve of the served batches)",
+        "roofline": {"bound": "hbm", "kernel": "k_qeq_direct, k_qeq_direct_cluster (QEq solves of the served batches)",
                      "achieved": qeq_achieved, "peak": hbm_peak, "unit": "GB/s", "frac": qeq_achieved / hbm_peak,
-                     "traffic": profiled_traffic("k_qeq_cluster"),
+                     "traffic": profiled_traffic("k_qeq_direct"),
                      "algorithmic_bytes_per_launch": qeq_bytes / max(serial_batches, 1), "dominant_stage": dominant,
                      "peak_source": "MEASURED_PEAKS.json hbm_gbs" if "hbm_gbs" in pk else "fallback 6800 GB/s",
                      "note": "achieved = matrix-free algorithmic bytes / QEq event time, averaged over the launches "
-                             "(one per batch); traffic = DRAM bytes of one served batch's launch from an ncu "
-                             "capture. The solve keeps its matrix rows on chip and is bound by the cluster "
-                             "exchanges and shared-memory gathers, not HBM"},
+                             "(one per batch); traffic = DRAM bytes of one served batch's launches from an ncu "
+                             "capture. The solve keeps its matrix on chip and is bound by the chain of diagonal "
+                             "blocks, the cluster barriers and the FP64 pipe, not HBM"},
         "stages_ms_per_pass": stages,
         "device_time": "value, ms_per_step and stages: the stream's batches (16,384 atoms at most, per force field) "
                        "evaluated one after another on one context, CUDA events per stage, no overlap between batches; "

@@ -277,12 +277,13 @@ long long xr_last_launches(const xr_ctx* ctx);
  * [5] torsion middle bonds (bo > 0.001). The first n (at most 6) are written. */
 int xr_last_list_sizes(const xr_ctx* ctx, long long* sizes, int n);
 
-/* QEq conjugate-gradient iterations of the last call (largest over its systems; no reference
- * counterpart: the reference solves the KKT system directly). */
+/* QEq iterations of the last call (largest over its systems): conjugate-gradient iterations, or the refinement steps
+ * of a system solved directly (up to 608 atoms). No reference counterpart: the reference solves the KKT system
+ * directly. */
 int xr_last_qeq_iterations(const xr_ctx* ctx);
 
-/* QEq work of the last call (no reference counterpart; instrumentation): the conjugate-gradient
- * iterations summed over its systems, and the algorithmic bytes of a matrix-free product summed
+/* QEq work of the last call (no reference counterpart; instrumentation): the iterations (as above)
+ * summed over its systems, and the algorithmic bytes of a matrix-free product summed
  * over every iteration of every system: iterations x (8 B per unordered pair + 16 B per atom). */
 int xr_last_qeq_work(const xr_ctx* ctx, long long* iterations, double* matvec_bytes);
 
