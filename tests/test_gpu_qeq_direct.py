@@ -45,7 +45,7 @@ def _dense(symbols, x, cell=None, charge=0.0):
     return oracle.qeq_charges(oracle._Model(ff, symbols, edges), np.sqrt((v * v).sum(axis=1)), charge)
 
 
-SIZES = [1, 2, 3, 31, 32, 33, 63, 64, 65, 95, 96, 97, 128, 129, 160, 191, 256, 257, 287, 288, 289,
+SIZES = [1, 2, 3, 31, 32, 33, 63, 64, 65, 95, 96, 97, 128, 129, 160, 191, 192, 193, 224, 225, 256, 257, 287, 288, 289,
          320, 321, 415, 416, 417, 512, 513, 607, 608, 609, 641, 704, 735, 736, 737]
 
 

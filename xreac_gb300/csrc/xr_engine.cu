@@ -746,10 +746,10 @@ bool plan_qeq_cluster(xr_ctx* c, const xr_system* sys, int nsys, const std::vect
 // run out, gets the CG solver whose iterations and waits those are.
 constexpr int kQeqDirectIterations = 400;
 // The largest system alone in its call that one block solves. A cluster pays two cluster barriers a tile step and has
-// eight blocks' FP64 for the products of periodic systems' long rows: with eight tile rows a block takes 152 us
-// for 240 atoms of water, open, and 197 in a cell, a cluster 168 and 182; with nine (288 atoms) a block 192 and 283, a cluster 191 and
-// 217.
-constexpr int kQeqDirectBlockAlone = 256;
+// eight blocks' FP64 for the products of long rows: a block takes 111 us for 192 atoms of water, open, and 178 in a
+// cell, a cluster 116 and 136; for 225 atoms 140 and 180 against 137 and 148, for 288 186 and 273 against 165 and 186;
+// for 99 open atoms 75 against 94.
+constexpr int kQeqDirectBlockAlone = 192;
 
 struct DirectPlan {
   std::vector<int> cluster, block, small;  // clusters of blocks; single blocks; single blocks of small systems

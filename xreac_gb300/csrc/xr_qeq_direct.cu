@@ -2,8 +2,8 @@
 //
 // A system of up to kQeqDirectMax atoms has its whole matrix in one block's shared memory. The CG
 // it would take otherwise needs 30 to 140 iterations of 2 to 7 us (two team reductions each).
-// Measured, CG then direct: 192 atoms 293 -> 115 us, a 288-atom periodic slab 420 -> 221 us, 3
-// atoms 61 -> 37 us, a batch of 192 systems of up to 64 atoms 179 -> 58 us. The KKT system of
+// Measured, CG then direct: 192 atoms 293 -> 112 us, 9 atoms 61 -> 38 us, a batch of 192 systems of
+// up to 64 atoms 179 -> 56 us. The KKT system of
 // src/xreac/energy.py:95-102 is solved by iterative refinement, as the FP32 CG's sweeps are: each
 // step solves H y = -g, sum y = 0 for the FP64 gradient g = H x + chi - lambda projected onto the
 // constraint, adds y to the FP64 charges, restores sum x = Q and forms the gradient again in FP64
@@ -557,9 +557,9 @@ __global__ void __launch_bounds__(512, 1) k_qeq_direct(XrWork w, XrFF ff, const 
 // its rows, the owner of row k + 1 inverting that row's diagonal tile meanwhile. A substitution sends
 // one tile of the vector a step (forward), or adds its product to the other rows' tiles at their
 // owners (backward). All control flow is the same in every block (it depends on cluster-wide sums
-// only), so the blocks meet at the hardware cluster barrier. Measured, CG then direct: 396 atoms 537 -> 266 us
-// (factorization 90, a substitution 26); a batch of 128 requests of up to 512 atoms, all classes side
-// by side, 1165 -> 351 us. Larger systems' chain of diagonal blocks is longer than a grid-wide team's CG: 648
+// only), so the blocks meet at the hardware cluster barrier. Measured, CG then direct: 375 atoms 541 -> 224 us, a
+// 288-atom periodic slab 420 -> 167 us; a batch of 128 requests of up to 512 atoms, all classes side
+// by side, 1165 -> 293 us. Larger systems' chain of diagonal blocks is longer than a grid-wide team's CG: 648
 // atoms, warm-started, took 424 us on a cluster of 16 blocks and take 277 on a team.
 __device__ inline unsigned smem_u32(const void* p) { return (unsigned)__cvta_generic_to_shared(p); }
 __device__ inline unsigned remote(const void* p, int rank) {
