@@ -916,7 +916,8 @@ class Calculator:
         return int(self._lib.xr_last_launches(self._ctx.handle))
 
     def qeq_work(self):
-        """(CG iterations summed over the last call's systems, their matrix-free algorithmic bytes)."""
+        """(QEq iterations summed over the last call's systems: CG iterations, or the refinement steps of direct
+        solves; their matrix-free algorithmic bytes)."""
         its = nat.c_longlong()
         b = nat.c_double()
         self._lib.xr_last_qeq_work(self._ctx.handle, nat.byref(its), nat.byref(b))
