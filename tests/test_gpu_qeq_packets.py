@@ -52,3 +52,17 @@ def test_exchange_that_runs_out_raises_and_the_context_recovers(n_mol, fail_at):
     got = calc.evaluate(**s)
     assert got.energy == want.energy
     np.testing.assert_array_equal(got.charges, want.charges)
+
+
+# two teams of 1,024-thread blocks (9,003 and 9,000 atoms, about 120 rows a block), whose plain rows lie side by side
+def test_teams_with_plain_rows_do_not_touch_each_other():
+    calc = calculator()
+    boxes = [system(n) for n in (3001, 3000)]
+    got = calc.evaluate_many(boxes)
+    for s, g in zip(boxes, got):
+        want = calc.evaluate(**s)
+        # the bound above at 9,003 atoms: 1e-13 * 0.5 * sqrt(9003) * sqrt(14) = 1.8e-11 for each of the two
+        np.testing.assert_allclose(g.charges, want.charges, atol=4e-11, rtol=0)
+    for _ in range(3):
+        for g, again in zip(got, calc.evaluate_many(boxes)):
+            np.testing.assert_array_equal(again.charges, g.charges)

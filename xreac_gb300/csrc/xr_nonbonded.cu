@@ -377,11 +377,13 @@ struct GridPackets {
   // 8 bytes per atom and buffer, among the FP32 vectors that only the solver over global rows uses
   static __device__ float* rows_of(const XrWork& w, float* F, int k) { return F + (k ? 6 : 2) * (size_t)w.A; }
   __device__ uint4* scalar(unsigned tag, int r) const { return scalars + 4 * ((tag & 1u) * nb + r); }
-  // Once per solve, before a barrier: the rank's packets carry no tag of an earlier solve.
+  // Once per solve, before a barrier: the rank's packets carry no tag of an earlier solve. Plain rows carry none, and
+  // the memory of row packets is other teams' rows there, which no barrier of this team orders.
   template <int T>
   static __device__ void clear(const XrWork& w, const GridTeam<T>& team, float* F, int a0, int r0, int r1) {
-    for (int r = 2 * r0 + (int)threadIdx.x; r < 2 * r1; r += blockDim.x)
-      rows_of(w, F, 0)[2 * a0 + r] = rows_of(w, F, 1)[2 * a0 + r] = 0.0f;
+    if constexpr (T <= kTeamThreads)
+      for (int r = 2 * r0 + (int)threadIdx.x; r < 2 * r1; r += blockDim.x)
+        rows_of(w, F, 0)[2 * a0 + r] = rows_of(w, F, 1)[2 * a0 + r] = 0.0f;
     if (threadIdx.x < 2)
       *reinterpret_cast<uint4*>(team.red + ((1 + threadIdx.x) * (size_t)team.nb + team.rank) * 8 + 6) = make_uint4(0u, 0u, 0u, 0u);
   }
