@@ -209,3 +209,20 @@ def test_skin_list_of_a_batch_and_of_the_water_box():
     assert c.list_info() == ("reused", 2)
     for a, b in zip(got, fresh.evaluate_many(moved)):
         _same(a, b)
+
+
+def test_a_reservation_drops_the_kept_skin_list():
+    """A reservation that moves the list's buffers: the next call builds the list anew, with the same result."""
+    from xreac_gb300 import Calculator, ForceField
+    from xreac_gb300.workloads import water_cluster
+
+    s = water_cluster(n_mol=30, box=9.7, min_oo=2.4, seed=5, jitter=0.05)
+    calc = Calculator(ForceField.bundled("ffield.reax.HO.2015"))
+    calc.set_neighbor_skin(0.3)
+    first = calc.evaluate(s.symbols, s.positions)
+    calc.evaluate(s.symbols, s.positions)
+    assert calc.list_info() == ("reused", 1)
+    calc.reserve(2000, 4)
+    again = calc.evaluate(s.symbols, s.positions)
+    assert calc.list_info() == ("built", 2)
+    assert again.energy == first.energy

@@ -2148,6 +2148,7 @@ int xr_get_bonds(xr_ctx* c, int index, int* i, int* j, int* S, double* bo, long 
 int xr_ctx_reserve(xr_ctx* c, int atoms, int systems, long long edges, long long bonds) {
   if (!c || atoms < 1 || systems < 1 || edges < 0 || bonds < 0) return XR_EINPUT;
   cudaSetDevice(c->device);
+  c->cache_valid = false;  // a skin list does not outlive its buffers, which may move
   const long long chunks = (long long)systems + atoms / XR_CHUNK_ATOMS + 1;
   // pinned host buffers too: a call within the reservation allocates and frees no page-locked memory
   // (whose allocation stalls, and whose release waits for the whole device, other threads' work included)
