@@ -68,3 +68,28 @@ def test_row_bitmaps(n_mol):
 
     s = water_box(n_mol=n_mol, box=max(20.5, (31.0 * n_mol) ** (1 / 3)), min_oo=2.4, seed=n_mol)
     _check(list(s.symbols), np.array(s.positions), s.cell, True, cells=True, calls=1)
+
+
+# far more row slots than edges: 298 molecules 8 A apart, alone and in a periodic cell, by image scan and cell list
+@pytest.mark.parametrize("cells", [False, True])
+@pytest.mark.parametrize("periodic", [False, True])
+def test_calls_within_a_reservation_allocate_nothing(periodic, cells):
+    from oracle import reaxff_oracle as oracle
+    from xreac_gb300 import Calculator, ForceField
+    from xreac_gb300.workloads import MOLECULES
+
+    ff = ForceField.bundled(FF)
+    symbols, water = MOLECULES["H2O"]()
+    sites = 8.0 * np.stack(np.unravel_index(np.arange(298), (7, 7, 7)), axis=1)
+    x = (sites[:, None, :] + np.asarray(water)).reshape(-1, 3)
+    symbols = list(symbols) * 298
+    cell = np.diag([56.0] * 3) if periodic else None
+    want = oracle.neighbor_list(x, float(ff.general[12]), cell, periodic or None)
+    calc = Calculator(ff)
+    calc.set_cell_list(cells)
+    calc.reserve(894, 1, edges_per_atom=len(want[0]) / 894, bonds_per_atom=3)
+    before = calc.memory()
+    calc.evaluate(symbols, x, cell=cell, pbc=periodic)
+    assert calc.memory() == before
+    for got, ref in zip(calc.neighbor_list(), want):
+        np.testing.assert_array_equal(got, ref)

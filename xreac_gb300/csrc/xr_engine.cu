@@ -117,6 +117,7 @@ struct xr_ctx {
   size_t ccell_atoms = 0;
   float4* cell_pos = nullptr;
   size_t ccell_pos = 0;
+  int reserved_atoms = 0, reserved_systems = 0;  // of the last xr_ctx_reserve
   int row_longest = 0;  // the longest row that did not fit the slots its system's density suggested
   double row_scale = 1.0;  // slots of k_scan_rows' periodic rows over what the density suggests: grows when one did not fit
   // Skin reuse (xr_ctx_set_skin): the list of the last call is reused by a call on the same systems
@@ -867,6 +868,18 @@ long long plan_cells(xr_ctx* c, int nsys, const xr_system* sys, double rl, XrSys
   return use ? total : 0;
 }
 
+// Whether cand_edge's memory has, or can be given, room for `slots` kept row entries. They save a second search but
+// no call needs them: a call within the context's reservation allocates nothing for them (the reservation sizes this buffer by
+// its edges), and one whose slots the device has no memory for goes without.
+bool row_room(xr_ctx* c, int A, int nsys, long long slots) {
+  const size_t need = (size_t)(slots + 1) / 2;
+  if (c->cand_edge && need <= c->ccand_edge) return true;
+  if (A <= c->reserved_atoms && nsys <= c->reserved_systems) return false;
+  if (grow(c, &c->cand_edge, &c->ccand_edge, need)) return true;
+  cudaGetLastError();
+  return false;
+}
+
 // Slots per row for a call whose rows come straight from the cell list (k_cell_rows): a third above what each
 // system's mean density gives, at least the longest row that exceeded that before; 0 where the call's systems do
 // not allow it (several images of an atom within the cutoff, too many atoms).
@@ -1094,21 +1107,13 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
       if (mode == kScan) {
         mode = kCell;
         row_cap = plan_cell_rows(c, nsys, sys, A, rc);
-        if (row_cap > 0) {
-          if (!grow(c, &c->cand_edge, &c->ccand_edge, ((size_t)A * row_cap + 1) / 2))
-            return cuda_fail(c, cudaErrorMemoryAllocation, "allocation");
-          mode = kCellRows;
-        }
+        if (row_cap > 0 && row_room(c, A, nsys, (long long)A * row_cap)) mode = kCellRows;
       }
     }
   }
   if (mode == kScan) {
     const long long slots = plan_scan_rows(c, nsys, sys, rc);
-    if (slots > 0) {
-      if (!grow(c, &c->cand_edge, &c->ccand_edge, (size_t)(slots + 1) / 2))
-        return cuda_fail(c, cudaErrorMemoryAllocation, "allocation");
-      mode = kScanRows;
-    }
+    if (slots > 0 && row_room(c, A, nsys, slots)) mode = kScanRows;
   }
   // energy-reduction chunks: each system's atoms in runs of XR_CHUNK_ATOMS, numbered in system order
   size_t nchunk = 0;
@@ -2168,6 +2173,8 @@ int xr_ctx_reserve(xr_ctx* c, int atoms, int systems, long long edges, long long
       !grow(c, &c->cell_atoms, &c->ccell_atoms, (size_t)atoms) || !grow(c, &c->cell_pos, &c->ccell_pos, (size_t)atoms) ||
       !grow(c, &c->cell_cnt, &c->ccell_cnt, 2 * (size_t)atoms + 64 * (size_t)systems + 1))
     return cuda_fail(c, cudaErrorMemoryAllocation, "reservation");
+  c->reserved_atoms = atoms;
+  c->reserved_systems = systems;
   return XR_OK;
 }
 
