@@ -93,3 +93,24 @@ def test_calls_within_a_reservation_allocate_nothing(periodic, cells):
     assert calc.memory() == before
     for got, ref in zip(calc.neighbor_list(), want):
         np.testing.assert_array_equal(got, ref)
+
+
+def test_slots_follow_the_longest_row():
+    """Rows that did not fit once fit from the next call on, and other systems keep their slots."""
+    from xreac_gb300 import Calculator, ForceField
+
+    calc = Calculator(ForceField.bundled(FF), max_expanded_atoms=1 << 30)
+    calc.set_cell_list(False)
+    symbols, x = _water(200, seed=7)  # liquid density in a corner of a nearly empty cell
+    cell = np.diag([90.0] * 3)
+    for _ in range(2):
+        calc.evaluate(symbols, x, cell=cell, pbc=True)
+    held = calc.memory()
+    longest = np.bincount(calc.neighbor_list()[0]).max()
+    assert 2 * held["candidates"] >= len(x) * longest
+    for _ in range(10):
+        calc.evaluate(symbols, x, cell=cell, pbc=True)
+    assert calc.memory() == held
+    symbols, x = _water(100, seed=8)
+    calc.evaluate(symbols, x, cell=np.diag([14.5] * 3), pbc=True)
+    assert calc.memory()["candidates"] == held["candidates"]

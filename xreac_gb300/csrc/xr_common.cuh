@@ -331,7 +331,7 @@ void xr_launch_topology(const XrWork& w, cudaStream_t st);  // xr_launch_prep, t
 void xr_launch_prep(const XrWork& w, cudaStream_t st);      // wrapped FP32 coordinates (k_prep)
 void xr_launch_count(const XrWork& w, cudaStream_t st);     // all-pairs image scan, counts (k_neighbors<false>)
 void xr_launch_rows(const XrWork& w, cudaStream_t st);      // all-pairs image scan, rows (k_neighbors<true>)
-// The image scan with its rows kept (XrSystem::row_cap; counts[6] set when a row did not fit), then, after
+// The image scan with its rows kept (XrSystem::row_cap; counts[6]: the longest row that did not fit), then, after
 // xr_launch_scan, the rows, pairs and bonds.
 void xr_launch_scan_rows(const XrWork& w, cudaStream_t st);
 void xr_launch_emit_rows(const XrWork& w, cudaStream_t st);

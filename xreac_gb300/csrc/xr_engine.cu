@@ -119,7 +119,6 @@ struct xr_ctx {
   size_t ccell_pos = 0;
   int reserved_atoms = 0, reserved_systems = 0;  // of the last xr_ctx_reserve
   int row_longest = 0;  // the longest row that did not fit the slots its system's density suggested
-  double row_scale = 1.0;  // slots of k_scan_rows' periodic rows over what the density suggests: grows when one did not fit
   // Skin reuse (xr_ctx_set_skin): the list of the last call is reused by a call on the same systems
   // (atom counts, types, cells, pbc, cutoff) in which no atom moved more than `skin` from where it was
   // when the list was built; the list holds every image within rc + 2 skin then (ASE's convention).
@@ -881,9 +880,9 @@ bool row_room(xr_ctx* c, int A, int nsys, long long slots) {
 }
 
 // Slots per row for a call whose rows come straight from the cell list (k_cell_rows): a third above what each
-// system's mean density gives, at least the longest row that exceeded that before; 0 where the call's systems do
-// not allow it (several images of an atom within the cutoff, too many atoms).
-int plan_cell_rows(const xr_ctx* c, int nsys, const xr_system* sys, int A, double rc) {
+// system's mean density gives, and with `learned` at least a tenth above the longest row that exceeded that before; 0
+// where the call's systems do not allow it (several images of an atom within the cutoff, too many atoms).
+int plan_cell_rows(const xr_ctx* c, int nsys, const xr_system* sys, int A, double rc, bool learned) {
   if (A >= 1 << 24) return 0;
   double most = 0.0;
   int largest = 0;
@@ -898,16 +897,18 @@ int plan_cell_rows(const xr_ctx* c, int nsys, const xr_system* sys, int A, doubl
     most = std::max(most, std::min<double>(sys[s].natoms, 1.35 * mean + 64.0));
     largest = std::max(largest, sys[s].natoms);
   }
-  const double cap = std::min<double>(largest, std::max<double>(most, c->row_longest * 1.1));
+  const double cap = std::min<double>(largest, std::max<double>(most, learned ? c->row_longest * 1.1 : 0.0));
   return cap * A > 1e9 ? 0 : ((int)cap + 3) / 4 * 4;
 }
 
 // Slots of the image scan's rows (k_scan_rows): every atom of a small open system, a third above what the mean density
-// gives in a periodic cell, else nearly twice a liquid's row; rows of up to 900 words lie within a reservation of 450
-// directed edges per atom. Returns the entries in all, 0 where the call's systems do not allow it (too many atoms or
-// images).
+// gives in a periodic cell, else nearly twice a liquid's row, and with `learned` at least a tenth above the longest row
+// that did not fit before (a cluster or a slab in a large cell: 600 atoms of water in a cell of 90 A have rows
+// of up to 359 where the mean suggests 68); rows of up to 900 words lie within a reservation of 450 directed edges per
+// atom. Returns the entries in all, 0 where the call's systems do not allow it (too many atoms or images).
 constexpr int kScanImages = 64;
-long long plan_scan_rows(xr_ctx* c, int nsys, const xr_system* sys, double rc) {
+long long plan_scan_rows(xr_ctx* c, int nsys, const xr_system* sys, double rc, bool learned) {
+  const long long least = learned ? (long long)(c->row_longest * 1.1) : 0;
   long long total = 0;
   for (int s = 0; s < nsys; ++s) {
     XrSystem& S = c->host_sys[s];
@@ -919,9 +920,9 @@ long long plan_scan_rows(xr_ctx* c, int nsys, const xr_system* sys, double rc) {
       const double* m = S.cell;
       const double volume = m[0] * (m[4] * m[8] - m[5] * m[7]) + m[1] * (m[5] * m[6] - m[3] * m[8]) + m[2] * (m[3] * m[7] - m[4] * m[6]);
       const double mean = n / volume * (4.0 / 3.0 * 3.14159265) * rc * rc * rc;
-      cap = std::min(cap, (long long)std::min(1e9, c->row_scale * 1.35 * mean + 64.0));
+      cap = std::min(cap, std::max(least, (long long)std::min(1e9, 1.35 * mean + 64.0)));
     } else if (n > 896 || images > 1) {
-      cap = std::min(cap, (long long)(c->row_scale * 768.0));
+      cap = std::min(cap, std::max(least, 768ll));
     }
     S.row_cap = (int)cap;
     S.row_off = total;
@@ -1106,14 +1107,24 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
         return cuda_fail(c, cudaErrorMemoryAllocation, "allocation");
       if (mode == kScan) {
         mode = kCell;
-        row_cap = plan_cell_rows(c, nsys, sys, A, rc);
-        if (row_cap > 0 && row_room(c, A, nsys, (long long)A * row_cap)) mode = kCellRows;
+        for (const bool learned : {true, false}) {  // (without what other systems taught where that has no room)
+          row_cap = plan_cell_rows(c, nsys, sys, A, rc, learned);
+          if (row_cap > 0 && row_room(c, A, nsys, (long long)A * row_cap)) {
+            mode = kCellRows;
+            break;
+          }
+        }
       }
     }
   }
   if (mode == kScan) {
-    const long long slots = plan_scan_rows(c, nsys, sys, rc);
-    if (slots > 0 && row_room(c, A, nsys, slots)) mode = kScanRows;
+    for (const bool learned : {true, false}) {
+      const long long slots = plan_scan_rows(c, nsys, sys, rc, learned);
+      if (slots > 0 && row_room(c, A, nsys, slots)) {
+        mode = kScanRows;
+        break;
+      }
+    }
   }
   // energy-reduction chunks: each system's atoms in runs of XR_CHUNK_ATOMS, numbered in system order
   size_t nchunk = 0;
@@ -1266,7 +1277,7 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(c, e, "neighbour count");
     if (int code = status_to_code(c, c->h_small[8])) return code;
     if (mode == kScanRows && c->h_small[6] != 0) {  // a row is longer than its slots: scan again for the rows
-      c->row_scale = std::min(64.0, c->row_scale * 1.5);
+      c->row_longest = std::max(c->row_longest, c->h_small[6]);
       mode = kScan;
     }
   }

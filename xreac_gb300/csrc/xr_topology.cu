@@ -319,8 +319,8 @@ __global__ void k_neighbors(XrWork w) {
 // and leaves each row, in canonical order, in its system's slots of cand_edge's memory; after the
 // counts' scan k_emit_rows places them. An entry is one word: the atom within its system (16 bits),
 // the bond and hydrogen-bond flags and the number of the image among the scan's (14 bits; a lane keeps
-// a 64-bit mask of its target's images). A row longer than its slots is counted but sets counts[6],
-// and the host has k_neighbors<true> scan again. Rows of several images a pair profit most. Count,
+// a 64-bit mask of its target's images). A row longer than its slots is counted and its length goes to
+// counts[6], and the host has k_neighbors<true> scan again. Rows of several images a pair profit most. Count,
 // then rows and reverse edges, against scanning twice: 24 slabs of 288 atoms 163 + 466 -> 171 + 51 us,
 // one 73 + 166 -> 69 + 37 us, 128 clusters of up to 512 atoms 80 + 122 -> 73 + 56 us.
 constexpr uint32_t kScanBond = 1u << 16, kScanHb = 1u << 17;
@@ -409,7 +409,7 @@ __global__ void k_scan_rows(XrWork w) {
     w.cnt[1 * L + i] = n_h;
     w.cnt[2 * L + i] = n_bh;
     w.cnt[3 * L + i] = n_ba;
-    if (n_e > cap) w.counts[6] = 1;
+    if (n_e > cap) atomicMax(w.counts + 6, n_e);
   }
 }
 
