@@ -114,3 +114,31 @@ def test_slots_follow_the_longest_row():
     symbols, x = _water(100, seed=8)
     calc.evaluate(symbols, x, cell=np.diag([14.5] * 3), pbc=True)
     assert calc.memory()["candidates"] == held["candidates"]
+
+
+def test_threads_whose_rows_need_different_shared_memory():
+    """Row bitmaps of more than 48 KB a block, of two sizes, from two contexts at once (the limit is a setting of
+    the process)."""
+    import threading
+
+    from test_gpu_qeq_rows import lattice_water
+
+    from xreac_gb300 import Calculator, ForceField
+
+    got, errors = {}, []
+
+    def work(n_mol):
+        try:
+            calc = Calculator(ForceField.bundled(FF))
+            symbols, x, cell = lattice_water(n_mol, seed=n_mol)
+            got[n_mol] = [calc.evaluate(symbols, x, cell=cell, pbc=True).energy for _ in range(12)]
+        except Exception as exc:  # noqa: BLE001 (reported by the main thread)
+            errors.append(exc)
+
+    threads = [threading.Thread(target=work, args=(n,)) for n in (11000, 13800)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors
+    assert all(len(set(v)) == 1 for v in got.values()) and len(got) == 2

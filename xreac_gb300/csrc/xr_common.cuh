@@ -327,6 +327,9 @@ enum BJ { BJ_BO = 0, BJ_PI, BJ_PP, BJ_SIG, BJ_BO0, BJ_PI0, BJ_PP0, BJ_CI, BJ_CJ,
 #define XR_CHUNK_ATOMS 32
 
 // Kernel launchers (defined in the .cu files, called by the engine).
+// The shared memory that k_rank_rows and k_row_sort may ask for, set once per context to their largest: the setting is the
+// process's, so a launch that set what it needs could meet another thread's smaller value.
+bool xr_topology_ready();
 void xr_launch_topology(const XrWork& w, cudaStream_t st);  // xr_launch_prep, then xr_launch_count
 void xr_launch_prep(const XrWork& w, cudaStream_t st);      // wrapped FP32 coordinates (k_prep)
 void xr_launch_count(const XrWork& w, cudaStream_t st);     // all-pairs image scan, counts (k_neighbors<false>)

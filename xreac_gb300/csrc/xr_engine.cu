@@ -1901,6 +1901,7 @@ int xr_ctx_create(int device, void* stream, xr_ctx** out) {
   for (cudaStream_t& s : c->side) made = made && cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking) == cudaSuccess;
   for (cudaEvent_t& v : c->fork_ev) made = made && cudaEventCreateWithFlags(&v, cudaEventDisableTiming) == cudaSuccess;
   cudaDeviceGetAttribute(&c->nsm, cudaDevAttrMultiProcessorCount, device);
+  made = made && xr_topology_ready();
   c->coop_per_sm = xr_qeq_coop_blocks_per_sm();
   c->qeq_direct = xr_qeq_direct_ready();
   if (c->qeq_direct) {

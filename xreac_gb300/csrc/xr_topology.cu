@@ -1121,10 +1121,18 @@ int xr_launch_cell_rows(const XrWork& w, cudaStream_t st) {
   return 1;
 }
 
+static constexpr size_t rank_bytes(int natoms) { return sizeof(uint32_t) * 3 * kRankWarps * (size_t)rank_words(natoms); }
+
+bool xr_topology_ready() {
+  return cudaFuncSetAttribute(k_rank_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)rank_bytes(XR_RANK_ATOMS)) ==
+             cudaSuccess &&
+         cudaFuncSetAttribute(k_row_sort, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              (int)(sizeof(unsigned long long) * XR_ROW_SORT_MAX)) == cudaSuccess;
+}
+
 void xr_launch_rank_rows(const XrWork& w, int natoms, cudaStream_t st) {
   const int words = rank_words(natoms);
-  const size_t bytes = sizeof(uint32_t) * 3 * kRankWarps * (size_t)words;
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(k_rank_rows, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+  const size_t bytes = rank_bytes(natoms);
   k_rank_rows<<<(w.A + kRankWarps - 1) / kRankWarps, 32 * kRankWarps, bytes, st>>>(w, words);
 }
 
@@ -1144,7 +1152,6 @@ void xr_launch_row_sort(const XrWork& w, int max_row, cudaStream_t st) {
   while (cap < max_row) cap <<= 1;
   if (max_row < 2) return;
   const size_t bytes = sizeof(unsigned long long) * cap;
-  if (bytes > 48 * 1024) cudaFuncSetAttribute(k_row_sort, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
   k_row_sort<<<w.A, 128, bytes, st>>>(w, cap);
 }
 
