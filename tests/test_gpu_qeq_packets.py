@@ -66,3 +66,22 @@ def test_teams_with_plain_rows_do_not_touch_each_other():
     for _ in range(3):
         for g, again in zip(got, calc.evaluate_many(boxes)):
             np.testing.assert_array_equal(again.charges, g.charges)
+
+
+def test_every_wait_has_its_own_number():
+    """Whatever wait of a solve a test makes run out, barrier, sum or packet exchange, the call raises; past the last one
+    it does not. A solve has more waits than iterations."""
+    calc = calculator()
+    s = system(343)
+    calc.evaluate(**s)
+    iterations = calc.qeq_work()[0]
+    raised = []
+    for k in range(1, 4 * iterations):
+        calc.set_wait_test(polls=2000, fail_at=k)
+        try:
+            calc.evaluate(**s)
+            raised.append(False)
+        except RuntimeError:
+            raised.append(True)
+    assert raised.index(False) > iterations
+    assert not any(raised[raised.index(False):])

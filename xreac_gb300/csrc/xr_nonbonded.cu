@@ -298,7 +298,7 @@ struct GridTeam {
         for (int k = 0; k < NV; ++k) rs[rank * 8 + k] = v[k];
         asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(bar) : "memory");
         const long long cap = wait_cap(w, 1ll << 24);
-        const bool poisoned = wait_poisoned(w, target / nb);
+        const bool poisoned = wait_poisoned(w, episode());
         long long it = 0;
         while (poisoned || ld_acquire(bar) < target) {
           if (++it > cap || ((it & 255) == 0 && (*(volatile int*)w.status & XR_S_BARRIER))) {
