@@ -7,9 +7,13 @@
 // src/xreac/energy.py:95-102 is solved by iterative refinement, as the FP32 CG's sweeps are: each
 // step solves H y = -g, sum y = 0 for the FP64 gradient g = H x + chi - lambda projected onto the
 // constraint, adds y to the FP64 charges, restores sum x = Q and forms the gradient again in FP64
-// from the unscaled entries. The FP64 gradient's norm decides convergence against the CG solver's
-// target. A step that does not cut the squared norm by 1e3 (a singular or badly indefinite matrix:
-// the elimination does not pivot) leaves the system to the CG solver, which starts over.
+// from the unscaled entries. The FP64 gradient's norm is held against the CG solver's target. The last
+// correction has no gradient after it: it is made from one that meets the target already, or from one that a step as
+// good as the one before it would bring to a hundredth of the target (of the squared norms). A step cuts the squared
+// norm by some 1e12, so that is the third as a rule, from a norm 1 to 30 times the target's, which a cut by 1e3
+// would do too. A step that does not cut the squared norm by 1e3 (a singular or badly indefinite matrix, or one whose
+// smallest eigenvalue FP32 does not resolve; the elimination does not pivot) leaves the system to the CG
+// solver, which starts over.
 //
 // The matrix is held as 32 x 32 tiles of its lower block triangle, column-major (rows of a column
 // contiguous), and factorized as L D L' with D the 32 x 32 diagonal blocks, whose inverses replace
