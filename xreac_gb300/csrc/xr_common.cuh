@@ -185,12 +185,11 @@ struct XrWork {
   int* cand_cnt;
   int2* cand_edge;
   // cell list of the call's atoms: atom_cell [A] (global cell index, -1 unbinned), atom_slot [A], the
-  // cells' atom ranges cell_cnt [ncells + 1] (counts, then their exclusive scan) and cell_atoms [A]
+  // cells' atom ranges cell_cnt [ncells + 1] (counts, then their exclusive scan) and cell_pos [A]
   int* atom_cell;
   int* atom_slot;
   int* cell_cnt;
-  int* cell_atoms;
-  float4* cell_pos;           // [A] wrapped FP32 positions in the order of cell_atoms, the atom in the fourth word
+  float4* cell_pos;           // [A] wrapped FP32 positions in cell order, the atom in the fourth word
   int ncells;
   int row_cap;                // slots per atom of the rows that k_cell_rows leaves in cand_edge's memory
   // edges
@@ -346,7 +345,7 @@ int xr_launch_candidates(const XrWork& w, bool fill, cudaStream_t st);
 // The edges within the cutoff of the candidate list: fill=false counts into cnt (scanned by
 // xr_launch_scan), fill=true writes the rows, pairs and bonds.
 void xr_launch_filter(const XrWork& w, bool fill, cudaStream_t st);
-// Cell list of the atoms binned by k_prep (atom_cell): counts per cell, their scan, cell_atoms.
+// Cell list of the atoms binned by k_prep (atom_cell): counts per cell, their scan, cell_pos.
 int xr_launch_cells(const XrWork& w, cudaStream_t st);
 // Candidate list at the cutoff of w.sys from the cell list, in no particular order within a row:
 // fill=false counts into cand_cnt, scans it (total into counts[5]) and records the longest row in

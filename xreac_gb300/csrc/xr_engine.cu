@@ -113,8 +113,6 @@ struct xr_ctx {
   size_t catom_slot = 0;
   int* cell_cnt = nullptr;
   size_t ccell_cnt = 0;
-  int* cell_atoms = nullptr;
-  size_t ccell_atoms = 0;
   float4* cell_pos = nullptr;
   size_t ccell_pos = 0;
   int reserved_atoms = 0, reserved_systems = 0;  // of the last xr_ctx_reserve
@@ -1102,7 +1100,7 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     ncells = plan_cells(c, nsys, sys, mode == kBuild ? rc + 2.0 * c->skin : rc, mode == kBuild ? c->h_sys_list : nullptr);
     if (ncells > 0) {
       if (!grow(c, &c->atom_cell, &c->catom_cell, (size_t)A) || !grow(c, &c->atom_slot, &c->catom_slot, (size_t)A) ||
-          !grow(c, &c->cell_atoms, &c->ccell_atoms, (size_t)A) || !grow(c, &c->cell_cnt, &c->ccell_cnt, (size_t)ncells + 1) ||
+          !grow(c, &c->cell_cnt, &c->ccell_cnt, (size_t)ncells + 1) ||
           !grow(c, &c->cell_pos, &c->ccell_pos, (size_t)A) || !grow(c, &c->cand_cnt, &c->ccand_cnt, (size_t)A + 1))
         return cuda_fail(c, cudaErrorMemoryAllocation, "allocation");
       if (mode == kScan) {
@@ -1186,7 +1184,6 @@ int run_batch(xr_ctx* c, const xr_ff* ff, int nsys, const xr_system* sys, unsign
     w.atom_cell = c->atom_cell;
     w.atom_slot = c->atom_slot;
     w.cell_cnt = c->cell_cnt;
-    w.cell_atoms = c->cell_atoms;
     w.cell_pos = c->cell_pos;
     w.ncells = (int)ncells;
     w.row_cap = row_cap;
@@ -1940,7 +1937,7 @@ void xr_ctx_destroy(xr_ctx* c) {
                   c->bond_i, c->bond_j, c->b_r, c->b_v, c->b_fwd, c->b_adj, c->b_e, c->dbrow, c->sys, c->energy,
                   c->props, c->status, c->counts, c->barrier, c->qmap, c->qsmall, c->qiters, c->qretry, c->red, c->qguess, c->qrhs, c->qadj, c->pgrad, c->bx_count,
                   c->arow, c->nact, c->nzrow, c->nnz, c->qb_first, c->qb_last, c->chunk_part, c->mids, c->nmids, c->mlist,
-                  c->cand_cnt, c->cand_edge, c->sys_list, c->atom_cell, c->atom_slot, c->cell_cnt, c->cell_atoms, c->cell_pos,
+                  c->cand_cnt, c->cand_edge, c->sys_list, c->atom_cell, c->atom_slot, c->cell_cnt, c->cell_pos,
                   c->mid_tiles, c->qsplit};
   for (void* p : bufs)
     if (p) cudaFree(p);
@@ -2182,7 +2179,7 @@ int xr_ctx_reserve(xr_ctx* c, int atoms, int systems, long long edges, long long
       !grow(c, &c->cand_cnt, &c->ccand_cnt, (size_t)atoms + 1) ||
       !grow(c, &c->cand_edge, &c->ccand_edge, (size_t)std::max<long long>(edges, 1)) ||
       !grow(c, &c->atom_cell, &c->catom_cell, (size_t)atoms) || !grow(c, &c->atom_slot, &c->catom_slot, (size_t)atoms) ||
-      !grow(c, &c->cell_atoms, &c->ccell_atoms, (size_t)atoms) || !grow(c, &c->cell_pos, &c->ccell_pos, (size_t)atoms) ||
+      !grow(c, &c->cell_pos, &c->ccell_pos, (size_t)atoms) ||
       !grow(c, &c->cell_cnt, &c->ccell_cnt, 2 * (size_t)atoms + 64 * (size_t)systems + 1))
     return cuda_fail(c, cudaErrorMemoryAllocation, "reservation");
   c->reserved_atoms = atoms;
@@ -2209,8 +2206,8 @@ long long xr_footprint_bytes(int atoms, int systems, long long edges, long long 
   const long long per_pair = 3 * sizeof(int) + 6 * sizeof(double);
   const long long per_bond = kBondBytes + 32;  // + the exported-bond record of the result block
   const long long chunks = (long long)systems + atoms / XR_CHUNK_ATOMS + 1;
-  // cand_cnt, atom_cell, atom_slot, cell_atoms, cell_cnt, cell_pos
-  const long long per_cells = 4 * sizeof(int) + 2 * sizeof(int) + sizeof(float4);
+  // cand_cnt, atom_cell, atom_slot, cell_cnt, cell_pos
+  const long long per_cells = 3 * sizeof(int) + 2 * sizeof(int) + sizeof(float4);
   const long long base = (long long)atoms * (per_atom + per_cells) + (long long)systems * (per_system + 64 * sizeof(int)) +
                          edges * (per_edge + sizeof(int2)) + (edges / 2) * per_pair + bonds * per_bond +
                          chunks * XR_PART_N * sizeof(double);

@@ -542,7 +542,6 @@ __global__ void k_cell_fill(XrWork w) {
   const int c = w.atom_cell[a];
   if (c < 0) return;
   const int k = w.cell_cnt[c] + w.atom_slot[a];
-  w.cell_atoms[k] = a;
   const float4 p = w.xw[a];
   w.cell_pos[k] = make_float4(p.x, p.y, p.z, __int_as_float(a));
 }
