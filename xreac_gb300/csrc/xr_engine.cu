@@ -707,13 +707,14 @@ void plan_qeq(xr_ctx* c, const xr_system* sys, int nsys, const std::vector<int>&
 }
 
 // Cluster plan: every system above kQeqSmall atoms is solved by one thread-block cluster
-// (4 blocks in a batch, 8 for a single system; rows split over them, reductions in distributed
-// shared memory), the others
-// by single blocks. Taken when no system is too large for a cluster to be the better choice: above
+// (of 8 blocks while all of the call's get one at once, else of 4; rows split over them, reductions in
+// distributed shared memory), the others by single blocks. Taken when no system is too large for a cluster to be the better choice: above
 // kQeqClusterMax atoms a single-system call spreads the rows over a grid-wide team instead, and
 // above kQeqBatchBlock atoms a batch does. h_qsmall receives the cluster systems, then the others,
 // each largest first.
-constexpr int kQeqClusterMax = 640;
+// The line is the direct solvers' end. A single system past it, on a cluster and on a team (QEq, cold, us): 612 atoms of water
+// 471 and 287, in a cell 619 and 302; 639 atoms 476 and 288, 759 and 298; 626 of C/H/O molecules 694 and 399, 559 and 330.
+constexpr int kQeqClusterMax = kQeqDirectCluster;
 
 bool plan_qeq_cluster(xr_ctx* c, const xr_system* sys, int nsys, const std::vector<int>& ids, int* csize, int* nblocks, int* nbig,
                       int* nsmall) {
