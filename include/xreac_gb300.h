@@ -144,7 +144,9 @@ const char* xr_last_error(const xr_ctx* ctx);
  * the whole device. */
 int xr_ctx_reserve(xr_ctx* ctx, int atoms, int systems, long long edges, long long bonds);
 
-/* Solver settings: QEq conjugate-gradient relative residual and iteration limit. */
+/* Solver settings: QEq relative residual and conjugate-gradient iteration limit (1e-13 and 2000 by default). A limit
+ * below 400 makes every system take the conjugate-gradient solver, which the limit is for; with 400 or more, systems of
+ * up to 608 atoms are solved directly, which takes a half to a third of the time. */
 int xr_ctx_set_qeq(xr_ctx* ctx, double tolerance, int max_iterations);
 
 /* Tests of the failure path of the QEq solver's team waits (no reference counterpart). Every wait

@@ -363,6 +363,10 @@ class Calculator:
         uniform start q = Q/n (also for warm starts from ``initial_charges``). The default 1e-13
         keeps charges within about 1e-12 e of the exact KKT solution, which holds fixed-charge
         forces of ionic systems (Ti/O) within 2e-8 kcal/mol/A of the reference.
+
+        ``max_iterations`` bounds the conjugate-gradient iterations. Below 400 every system takes that
+        solver; with 400 or more, systems of up to 608 atoms are solved directly, which takes a half to
+        a third of the time.
         """
         if self._lib.xr_ctx_set_qeq(self._ctx.handle, float(tolerance), int(max_iterations)) != nat.XR_OK:
             raise ValueError("QEq tolerance must be positive and the iteration limit at least 1")

@@ -741,13 +741,15 @@ bool plan_qeq_cluster(xr_ctx* c, const xr_system* sys, int nsys, const std::vect
 }
 
 // The systems small enough for the direct solvers (xr_qeq_direct.cu) by class, each largest first, and the
-// others (for the CG plans). A caller that bounds the CG iterations, or the test that makes a team wait
-// run out, gets the CG solver whose iterations and waits those are.
+// others (for the CG plans). A caller that bounds the iterations below this number, or the test that makes a team
+// wait run out, gets the CG solver whose iterations and waits those are.
 constexpr int kQeqDirectIterations = 400;
-// The largest system alone in its call that one block solves. A cluster pays two cluster barriers a tile step and has
-// eight blocks' FP64 for the products of long rows: a block takes 111 us for 192 atoms of water, open, and 178 in a
-// cell, a cluster 116 and 136; for 225 atoms 140 and 180 against 137 and 148, for 288 186 and 273 against 165 and 186;
-// for 99 open atoms 75 against 94.
+// The largest system alone in its call that one block solves; in a batch a block solves up to kQeqDirectMax atoms. A
+// cluster pays two cluster barriers a tile step and has eight blocks' FP64 for the products of long rows: a block takes
+// 111 us for 192 atoms of water, open, and 178 in a cell, a cluster 116 and 136; for 225 atoms 140 and 180 against 137 and
+// 148, for 288 186 and 273 against 165 and 186; for 99 open atoms 75 against 94. The line is where the open
+// systems' cross; the rule looks at the number of atoms alone, and a cell whose rows are full costs a block more from
+// fewer atoms on (192 in a cell: 42 us), as do 193 to 288 atoms in a batch too small to fill the chip.
 constexpr int kQeqDirectBlockAlone = 192;
 
 struct DirectPlan {
