@@ -27,7 +27,7 @@ One step = one pass of the whole stream through the continuous-batching server
   the torch-backed autograd stand-in of ``tests/golden/shim``) on a sample of the stream; the CPU
   oracle (the reference's algorithm restated) only where that install is absent.
 
-``--impl reference`` times the same reference, one ``xreac.Calculator.evaluate`` per request of the
+``--impl reference`` times the same reference (without that install it says so and times nothing), one ``xreac.Calculator.evaluate`` per request of the
 same seeded stream (consecutive requests, each step a bounded sample), with every host thread, and
 prints the same JSON line with ``"impl": "reference"`` and the same ``config``. That arm imports
 nothing of the product package: the stream comes from ``xreac_gb300/workloads.py`` loaded from its
@@ -220,7 +220,7 @@ def profiled_traffic(kernel):
 
 
 def profiled_fp64(kernel):
-    """FP64-pipe utilisation (% of peak, elapsed) of ``kernel`` from an ``ncu`` capture, recorded in
+    """FP64-pipe utilisation (% of peak, of the active cycles) of ``kernel`` from an ``ncu`` capture, recorded in
     profiles/fp64_pipe.txt."""
     path = ROOT / "profiles" / "fp64_pipe.txt"
     try:
@@ -343,7 +343,7 @@ def stream_pass(reqs, tag, part=None):
 
 
 class CpuArm:
-    """The CPU implementation timed as the reference: the unmodified xreac from baseline/_ref
+    """The CPU implementation timed beside the device: the unmodified xreac from baseline/_ref
     (``kind`` "reference"), or, where it is absent, the CPU oracle ("port")."""
 
     def __init__(self):
@@ -398,13 +398,16 @@ def bench_config(atoms):
 def run_reference(args, world, rank):
     if rank != 0:
         return 0
+    arm = CpuArm()
+    if arm.kind != "reference":  # the port's time would not be the reference's
+        print(json.dumps({"impl": "reference", "unavailable": arm.why}), flush=True)
+        return 0
     import torch
 
     cores = os.cpu_count() or 1
     torch.set_num_threads(cores)
     stream = workloads_module().request_stream()
     atoms_per_pass = sum(r.system.n for r in stream)
-    arm = CpuArm()
     step_budget = float(os.environ.get("XR_REFERENCE_STEP_S", "5"))
     pos = 0
     for _ in range(max(args.warmup, 1)):
