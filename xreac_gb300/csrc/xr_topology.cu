@@ -457,8 +457,8 @@ __global__ void k_emit_rows(XrWork w) {
 // Candidate list: every image (j, S) within the descriptor's cutoff (the list cutoff rc + 2 skin,
 // from a second set of descriptors), in canonical order, without flags: one counter per atom
 // (FILL=false, into cand_cnt) or the rows (FILL=true, cand_edge = {j, shift bits}). Each image is classified once a
-// pass where a target has at most 64: the fill did it twice, and a 12-step relaxation of 648 atoms, which
-// builds one list, took 8,469 us (8,417).
+// pass where a target has at most 64: the fill did it twice, and a relaxation of 648 atoms (10 steps, 12
+// evaluations), which builds one list, took 8,469 us (8,417).
 template <bool FILL>
 __global__ void k_candidates(XrWork w) {
   const int lane = threadIdx.x & 31;
