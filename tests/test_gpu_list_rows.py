@@ -142,3 +142,17 @@ def test_threads_whose_rows_need_different_shared_memory():
         t.join()
     assert not errors
     assert all(len(set(v)) == 1 for v in got.values()) and len(got) == 2
+
+
+def test_a_second_smaller_reservation_keeps_the_first():
+    from xreac_gb300 import Calculator, ForceField
+
+    calc = Calculator(ForceField.bundled(FF))
+    calc.set_cell_list(False)
+    rng = np.random.default_rng(3)
+    x = 8.0 * np.stack(np.unravel_index(np.arange(800), (10, 10, 8)), axis=1) + rng.uniform(-0.1, 0.1, (800, 3))
+    calc.reserve(800, 1, edges_per_atom=20, bonds_per_atom=1)
+    calc.reserve(10, 1, edges_per_atom=20, bonds_per_atom=1)
+    before = calc.memory()
+    calc.evaluate(["O"] * 800, x)
+    assert calc.memory() == before

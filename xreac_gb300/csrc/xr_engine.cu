@@ -115,7 +115,7 @@ struct xr_ctx {
   size_t ccell_cnt = 0;
   float4* cell_pos = nullptr;
   size_t ccell_pos = 0;
-  int reserved_atoms = 0, reserved_systems = 0;  // of the last xr_ctx_reserve
+  int reserved_atoms = 0, reserved_systems = 0;  // the most of every xr_ctx_reserve
   int row_longest = 0;  // the longest row that did not fit the slots its system's density suggested
   // Skin reuse (xr_ctx_set_skin): the list of the last call is reused by a call on the same systems
   // (atom counts, types, cells, pbc, cutoff) in which no atom moved more than `skin` from where it was
@@ -2185,8 +2185,8 @@ int xr_ctx_reserve(xr_ctx* c, int atoms, int systems, long long edges, long long
       !grow(c, &c->cell_pos, &c->ccell_pos, (size_t)atoms) ||
       !grow(c, &c->cell_cnt, &c->ccell_cnt, 2 * (size_t)atoms + 64 * (size_t)systems + 1))
     return cuda_fail(c, cudaErrorMemoryAllocation, "reservation");
-  c->reserved_atoms = atoms;
-  c->reserved_systems = systems;
+  c->reserved_atoms = std::max(c->reserved_atoms, atoms);
+  c->reserved_systems = std::max(c->reserved_systems, systems);
   return XR_OK;
 }
 
